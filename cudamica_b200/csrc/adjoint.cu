@@ -23,6 +23,11 @@
 namespace amica {
 cudaError_t launch_estep_plain(const EStepArgs& a, int NP, int nclusters, cudaStream_t st);
 cudaError_t launch_estep_tc(const EStepArgs& a, int NP, int nclusters, cudaStream_t st, int split, int shape);
+// mstep.cu
+cudaError_t launch_reduce(const double* partial, double* raw, double* stats, int nslots, int M, int n, int m,
+                          int psi_step, int psi_is_phi, cudaStream_t st);
+cudaError_t launch_adjoint_dw(const double* raw, const double* A, double* out, int n, int m, int M,
+                              cudaStream_t st);
 }
 
 using namespace amica;
@@ -41,46 +46,33 @@ __device__ double psi_dev(double x) {
     return r;
 }
 
-__global__ void k_adjoint_reduce(const double* __restrict__ partial, double* __restrict__ raw,
-                                 int nclusters, int M, int stride) {
-    const int64_t total = (int64_t)M * stride;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int q = 0; q < nclusters; q++) s += partial[(size_t)q * total + e];
-        raw[e] = s;
-    }
-}
-
-// out: [0] sum P (relative), then dW (M n n, column-major), dmu, dbeta, drho (M m n)
-__global__ void k_adjoint_finalize(const double* __restrict__ raw, const double* __restrict__ A,
+// out: [0] sum P (relative), then dW (M n n, column-major), dmu, dbeta, drho
+// (M m n).  blockIdx.y = model; dW here only where the n x n block is
+// Psi = sum g x^T (sum g (x - c)^T = Psi - gsum c^T); where it is phi, dW is a
+// product with A and comes from launch_adjoint_dw.
+__global__ void __launch_bounds__(256) k_adjoint_finalize(const double* __restrict__ raw, const double* __restrict__ A,
                                    const double* __restrict__ c, const double* __restrict__ beta,
                                    const double* __restrict__ rho, double* __restrict__ out, int n,
                                    int m, int M, int psi_is_phi) {
-    const int h = blockIdx.x;
+    const int h = blockIdx.y;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     PartLayout PL{n, m};
     const double* R = raw + (size_t)h * PL.stride();
     const double vsum = R[1];
-    if (h == 0 && threadIdx.x == 0) out[0] = R[0];
-    double* dW = out + 1 + (size_t)h * n * n;
-    const double* Ah = A + (size_t)h * n * n;
-    const double* Psi = R + PL.psi();
-    const double* gs = R + PL.gs();
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int i = e % n, k = e / n;   // dW(i,k) stored at k*n + i
-        // W^{-T}(i,k) = A(k,i); sum_t g (x - c)^T = Psi - gsum c^T = phi W^{-T} = phi A^T
-        double gx;
-        if (psi_is_phi) {
-            gx = 0.0;
-            for (int l = 0; l < n; l++) gx += Psi[(size_t)l * n + i] * Ah[(size_t)l * n + k];
-        } else {
-            gx = Psi[(size_t)k * n + i] - gs[i] * c[(size_t)h * n + k];
+    if (h == 0 && t0 == 0) out[0] = R[0];
+    if (!psi_is_phi) {
+        double* dW = out + 1 + (size_t)h * n * n;
+        const double* Ah = A + (size_t)h * n * n;
+        const double* Psi = R + PL.psi();
+        const double* gs = R + PL.gs();
+        for (int e = t0; e < n * n; e += nt) {
+            const int i = e % n, k = e / n;   // dW(i,k) stored at k*n + i; W^{-T}(i,k) = A(k,i)
+            dW[e] = vsum * Ah[(size_t)i * n + k] - (Psi[(size_t)k * n + i] - gs[i] * c[(size_t)h * n + k]);
         }
-        dW[e] = vsum * Ah[(size_t)i * n + k] - gx;
     }
     const size_t off_mu = 1 + (size_t)M * n * n;
     const size_t mnM = (size_t)M * m * n;
-    for (int e = threadIdx.x; e < m * n; e += blockDim.x) {
+    for (int e = t0; e < m * n; e += nt) {
         const size_t idx = (size_t)h * m * n + e;
         const double bt = beta[idx], r = rho[idx];
         const double us = R[PL.mix(kUs) + e];
@@ -105,17 +97,20 @@ cudaError_t launch_adjoint(const EStepArgs& a0, int NP, double* grad_partial, in
     return use_tc ? launch_estep_tc(a, NP, nclusters, st, 0, tc_shape) : launch_estep_plain(a, NP, nclusters, st);
 }
 
-cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int nclusters, int n,
+// The product phi A^T runs as the M-step's tiled FP64 GEMM: with one CTA per
+// model walking it entry by entry this step took 333 us at n = 100, M = 2, and
+// the slot sum with one thread per entry 98 us.
+cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int nslots, int psi_step, int n,
                                     int m, int M, const double* A, const double* c,
                                     const double* beta, const double* rho, double* out,
                                     int psi_is_phi, cudaStream_t st) {
-    PartLayout PL{n, m};
-    const int64_t total = (int64_t)M * PL.stride();
-    int grid = (int)((total + 255) / 256);
-    if (grid > 4096) grid = 4096;
-    k_adjoint_reduce<<<grid, 256, 0, st>>>(grad_partial, raw, nclusters, M, PL.stride());
-    k_adjoint_finalize<<<M, 256, 0, st>>>(raw, A, c, beta, rho, out, n, m, M, psi_is_phi);
-    return cudaGetLastError();
+    cudaError_t e = launch_reduce(grad_partial, raw, nullptr, nslots, M, n, m, psi_step, 0, st);
+    if (e != cudaSuccess) return e;
+    const int len = psi_is_phi ? m * n : n * n;
+    k_adjoint_finalize<<<dim3((len + 255) / 256, M), 256, 0, st>>>(raw, A, c, beta, rho, out, n, m, M, psi_is_phi);
+    e = cudaGetLastError();
+    if (e != cudaSuccess || !psi_is_phi) return e;
+    return launch_adjoint_dw(raw, A, out + 1, n, m, M, st);
 }
 
 }  // namespace amica

@@ -73,7 +73,7 @@ cudaError_t launch_shard_finish(const float* raw, int64_t T, int n, int do_spher
 // adjoint.cu
 cudaError_t launch_adjoint(const EStepArgs& a, int NP, double* grad_partial, int nclusters,
                            cudaStream_t st, bool use_tc, int tc_shape);
-cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int nclusters, int n,
+cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int nslots, int psi_step, int n,
                                     int m, int M, const double* A, const double* c,
                                     const double* beta, const double* rho, double* out,
                                     int psi_is_phi, cudaStream_t st);
@@ -905,7 +905,7 @@ int amica_loglik_adjoint(amica_ctx* c, double* ll, double* dW, double* dmu, doub
         CK(cudaMemsetAsync(c->b.partial, 0, sizeof(double) * (size_t)nsl * M * PL.stride(), c->st));
     }
     CK(launch_adjoint(a, c->NP, c->b.partial, ncl, c->st, c->use_tc, c->tc_shape));
-    CK(launch_adjoint_finalize(c->b.partial, c->b.raw, nsl, n, m, M, c->b.A, c->b.c,
+    CK(launch_adjoint_finalize(c->b.partial, c->b.raw, nsl, c->hc.psi_step, n, m, M, c->b.A, c->b.c,
                                c->b.beta, c->b.rho, c->d_grad, c->hc.psi_is_phi, c->st));
     TRY(check_device_error(c));
     std::vector<double> g(glen);

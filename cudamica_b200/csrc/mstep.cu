@@ -672,10 +672,12 @@ __device__ __forceinline__ double b_entry(const double* __restrict__ phi, double
 //          on the fly from phi, kappa, lambda and sigma2
 //   kind 1 (phi from Psi):  Out = (Psi - gsum c^T) W^T, written into the
 //          statistics vector's phi block
+//   kind 2 (adjoint):  Out = vsum A^T - phi A^T, phi and vsum from the sums of
+//          the gradient sweep (dL/dW_h; src/amica.cu:1535-1550 forms phi only)
 struct GemmArgs {
     int kind, n, m;
     const double* X; size_t strideX;
-    const double* Y; size_t strideY;        // kind 1: W
+    const double* Y; size_t strideY;        // kind 1: W, kind 2: A
     double* Out; size_t strideOut;
     const double* gs; size_t strideG;       // kind 1
     const double* c;                        // kind 1
@@ -683,6 +685,7 @@ struct GemmArgs {
     const Ctrl* ctrl;                       // kind 0
     const double* stats;                    // kind 0: phi and vsum
     const double* work;                     // kind 0: kappa, lambda, sigma2
+    const double* vsum; size_t strideV;     // kind 2
 };
 
 __global__ void __launch_bounds__(256) k_gemm64(GemmArgs g) {
@@ -692,7 +695,7 @@ __global__ void __launch_bounds__(256) k_gemm64(GemmArgs g) {
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;   // ty: 0..7
     const double* Xh = g.X + g.strideX * h;
-    const double* Yh = g.kind == 1 ? g.Y + g.strideY * h : nullptr;
+    const double* Yh = g.kind != 0 ? g.Y + g.strideY * h : nullptr;
     StatLayout SL{n, g.m};
     const double* phi = g.kind == 0 ? g.stats + SL.base(h) + SL.phi() : nullptr;
     const double ivs = g.kind == 0 ? 1.0 / g.stats[SL.base(h) + SL.vs()] : 0.0;
@@ -718,7 +721,7 @@ __global__ void __launch_bounds__(256) k_gemm64(GemmArgs g) {
                 if (g.kind == 1) xv -= g.gs[g.strideG * h + r] * g.c[(size_t)h * n + k];
             }
             xs[tx][rr] = xv;
-            // Y(k0 + rr, c0 + tx): kind 0 -> B_h(k, col); kind 1 -> W^T(k, col) = W(col, k)
+            // Y(k0 + rr, c0 + tx): kind 0 -> B_h(k, col); kinds 1, 2 -> Y^T(k, col) = Y(col, k)
             const int col = c0 + tx;
             double yv = 0.0;
             if (k < n && col < n)
@@ -744,7 +747,8 @@ __global__ void __launch_bounds__(256) k_gemm64(GemmArgs g) {
         if (col >= n) continue;
         double* o = g.Out + g.strideOut * h + (size_t)col * n + r;
         if (g.kind == 0) *o = Xh[(size_t)col * n + r] + s * acc[q];
-        else *o = acc[q];
+        else if (g.kind == 1) *o = acc[q];
+        else *o = g.vsum[g.strideV * h] * Yh[(size_t)r * n + col] - acc[q];
     }
 }
 
@@ -853,25 +857,39 @@ __global__ void __launch_bounds__(1024) k_reparm(int update_A, int do_reparm, do
 // keeps phi in one slot per cluster); when it already is phi it also goes
 // straight into the statistics vector.  Replaces the block/device reductions of
 // src/amica.cu:1618-1920.
-__global__ void k_reduce(const double* __restrict__ partial, double* __restrict__ raw,
-                         double* __restrict__ stats, int nslots, int M, int n, int m, int psi_step,
-                         int psi_is_phi) {
+//
+// A CTA owns 32 consecutive entries; warp w adds slots w, w + nwarps, ... (one
+// 256-byte row of each) and the warps' sums are added in order.  Bound by the
+// latency of the dependent slot loop, not by the (L2-resident) partials: with
+// one thread per entry the 1776 slots of a 32-channel fit took 259 us, and the
+// 888 of a 64-channel one 133 us.
+constexpr int kReduceMaxWarps = 32;
+__global__ void __launch_bounds__(32 * kReduceMaxWarps) k_reduce(
+    const double* __restrict__ partial, double* __restrict__ raw, double* __restrict__ stats, int nslots,
+    int M, int n, int m, int psi_step, int psi_is_phi) {
+    __shared__ double sh[kReduceMaxWarps][32];
     PartLayout PL{n, m};
     StatLayout SL{n, m};
     const int stride = PL.stride(), psi0 = PL.psi();
     const int64_t total = (int64_t)M * stride;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int h = (int)(e / stride);
-        const int off = (int)(e - (int64_t)h * stride);
-        const bool in_psi = off >= psi0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int64_t e = (int64_t)blockIdx.x * 32 + lane;
+    const int h = (int)(e / stride);
+    const int off = (int)(e - (int64_t)h * stride);
+    const bool in_psi = off >= psi0;
+    double s = 0.0;
+    if (e < total) {
         const int step = in_psi ? psi_step : 1;
-        double s = 0.0;
-#pragma unroll 4
-        for (int q = 0; q < nslots; q += step) s += partial[(size_t)q * total + e];
-        raw[e] = s;
-        if (in_psi && psi_is_phi) stats[SL.base(h) + SL.phi() + (off - psi0)] = s;
+        const double* p = partial + e;
+#pragma unroll 8
+        for (int q = warp * step; q < nslots; q += nw * step) s += p[(size_t)q * total];
     }
+    sh[warp][lane] = s;
+    __syncthreads();
+    if (warp != 0 || e >= total) return;
+    for (int w = 1; w < nw; w++) s += sh[w][lane];
+    raw[e] = s;
+    if (in_psi && psi_is_phi) stats[SL.base(h) + SL.phi() + (off - psi0)] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -1197,15 +1215,26 @@ cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream
     return cudaGetLastError();
 }
 
+// stats receives the n x n block when psi_is_phi (else it may be null).  Warps
+// per CTA: about 16 slots each, so that a warp's loop is two batches of eight
+// independent loads (4 warps at the least, to fill the SMs' load queues).
+cudaError_t launch_reduce(const double* partial, double* raw, double* stats, int nslots, int M, int n, int m,
+                          int psi_step, int psi_is_phi, cudaStream_t st) {
+    PartLayout PL{n, m};
+    const int64_t total = (int64_t)M * PL.stride();
+    int nw = 4;
+    while (nw < kReduceMaxWarps && nw * 16 < nslots) nw *= 2;
+    k_reduce<<<(unsigned)((total + 31) / 32), 32 * nw, 0, st>>>(partial, raw, stats, nslots, M, n, m, psi_step,
+                                                                psi_is_phi);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nclusters,
                                    cudaStream_t st) {
     PartLayout PL{h.n, h.m};
     StatLayout SL{h.n, h.m};
-    const int64_t total = (int64_t)h.M * PL.stride();
-    int grid = (int)((total + 255) / 256);
-    if (grid > 4096) grid = 4096;
-    k_reduce<<<grid, 256, 0, st>>>(b.partial, b.raw, b.stats, nclusters, h.M, h.n, h.m,
-                                   h.psi_step > 0 ? h.psi_step : 1, h.psi_is_phi);
+    launch_reduce(b.partial, b.raw, b.stats, nclusters, h.M, h.n, h.m, h.psi_step > 0 ? h.psi_step : 1,
+                  h.psi_is_phi, st);
     k_finalize<<<h.M, kT, 0, st>>>(b.raw, b.W, b.A, b.c, b.beta, b.rho, b.ltc64, b.ctrl, b.stats,
                                    h.n, h.m, h.psi_is_phi);
     if (!h.psi_is_phi) {
@@ -1219,6 +1248,21 @@ cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h,
         ga.c = b.c;
         k_gemm64<<<g, 256, 0, st>>>(ga);
     }
+    return cudaGetLastError();
+}
+
+// dL/dW_h = vsum W^{-T} - phi W^{-T} (W^{-1} = A) from the gradient sweep's sums
+// (tensor-core form, whose n x n block is phi), M matrices of n x n at out.
+cudaError_t launch_adjoint_dw(const double* raw, const double* A, double* out, int n, int m, int M,
+                              cudaStream_t st) {
+    PartLayout PL{n, m};
+    GemmArgs ga{};
+    ga.kind = 2; ga.n = n; ga.m = m;
+    ga.X = raw + PL.psi(); ga.strideX = PL.stride();
+    ga.Y = A; ga.strideY = (size_t)n * n;
+    ga.Out = out; ga.strideOut = (size_t)n * n;
+    ga.vsum = raw + 1; ga.strideV = PL.stride();
+    k_gemm64<<<dim3((n + 31) / 32, (n + 31) / 32, M), 256, 0, st>>>(ga);
     return cudaGetLastError();
 }
 
