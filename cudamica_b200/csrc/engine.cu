@@ -78,6 +78,7 @@ cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int
                                     const double* beta, const double* rho, double* out,
                                     int psi_is_phi, cudaStream_t st);
 
+size_t reject_ws_len(int64_t T);
 cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream_t st);
 cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nclusters,
                                    cudaStream_t st);
@@ -266,11 +267,12 @@ int enqueue_estep(amica_ctx* c) {
 
 // Kernels one iteration launches: inverse/derive, E-step, reduce, finalize
 // (+ phi from Psi in the plain form), params, ctrl, A update (when A is
-// updated), reparametrisation, the finiteness check (+ rejection when enabled).
+// updated), reparametrisation, the finiteness check (+ three for rejection when
+// enabled).
 int launches_per_iteration(const amica_ctx* c) {
     // the split form adds the W split and its two tensor-core contractions
     const int split = c->use_split ? 3 : 0;
-    return 8 + split + (c->hc.psi_is_phi ? 0 : 1) + (c->hc.update_A ? 1 : 0) + (c->hc.do_reject ? 1 : 0);
+    return 8 + split + (c->hc.psi_is_phi ? 0 : 1) + (c->hc.update_A ? 1 : 0) + (c->hc.do_reject ? 3 : 0);
 }
 
 int enqueue_iteration(amica_ctx* c) {
@@ -473,8 +475,7 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     AL(b.raw, M * (size_t)PL.stride());
     AL(b.stats, (size_t)amica_stats_len(n, M, m));
     AL(b.work, M * 4 * n);
-    const int64_t nch = (T + 4095) / 4096;
-    AL(b.chunk, 2 * nch + 2);
+    AL(b.chunk, reject_ws_len(T));
     if (n > 128) AL(b.gj, (size_t)M * nn + (size_t)M * n);
     AL(b.bflag, M); AL(b.use_newton, M);
     AL(b.Wf, (size_t)M * NP * NP); AL(b.wcf, (size_t)M * NP); AL(b.mp, (size_t)M * m * NP);

@@ -1097,87 +1097,160 @@ __global__ void k_ctrl(MCfg cf, const double* __restrict__ stats, Ctrl* ctrl,
 // Rejection pass (engine-defined; the reference has none): over kept samples,
 // mean and std (n-1) of P in FP64, 4096-sample chunks summed in order, then the
 // chunk sums in order; drop kept samples with P < mean - rejsig * std.  Runs
-// only on the iterations the schedule selects.  One CTA.
-__global__ void __launch_bounds__(kT) k_reject(MCfg cf, Ctrl* ctrl, const float* __restrict__ P,
-                                               uint8_t* keep, int64_t T, double* chunk,
-                                               IterRec* hist, int64_t hist_cap, int force) {
+// only on the iterations the schedule selects.
+//
+// Each chunk is one CTA: its samples are loaded by all threads and laid out in
+// shared memory as FP64 terms, a dropped sample as -0 (x + -0 is x for every x),
+// and one thread adds them in order: the order of the sum is part of the rule,
+// so the chain of 4096 dependent FP64 additions is what bounds a pass.  The last
+// CTA to finish (ws->done) adds the chunk sums.  Three launches: the mean, the
+// second moment and threshold, the mask.  One CTA of one thread per chunk, which
+// read its samples from global memory one by one, took 1517 us at T = 300,000.
+constexpr int kRejChunk = 4096;
+struct RejectWs {            // after the chunk sums and chunk counts in the buffer `chunk`
+    double mean, thr;
+    long long nkept, dropped;
+    unsigned done[3];
+};
+__device__ __forceinline__ RejectWs* reject_ws(double* chunk, int64_t T) {
+    return reinterpret_cast<RejectWs*>(chunk + 2 * ((T + kRejChunk - 1) / kRejChunk));
+}
+// ctrl is not written before every CTA of the mask pass has read it here
+__device__ __forceinline__ bool reject_due(const MCfg& cf, const Ctrl* ctrl, int force) {
+    const int64_t it = ctrl->iter;
+    return force || (cf.do_reject && ctrl->rej_passes < cf.maxrej && it >= cf.rejstart &&
+                     ((it - cf.rejstart) % (cf.rejint > 0 ? cf.rejint : 1)) == 0);
+}
+// true in every thread of the CTA that is the last of the grid to call this
+__device__ __forceinline__ bool last_cta(unsigned* done) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
+// PASS 0: chunk sums of P and counts, then the mean; PASS 1: chunk sums of
+// (P - mean)^2, then the threshold.
+template <int PASS>
+__global__ void __launch_bounds__(kT) k_reject_sum(MCfg cf, Ctrl* ctrl, const float* __restrict__ P,
+                                                   const uint8_t* __restrict__ keep, int64_t T, double* chunk,
+                                                   int force) {
+    if (!reject_due(cf, ctrl, force)) return;
+    __shared__ __align__(16) double term[kRejChunk];
+    __shared__ int cnt_s;
     const int tid = threadIdx.x;
-    __shared__ int run;
-    __shared__ double mean_s, thr_s;
-    __shared__ long long nk_s;
-    if (tid == 0) {
-        const Ctrl c = *ctrl;
-        const int64_t it = c.iter;
-        run = force || (cf.do_reject && c.rej_passes < cf.maxrej && it >= cf.rejstart &&
-                        ((it - cf.rejstart) % (cf.rejint > 0 ? cf.rejint : 1)) == 0);
-    }
-    __syncthreads();
-    if (!run) return;
-    const int64_t CH = 4096;
-    const int64_t nch = (T + CH - 1) / CH;
+    const int64_t nch = (T + kRejChunk - 1) / kRejChunk;
+    RejectWs* ws = reject_ws(chunk, T);
     long long* cnt = reinterpret_cast<long long*>(chunk + nch);
-    for (int64_t q = tid; q < nch; q += kT) {
-        double s = 0.0;
-        long long k = 0;
-        const int64_t e = (q + 1) * CH < T ? (q + 1) * CH : T;
-        for (int64_t t = q * CH; t < e; t++)
-            if (keep[t]) { s = __dadd_rn(s, (double)P[t]); k++; }
-        chunk[q] = s;
-        cnt[q] = k;
-    }
+    if (PASS == 1 && *(volatile long long*)&ws->nkept < 2) return;
+    const double mean = PASS == 1 ? *(volatile double*)&ws->mean : 0.0;
+    const int64_t t0 = (int64_t)blockIdx.x * kRejChunk;
+    const int len = (int)(T - t0 < kRejChunk ? T - t0 : kRejChunk);
+    const int padded = (len + 7) & ~7;
+    if (tid == 0) cnt_s = 0;
     __syncthreads();
-    if (tid == 0) {
-        double s = 0.0;
-        long long k = 0;
-        for (int64_t q = 0; q < nch; q++) { s = __dadd_rn(s, chunk[q]); k += cnt[q]; }
-        nk_s = k;
-        mean_s = (k > 0) ? __ddiv_rn(s, (double)k) : 0.0;
-    }
-    __syncthreads();
-    if (nk_s < 2) return;
-    const double mean = mean_s;
-    for (int64_t q = tid; q < nch; q += kT) {
-        double s = 0.0;
-        const int64_t e = (q + 1) * CH < T ? (q + 1) * CH : T;
-        for (int64_t t = q * CH; t < e; t++)
-            if (keep[t]) {
-                const double d = __dsub_rn((double)P[t], mean);
-                s = __dadd_rn(s, __dmul_rn(d, d));
+    int k = 0;
+    for (int i = tid; i < padded; i += kT) {
+        double v = -0.0;
+        if (i < len && keep[t0 + i]) {
+            v = (double)P[t0 + i];
+            if (PASS == 1) {
+                const double d = __dsub_rn(v, mean);
+                v = __dmul_rn(d, d);
             }
-        chunk[q] = s;
+            k++;
+        }
+        term[i] = v;
     }
+    if (PASS == 0 && k) atomicAdd(&cnt_s, k);
     __syncthreads();
     if (tid == 0) {
         double s = 0.0;
-        for (int64_t q = 0; q < nch; q++) s = __dadd_rn(s, chunk[q]);
-        const double sd = __dsqrt_rn(__ddiv_rn(s, (double)(nk_s - 1)));
-        thr_s = __dsub_rn(mean, __dmul_rn(cf.rejsig, sd));
+        const double2* t2 = reinterpret_cast<const double2*>(term);
+#pragma unroll 4
+        for (int i = 0; i < padded / 2; i++) {
+            const double2 v = t2[i];
+            s = __dadd_rn(__dadd_rn(s, v.x), v.y);
+        }
+        chunk[blockIdx.x] = s;
+        if (PASS == 0) cnt[blockIdx.x] = cnt_s;
+    }
+    if (!last_cta(&ws->done[PASS])) return;
+    // the chunk sums in order, through shared memory
+    double s = 0.0;
+    long long n = 0;
+    for (int64_t q0 = 0; q0 < nch; q0 += kT) {
+        const int w = (int)(nch - q0 < kT ? nch - q0 : kT);
+        __syncthreads();
+        if (tid < w) {
+            term[tid] = __ldcg(chunk + q0 + tid);
+            term[kT + tid] = __longlong_as_double(__ldcg(cnt + q0 + tid));
+        }
+        __syncthreads();
+        if (tid == 0)
+            for (int q = 0; q < w; q++) {
+                s = __dadd_rn(s, term[q]);
+                n += __double_as_longlong(term[kT + q]);
+            }
+    }
+    if (tid != 0) return;
+    if (PASS == 0) {
+        ws->nkept = n;
+        ws->mean = (n > 0) ? __ddiv_rn(s, (double)n) : 0.0;
+    } else {
+        const double sd = __dsqrt_rn(__ddiv_rn(s, (double)(n - 1)));
+        ws->thr = __dsub_rn(mean, __dmul_rn(cf.rejsig, sd));
         ctrl->rej_mean = mean;
         ctrl->rej_std = sd;
     }
-    __syncthreads();
-    const double thr = thr_s;
-    long long dropped = 0;
-    for (int64_t t = tid; t < T; t += kT)
+    ws->done[PASS] = 0;
+}
+
+__global__ void __launch_bounds__(kT) k_reject_mask(MCfg cf, Ctrl* ctrl, const float* __restrict__ P,
+                                                    uint8_t* keep, int64_t T, double* chunk, IterRec* hist,
+                                                    int64_t hist_cap, int force) {
+    if (!reject_due(cf, ctrl, force)) return;
+    RejectWs* ws = reject_ws(chunk, T);
+    if (*(volatile long long*)&ws->nkept < 2) return;
+    const double thr = *(volatile double*)&ws->thr;
+    int dropped = 0;
+    for (int64_t t = blockIdx.x * (int64_t)kT + threadIdx.x; t < T; t += (int64_t)gridDim.x * kT)
         if (keep[t] && (double)P[t] < thr) { keep[t] = 0; dropped++; }
-    __shared__ double shd[33];
-    const double dd = block_sum((double)dropped, shd);
-    if (tid == 0) {
-        const int64_t d = (int64_t)dd;
+    dropped = __reduce_add_sync(0xffffffffu, dropped);
+    if ((threadIdx.x & 31) == 0 && dropped) atomicAdd((unsigned long long*)&ws->dropped, (unsigned long long)dropped);
+    if (!last_cta(&ws->done[2])) return;
+    if (threadIdx.x == 0) {
+        const int64_t d = (int64_t)atomicAdd((unsigned long long*)&ws->dropped, 0ull);
         ctrl->nkeep -= d;
         ctrl->nrej_total += d;
         ctrl->rej_passes += 1;
         ctrl->last_rejected = d;
         const int64_t it = ctrl->iter;
         if (hist && it >= 1 && it - 1 < hist_cap) hist[it - 1].nrejected = d;
+        ws->dropped = 0;
+        ws->done[2] = 0;
     }
+}
+
+void reject_pass(const MCfg& cf, Ctrl* ctrl, const float* P, uint8_t* keep, int64_t T, double* chunk,
+                 IterRec* hist, int64_t hist_cap, int force, cudaStream_t st) {
+    const unsigned nch = (unsigned)((T + kRejChunk - 1) / kRejChunk);
+    k_reject_sum<0><<<nch, kT, 0, st>>>(cf, ctrl, P, keep, T, chunk, force);
+    k_reject_sum<1><<<nch, kT, 0, st>>>(cf, ctrl, P, keep, T, chunk, force);
+    const unsigned grid = (unsigned)std::min<int64_t>((T + 4 * kT - 1) / (4 * kT), 592);
+    k_reject_mask<<<grid, kT, 0, st>>>(cf, ctrl, P, keep, T, chunk, hist, hist_cap, force);
 }
 
 }  // namespace
 
 namespace amica {
 
-
+// doubles of the rejection pass's workspace (zeroed once): chunk sums, chunk
+// counts and the counters that each pass leaves at zero
+size_t reject_ws_len(int64_t T) { return 2 * ((T + kRejChunk - 1) / kRejChunk) + (sizeof(RejectWs) + 7) / 8; }
 
 static MCfg to_mcfg(const MStepCfgHost& h) {
     MCfg c;
@@ -1309,14 +1382,14 @@ cudaError_t launch_mstep(const MStepBuffers& b, const MStepCfgHost& h, const flo
                                              (int64_t)h.M * h.n, nmix, h.M, b.err);
     }
     if (h.do_reject && P_rel && keep)
-        k_reject<<<1, kT, 0, st>>>(cf, b.ctrl, P_rel, keep, T, b.chunk, b.hist, b.hist_cap, 0);
+        reject_pass(cf, b.ctrl, P_rel, keep, T, b.chunk, b.hist, b.hist_cap, 0, st);
     return cudaGetLastError();
 }
 
 cudaError_t launch_reject_now(const MStepBuffers& b, const MStepCfgHost& h, const float* P_rel,
                               uint8_t* keep, int64_t T, cudaStream_t st) {
     const MCfg cf = to_mcfg(h);
-    k_reject<<<1, kT, 0, st>>>(cf, b.ctrl, P_rel, keep, T, b.chunk, b.hist, b.hist_cap, 1);
+    reject_pass(cf, b.ctrl, P_rel, keep, T, b.chunk, b.hist, b.hist_cap, 1, st);
     return cudaGetLastError();
 }
 
