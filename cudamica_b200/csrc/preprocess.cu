@@ -17,6 +17,11 @@
 
 #include "common.cuh"
 
+namespace amica {
+// sphere_eig.cu
+cudaError_t launch_eig_cluster(const double* C, double* V, double* evals, int n, int* done, cudaStream_t st);
+}  // namespace amica
+
 namespace {
 
 constexpr int kChunk = 2048;   // samples per CTA in the reductions
@@ -62,29 +67,35 @@ __global__ void k_scale_scatter(const double* __restrict__ scatter, int n, doubl
 }
 
 // S = V diag(2/sqrt(d)) V^T (do_sphere 1), diag(1/std) (2) or I (0); ldetS.
-__global__ void k_sphere(const double* __restrict__ V, const double* __restrict__ evals,
-                         const double* __restrict__ var, int n, int do_sphere,
-                         double* __restrict__ S, double* __restrict__ ldetS) {
-    for (int e = threadIdx.x + blockIdx.x * blockDim.x; e < n * n; e += blockDim.x * gridDim.x) {
+// The scales are formed once per CTA (formed in the inner loop they took the
+// kernel 82 us at n = 128).
+__global__ void __launch_bounds__(256) k_sphere(const double* __restrict__ V, const double* __restrict__ evals,
+                                                const double* __restrict__ var, int n, int do_sphere,
+                                                double* __restrict__ S, double* __restrict__ ldetS) {
+    __shared__ double scale[256], part[8];
+    const int tid = threadIdx.x;
+    if (tid < n) scale[tid] = do_sphere == 1 ? 2.0 / sqrt(evals[tid]) : do_sphere == 2 ? 1.0 / sqrt(var[tid]) : 1.0;
+    __syncthreads();
+    for (int e = tid + blockIdx.x * blockDim.x; e < n * n; e += blockDim.x * gridDim.x) {
         const int i = e % n, k = e / n;
         double v = 0.0;
         if (do_sphere == 1) {
-            for (int q = 0; q < n; q++)
-                v += V[(size_t)q * n + i] * (2.0 / sqrt(evals[q])) * V[(size_t)q * n + k];
-        } else if (do_sphere == 2) {
-            v = (i == k) ? 1.0 / sqrt(var[i]) : 0.0;
+#pragma unroll 8
+            for (int q = 0; q < n; q++) v += V[(size_t)q * n + i] * scale[q] * V[(size_t)q * n + k];
         } else {
-            v = (i == k) ? 1.0 : 0.0;
+            v = (i == k) ? scale[i] : 0.0;
         }
         S[e] = v;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double ld = 0.0;
-        for (int q = 0; q < n; q++) {
-            if (do_sphere == 1) ld += log(2.0 / sqrt(evals[q]));
-            else if (do_sphere == 2) ld += log(fabs(1.0 / sqrt(var[q])));
+    if (blockIdx.x == 0) {
+        double ld = tid < n ? log(scale[tid]) : 0.0;
+        for (int o = 16; o > 0; o >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, o);
+        if ((tid & 31) == 0) part[tid >> 5] = ld;
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < 8; w++) ld += part[w];
+            *ldetS = -ld;
         }
-        *ldetS = -ld;
     }
 }
 
@@ -195,7 +206,9 @@ __device__ __forceinline__ int pk_sym(int i, int j) { return i <= j ? pk_idx(i, 
 constexpr int kJacThreads = 1024;
 __global__ void __launch_bounds__(kJacThreads, 1) k_jacobi_smem(const double* __restrict__ C,
                                                                 double* __restrict__ Vout,
-                                                                double* __restrict__ evals, int n) {
+                                                                double* __restrict__ evals, int n,
+                                                                const int* __restrict__ done) {
+    if (*done) return;                                  // launch_eig_cluster has decomposed C
     extern __shared__ __align__(16) double jsm[];
     const int np = (n * (n + 1)) / 2;
     double* ap = jsm;                                   // packed upper triangle
@@ -421,7 +434,9 @@ struct JacGlobal {
 __global__ void __launch_bounds__(kJacThreads, 1) k_jacobi_grid(const double* __restrict__ C,
                                                                 double* __restrict__ V,
                                                                 double* __restrict__ evals, int n,
-                                                                JacGlobal g, int* err) {
+                                                                JacGlobal g, int* err,
+                                                                const int* __restrict__ done) {
+    if (*done) return;                                  // the same in every block
     __shared__ double cs[128], sn[128];
     __shared__ int pp[128], qq[128];
     __shared__ double red[32];
@@ -728,11 +743,18 @@ cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const d
     double* V = evwork;
     double* ev = evwork + (size_t)n * n;
     double* var = ev + n;
+    int* done = reinterpret_cast<int*>(var + n);
+    if (do_sphere == 1) {
+        // the armed test hook is about the cooperative solver's waits: let it run
+        e = fault_wait_cycles > 0 ? cudaMemsetAsync(done, 0, sizeof(int), st)
+                                  : amica::launch_eig_cluster(cov, V, ev, n, done, st);
+        if (e != cudaSuccess) return e;
+    }
     if (do_sphere == 1 && !big) {
         const size_t jsmem = sizeof(double) * (size_t)((((n * (n + 1)) / 2 + 1) & ~1) + n * n);
         e = cudaFuncSetAttribute(k_jacobi_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem);
         if (e != cudaSuccess) return e;
-        k_jacobi_smem<<<1, kJacThreads, jsmem, st>>>(cov, V, ev, n);
+        k_jacobi_smem<<<1, kJacThreads, jsmem, st>>>(cov, V, ev, n, done);
     } else if (do_sphere == 1) {
         // Jacobi state in the partial buffer: packed triangle, the stopping-test
         // partials, the barrier counter and the abort flag
@@ -751,7 +773,7 @@ cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const d
         e = cudaMemsetAsync(part + np + 2 * nb, 0, 2 * sizeof(double), st);
         if (e != cudaSuccess) return e;
         double* covp = const_cast<double*>(cov);
-        void* args[] = {(void*)&covp, (void*)&V, (void*)&ev, (void*)&n, (void*)&jg, (void*)&err};
+        void* args[] = {(void*)&covp, (void*)&V, (void*)&ev, (void*)&n, (void*)&jg, (void*)&err, (void*)&done};
         e = cudaLaunchCooperativeKernel((const void*)k_jacobi_grid, dim3(nb), dim3(kJacThreads), args, 0, st);
         if (e != cudaSuccess) return e;
     } else if (do_sphere == 2 && !var_ready) {
