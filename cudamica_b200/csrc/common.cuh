@@ -182,3 +182,10 @@ __device__ __forceinline__ float ptx_rcp(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// D(8x8) += A(8x4) B(4x8) in FP64 (mma.sync; tcgen05 has no FP64 kind): lane
+// (g, q) = (lane / 4, lane % 4) holds A(g, q), B(q, g) and D(g, 2q), D(g, 2q + 1)
+__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}

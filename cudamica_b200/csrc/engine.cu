@@ -61,11 +61,12 @@ cudaError_t launch_preprocess(const float* raw, int64_t T, int n, int do_sphere,
                               double* cov, double* sphere, double* evwork, double* ldetS_dev,
                               float* x, int ldx, int tf32, int* err, cudaStream_t st,
                               long long fault_wait_cycles);
+size_t preprocess_min_ws(int n);
 cudaError_t launch_convert_sphered(const double* xs, int64_t T, int n, float* x, int ldx, int tf32,
                                    cudaStream_t st);
 cudaError_t launch_shard_colsum(const float* raw, int64_t T, int n, double* sums, cudaStream_t st);
 cudaError_t launch_shard_scatter(const float* raw, int64_t T, int n, const double* sums, int64_t T_total,
-                                 double* means, double* scatter, cudaStream_t st);
+                                 double* means, double* scatter, int* err, cudaStream_t st);
 cudaError_t launch_shard_finish(const float* raw, int64_t T, int n, int do_sphere, const double* means,
                                 const double* scatter, int64_t T_total, double* cov, double* sphere,
                                 double* evwork, double* ldetS_dev, float* x, int ldx, int tf32, int* err,
@@ -487,7 +488,7 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     AL(c->d_keep, T); AL(c->d_Lt, M * T); AL(c->d_P, T);
     // 3 zero samples past T: the tensor-core form reads the data as rows of up
     // to 4 samples
-    AL(c->d_x, (size_t)(T + 3) * NP);
+    AL(c->d_x, std::max((size_t)(T + 3) * NP, 2 * preprocess_min_ws((int)n)));   // the sphering's scratch first
     AL(c->d_means, n); AL(c->d_sphere, nn); AL(c->d_cov, nn); AL(c->d_evwork, 4 * nn + 4 * n);
     AL(c->d_ldetS, 1);
     c->backup_len = param_len(c) + (sizeof(Ctrl) + 7) / 8;
@@ -538,7 +539,8 @@ static int load_raw(amica_ctx* c, const float* x, int64_t n, int64_t T, cudaMemc
     if (!c || !x) return AMICA_ERR_INVALIDPARAM;
     if (n != c->n || T != c->T) return AMICA_ERR_INVALIDPARAM;
     CK(cudaSetDevice(c->dev));
-    if (!c->d_rawx) CK(cudaMalloc(&c->d_rawx, sizeof(float) * (size_t)T * n));
+    // 16 spare bytes: the preprocessing reads the data in 16-byte units
+    if (!c->d_rawx) CK(cudaMalloc(&c->d_rawx, sizeof(float) * ((size_t)T * n + 4)));
     CK(cudaMemcpyAsync(c->d_rawx, x, sizeof(float) * (size_t)T * n, kind, c->st));
     c->have_data = true;
     c->have_x = false;
@@ -1090,7 +1092,8 @@ int amica_shard_scatter(amica_ctx* c, const double* d_sums_total, int64_t T_tota
     if (!c || !d_sums_total || !d_scatter || T_total < c->T) return AMICA_ERR_INVALIDPARAM;
     if (!c->have_data) return AMICA_ERR_STATE;
     CK(cudaSetDevice(c->dev));
-    CK(launch_shard_scatter(c->d_rawx, c->T, c->n, d_sums_total, T_total, c->d_means, d_scatter, c->st));
+    CK(launch_shard_scatter(c->d_rawx, c->T, c->n, d_sums_total, T_total, c->d_means, d_scatter, c->b.err,
+                            c->st));
     CK(cudaStreamSynchronize(c->st));
     TRY(check_device_error(c));
     c->have_shard_mean = true;

@@ -73,14 +73,6 @@ constexpr size_t kInvSmem = sizeof(double) * ((size_t)kInvN * kLdA + 3 * (size_t
 
 __device__ __forceinline__ void bar_panel() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
 
-// D(8x8) += A(8x4) B(4x8) in FP64: lane (g, q) = (lane / 4, lane % 4) holds
-// A(g, q), B(q, g) and D(g, 2q), D(g, 2q + 1)
-__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // pivot key of row r holding v (0: not a candidate)
 __device__ __forceinline__ uint32_t pivot_key(double v, bool usable, int r) {
     return usable ? ((((uint32_t)__double2hiint(v)) & 0x7fffff80u) | (uint32_t)(127 - r)) + 128u : 0u;

@@ -12,10 +12,12 @@
 //   ldetS     -log|det S| = -sum log of the eigen-scales
 //   x         S (x - mean) in FP64, rounded once to FP32 into the padded
 //             sample-major layout the E-step reads.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
 #include "common.cuh"
+#include "tc_ptx.cuh"
 
 namespace amica {
 // sphere_eig.cu
@@ -24,35 +26,76 @@ cudaError_t launch_eig_cluster(const double* C, double* V, double* evals, int n,
 
 namespace {
 
-constexpr int kChunk = 2048;   // samples per CTA in the reductions
-
-__global__ void k_colsum(const float* __restrict__ x, int64_t T, int n, double* __restrict__ part) {
-    const int64_t t0 = (int64_t)blockIdx.x * kChunk;
-    const int64_t t1 = t0 + kChunk < T ? t0 + kChunk : T;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s = 0.0;
-        for (int64_t t = t0; t < t1; t++) s += (double)x[t * n + i];
+// Column sums of a contiguous run of samples per CTA: a group of ceil(n / 32)
+// warps reads one sample (coalesced), the CTA's groups take samples in turn with
+// eight in flight per thread, and the groups' sums are added in order.  Bound by
+// HBM (0.10 ms for the 512 MB of n = 128, T = 1M); with one thread per channel and no more than n threads busy per CTA it
+// took 561 us at n = 128, T = 1M (512 MB) and 569 us at n = 160, T = 50k.
+constexpr int kSumThreads = 256;
+__global__ void __launch_bounds__(kSumThreads) k_colsum(const float* __restrict__ x, int64_t T, int n, int64_t chunk,
+                                                        double* __restrict__ part) {
+    __shared__ double sh[kSumThreads];
+    const int width = (n + 31) & ~31;                  // <= kSumThreads
+    const int ngrp = kSumThreads / width;
+    const int grp = threadIdx.x / width, i = threadIdx.x - grp * width;
+    const int64_t t0 = (int64_t)blockIdx.x * chunk;
+    const int64_t t1 = t0 + chunk < T ? t0 + chunk : T;
+    double s = 0.0;
+    if (grp < ngrp && i < n) {
+        int64_t t = t0 + grp;
+        for (; t + 7 * ngrp < t1; t += 8 * ngrp) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = x[(t + u * ngrp) * n + i];
+#pragma unroll
+            for (int u = 0; u < 8; u++) s += (double)v[u];
+        }
+        for (; t < t1; t += ngrp) s += (double)x[t * n + i];
+    }
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    if (grp == 0 && i < n) {
+        for (int g = 1; g < ngrp; g++) s += sh[g * width + i];
         part[(size_t)blockIdx.x * n + i] = s;
     }
 }
 
-// mean = (sum of the per-CTA partial sums) / div; div = 1 gives the sums
-__global__ void k_mean(const double* __restrict__ part, int nblk, int n, double div,
-                       double* __restrict__ mean) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblk; b++) s += part[(size_t)b * n + i];
-        mean[i] = s / div;
+// out[e] = (sum over nblk partials of part[b * len + e], in a fixed order) / div
+// for e < len: a CTA owns 32 entries, its 16 warps share the partials
+constexpr int kFoldWarps = 16;
+__device__ __forceinline__ double fold_partials(const double* __restrict__ part, int nblk, size_t len, size_t e,
+                                                bool in) {
+    __shared__ double sh[kFoldWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double s = 0.0;
+    if (in) {
+#pragma unroll 8
+        for (int b = warp; b < nblk; b += kFoldWarps) s += part[(size_t)b * len + e];
     }
+    sh[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0)
+        for (int w = 1; w < kFoldWarps; w++) s += sh[w][lane];
+    return s;                                          // warp 0
+}
+__global__ void __launch_bounds__(32 * kFoldWarps) k_mean(const double* __restrict__ part, int nblk, int n,
+                                                          double div, double* __restrict__ mean) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const double s = fold_partials(part, nblk, n, i, i < n);
+    if (threadIdx.x < 32 && i < n) mean[i] = s / div;
 }
 
-__global__ void k_cov_reduce(const double* __restrict__ part, int nblk, int n, double div,
-                             double* __restrict__ C) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n * n) return;
-    double s = 0.0;
-    for (int b = 0; b < nblk; b++) s += part[(size_t)b * n * n + e];
-    C[e] = s / div;
+// The partial covariances hold the 32 x 32 tiles on and above the diagonal.
+__global__ void __launch_bounds__(32 * kFoldWarps) k_cov_reduce(const double* __restrict__ part, int nblk, int n,
+                                                                double div, double* __restrict__ C) {
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31);
+    const int i = e % n, k = e / n;                    // element (i, k) at k * n + i
+    const bool in = e < n * n && (i >> 5) <= (k >> 5);
+    const double s = fold_partials(part, nblk, (size_t)n * n, e, in);
+    if (threadIdx.x < 32 && in) {
+        C[e] = s / div;
+        C[(size_t)i * n + k] = s / div;
+    }
 }
 
 // The sharded form's inputs to k_sphere: the covariance (scatter / T) and, for
@@ -130,8 +173,6 @@ __global__ void k_var(const float* __restrict__ x, int64_t T, int n, const doubl
     }
 }
 
-// x_out[t][i] = sum_k S(i,k) (x[t][k] - mean[k]) in FP64, rounded to FP32;
-// padded channels are zero.
 // Round to the TF32 grid, nearest with ties away from zero (the tensor cores
 // read only the top 19 bits of an FP32 operand, i.e. truncate; storing the data
 // pre-rounded makes the TF32 contraction see an unbiased value).
@@ -141,53 +182,155 @@ __device__ __forceinline__ float round_tf32(float v) {
     return __uint_as_float(r);
 }
 
-// Partial covariance: one persistent CTA per SM over a contiguous sample range;
-// thread (bi, bk) owns the 8 x 8 block C[8 bi .. 8 bi + 7][8 bk .. 8 bk + 7] in
-// registers (n <= 128: 16 x 16 blocks, 256 threads).  Samples are staged 32 at
-// a time, centred, in shared memory.
-constexpr int kCovRows = 32;
-__global__ void __launch_bounds__(256, 1) k_cov8(const float* __restrict__ x, int64_t T, int n,
-                                                 int64_t chunk, const double* __restrict__ mean,
-                                                 double* __restrict__ part) {
-    __shared__ __align__(16) double xs[kCovRows][128];
-    const int bi = threadIdx.x & 15, bk = threadIdx.x >> 4;
+// A stage of raw samples for the two kernels below: [t0, t0 + rows) up to T is
+// one contiguous run of floats that starts on a 16-byte boundary (t0 a multiple
+// of 16), so one bulk copy brings it; its size is rounded up to 16 bytes (the
+// raw buffer has 16 spare bytes at its end).
+__device__ __forceinline__ void load_run(float* dst, const float* x, int64_t t0, int64_t T, int rows, int n,
+                                         uint64_t* bar) {
+    const int64_t left = T - t0;
+    const uint32_t bytes = ((uint32_t)(left < rows ? left : rows) * (uint32_t)n * 4u + 15u) & ~15u;
+    mbar_expect_tx(bar, bytes);
+    bulk_load(smem_u32(dst), x + t0 * n, bytes, bar);
+}
+// f(row, channel) over this thread's elements of a stage: the (row, 32-channel
+// block) pairs warp, warp + nw, ... of rows x nb
+template <class F>
+__device__ __forceinline__ void each_element(int rows, int nb, int nw, F&& f) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int dr = nw / nb, db = nw - dr * nb;
+    int r = warp / nb, blk = warp - r * nb;
+    while (r < rows) {
+        f(r, blk * 32 + lane);
+        r += dr;
+        blk += db;
+        if (blk >= nb) { blk -= nb; r++; }
+    }
+}
+
+// Partial covariance sum_t xc_t xc_t^T (xc = x - mean) in FP64 on the tensor
+// cores (mma.sync m8n8k4), one persistent CTA per SM over a contiguous sample
+// range.  The channels form 32 x 32 tiles of which only those on and above the
+// diagonal are computed: warp = (tile, replica), a replica taking every
+// nrep-th group of four samples.  A fragment (four samples of eight channels)
+// has the same layout as either operand.  A stage arrives by one bulk copy during
+// the products of the one before and is centred into one of two FP64 tiles (row
+// stride 4 doubles modulo 16: fragment loads free of bank conflicts), so that a
+// stage has one barrier and warps that are done with one tile convert into the
+// other.  Bound by the FP64 pipe: at n = 128, T = 1M the ten tiles are 2.05e10
+// flop, 0.56 ms at the 36.7 TFLOP/s that this instruction reaches; it takes 0.84
+// ms (the FP64 pipe 59% busy with 32-sample stages, more with 64).  (The 8 x 8
+// register blocking on the FMA pipe that it replaced computed all of C, in 128
+// channels whatever n: 2.6 ms there, and 3.3e10 flop at n = 32 as well.)
+struct CovPlan {
+    int nb, ntl, nrep, ysplit, rows;   // channel blocks, tiles per CTA, replicas, CTAs per sample range, samples per stage
+    int threads;
+    size_t smem;
+};
+CovPlan cov_plan(int n) {
+    CovPlan p;
+    p.nb = (n + 31) / 32;
+    const int tiles = p.nb * (p.nb + 1) / 2;
+    p.ysplit = tiles <= 20 ? 1 : tiles == 21 ? 3 : 2;  // 20 warps of 96 registers fill an SM; 28 and 36 are even
+    p.ntl = tiles / p.ysplit;
+    p.nrep = p.ntl == 1 ? 8 : p.ntl == 3 ? 4 : p.ntl <= 10 ? 2 : 1;
+    p.rows = p.nb == 1 ? 128 : p.nb <= 5 ? 64 : 32;
+    p.threads = 32 * p.ntl * p.nrep;
+    p.smem = sizeof(double) * 2 * (size_t)p.rows * (32 * p.nb + 4) + sizeof(float) * (size_t)p.rows * n;
+    const size_t fold = sizeof(double) * (size_t)p.ntl * 1024;   // replicas are added through the FP64 tiles
+    if (p.nrep > 1 && p.smem < fold) p.smem = fold;
+    return p;
+}
+constexpr int kCovMaxThreads = 640;
+__global__ void __launch_bounds__(kCovMaxThreads, 1) k_cov_mma(const float* __restrict__ x, int64_t T, int n,
+                                                              int64_t chunk, const double* __restrict__ mean,
+                                                              double* __restrict__ part, int nb, int ntl, int nrep,
+                                                              int rows, int* err) {
+    extern __shared__ __align__(16) double cv[];
+    const int ld = 32 * nb + 4;
+    double* xs = cv;                                   // [2][rows][ld], centred
+    float* raw = reinterpret_cast<float*>(cv + 2 * (size_t)rows * ld);   // [rows][n]
+    __shared__ double mean_s[256];
+    __shared__ uint64_t bar;
+    __shared__ int abort_s;
+    volatile int* abort_flag = &abort_s;
+    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int rep = warp / ntl;
+    int tile = warp - rep * ntl + blockIdx.y * ntl, kb = 0;
+    while (tile > kb) { tile -= kb + 1; kb++; }        // column kb holds tiles (0 .. kb, kb)
+    const int ib = tile;
     const int64_t t0 = (int64_t)blockIdx.x * chunk;
     const int64_t t1 = t0 + chunk < T ? t0 + chunk : T;
-    double acc[8][8];
+    for (int i = tid; i < 256; i += nthr) mean_s[i] = i < n ? mean[i] : 0.0;
+    if (tid == 0) {
+        abort_s = 0;
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (t0 < t1) load_run(raw, x, t0, t1, rows, n, &bar);
+    }
+    double acc[4][4][2];
 #pragma unroll
-    for (int a = 0; a < 8; a++)
+    for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int b = 0; b < 8; b++) acc[a][b] = 0.0;
-    for (int64_t tb = t0; tb < t1; tb += kCovRows) {
+        for (int c = 0; c < 4; c++) acc[a][c][0] = acc[a][c][1] = 0.0;
+    __syncthreads();                                   // mean_s, the barrier
+    uint32_t stage = 0;
+    for (int64_t tb = t0; tb < t1; tb += rows, stage++) {
+        double* xb = xs + (size_t)(stage & 1) * rows * ld;
+        mbar_wait(&bar, stage & 1, abort_flag, err);
+        each_element(rows, nb, nw, [&](int r, int i) {
+            xb[r * ld + i] = (tb + r < t1 && i < n) ? (double)raw[r * n + i] - mean_s[i] : 0.0;
+        });
         __syncthreads();
-        for (int e = threadIdx.x; e < kCovRows * 128; e += 256) {
-            const int r = e >> 7, i = e & 127;
-            const int64_t t = tb + r;
-            xs[r][i] = (t < t1 && i < n) ? (double)x[t * n + i] - mean[i] : 0.0;
-        }
-        __syncthreads();
+        if (tid == 0 && tb + rows < t1) load_run(raw, x, tb + rows, t1, rows, n, &bar);
 #pragma unroll 2
-        for (int r = 0; r < kCovRows; r++) {
-            double xi[8], xk[8];
+        for (int r0 = 4 * rep; r0 < rows; r0 += 4 * nrep) {
+            const double* row = xb + (r0 + q) * ld + g;
+            double fa[4], fb[4];
 #pragma unroll
-            for (int a = 0; a < 8; a += 2) {
-                const double2 u = *reinterpret_cast<const double2*>(&xs[r][8 * bi + a]);
-                const double2 w = *reinterpret_cast<const double2*>(&xs[r][8 * bk + a]);
-                xi[a] = u.x; xi[a + 1] = u.y; xk[a] = w.x; xk[a + 1] = w.y;
+            for (int a = 0; a < 4; a++) {
+                fa[a] = row[32 * ib + 8 * a];
+                fb[a] = row[32 * kb + 8 * a];
             }
 #pragma unroll
-            for (int a = 0; a < 8; a++)
+            for (int a = 0; a < 4; a++)
 #pragma unroll
-                for (int b = 0; b < 8; b++) acc[a][b] = fma(xi[a], xk[b], acc[a][b]);
+                for (int c = 0; c < 4; c++) dmma884(acc[a][c][0], acc[a][c][1], fa[a], fb[c]);
         }
     }
+    // replicas into replica 0, in order
+    double* fold = cv + (size_t)(warp - rep * ntl) * 1024 + lane;
+    for (int w = 1; w < nrep; w++) {
+        __syncthreads();
+        if (rep == w) {
 #pragma unroll
-    for (int a = 0; a < 8; a++)
+            for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int b = 0; b < 8; b++) {
-            const int i = 8 * bi + a, k = 8 * bk + b;
-            if (i < n && k < n) part[(size_t)blockIdx.x * n * n + (size_t)k * n + i] = acc[a][b];
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int u = 0; u < 2; u++) fold[((a * 4 + c) * 2 + u) * 32] = acc[a][c][u];
         }
+        __syncthreads();
+        if (rep == 0) {
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int u = 0; u < 2; u++) acc[a][c][u] += fold[((a * 4 + c) * 2 + u) * 32];
+        }
+    }
+    if (rep != 0) return;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int i = 32 * ib + 8 * a + g, k = 32 * kb + 8 * c + 2 * q + u;
+                if (i < n && k < n) part[(size_t)blockIdx.x * n * n + (size_t)k * n + i] = acc[a][c][u];
+            }
 }
 
 // Parallel-ordered cyclic Jacobi eigendecomposition of the symmetric n x n
@@ -332,62 +475,6 @@ __global__ void __launch_bounds__(kJacThreads, 1) k_jacobi_smem(const double* __
 }
 
 // ---------------------------------------------------------------------------
-// 128 < n <= 256.  The n <= 128 kernels keep the whole problem in one SM; here
-// the covariance runs k_cov8's register blocking on the four 128 x 128
-// quadrants, the eigendecomposition spreads the same Jacobi rounds over a
-// cooperative grid, and the sphering keeps a 64-row slice of S per CTA.
-
-// k_cov8 for the quadrant (oi, ok) of C (rows oi .., columns ok ..): blockIdx.y
-// selects the quadrant; both 128-channel sample slices are staged.
-__global__ void __launch_bounds__(256, 1) k_cov8q(const float* __restrict__ x, int64_t T, int n,
-                                                  int64_t chunk, const double* __restrict__ mean,
-                                                  double* __restrict__ part) {
-    extern __shared__ __align__(16) double cq[];
-    double (*xi_s)[128] = reinterpret_cast<double (*)[128]>(cq);
-    double (*xk_s)[128] = reinterpret_cast<double (*)[128]>(cq + kCovRows * 128);
-    const int oi = 128 * (blockIdx.y & 1), ok = 128 * (blockIdx.y >> 1);
-    const int bi = threadIdx.x & 15, bk = threadIdx.x >> 4;
-    const int64_t t0 = (int64_t)blockIdx.x * chunk;
-    const int64_t t1 = t0 + chunk < T ? t0 + chunk : T;
-    double acc[8][8];
-#pragma unroll
-    for (int a = 0; a < 8; a++)
-#pragma unroll
-        for (int b = 0; b < 8; b++) acc[a][b] = 0.0;
-    for (int64_t tb = t0; tb < t1; tb += kCovRows) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < kCovRows * 128; e += 256) {
-            const int r = e >> 7, i = e & 127;
-            const int64_t t = tb + r;
-            const bool in = t < t1;
-            xi_s[r][i] = (in && oi + i < n) ? (double)x[t * n + oi + i] - mean[oi + i] : 0.0;
-            xk_s[r][i] = (in && ok + i < n) ? (double)x[t * n + ok + i] - mean[ok + i] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 2
-        for (int r = 0; r < kCovRows; r++) {
-            double xi[8], xk[8];
-#pragma unroll
-            for (int a = 0; a < 8; a += 2) {
-                const double2 u = *reinterpret_cast<const double2*>(&xi_s[r][8 * bi + a]);
-                const double2 w = *reinterpret_cast<const double2*>(&xk_s[r][8 * bk + a]);
-                xi[a] = u.x; xi[a + 1] = u.y; xk[a] = w.x; xk[a + 1] = w.y;
-            }
-#pragma unroll
-            for (int a = 0; a < 8; a++)
-#pragma unroll
-                for (int b = 0; b < 8; b++) acc[a][b] = fma(xi[a], xk[b], acc[a][b]);
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 8; a++)
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            const int i = oi + 8 * bi + a, k = ok + 8 * bk + b;
-            if (i < n && k < n) part[(size_t)blockIdx.x * n * n + (size_t)k * n + i] = acc[a][b];
-        }
-}
-
 // Grid-wide barrier for a cooperative launch: a monotonic arrival counter;
 // barrier number b completes when it reaches (b + 1) * gridDim.x.  The wait is
 // bounded (~1 s); on expiry it records kErrWaitTimeout and sets *abort, after
@@ -563,116 +650,108 @@ __global__ void __launch_bounds__(kJacThreads, 1) k_jacobi_grid(const double* __
     for (int i = gtid; i < n; i += gthreads) evals[i] = __ldcg(ap + pk_idx(i, i));
 }
 
-// x_out[t][i] for 128 < n <= 256: blockIdx.y picks 64 output channels whose
-// rows of S stay in shared memory; 16-sample tiles, one (sample, 2 channels)
-// per thread; the same k-ascending FMA order as k_apply_sphere8.
-constexpr int kSphTileQ = 16;
-__global__ void __launch_bounds__(512, 1) k_apply_sphere_q(const float* __restrict__ x, int64_t T,
-                                                           int n, const double* __restrict__ mean,
-                                                           const double* __restrict__ S,
-                                                           float* __restrict__ xo, int ldx, int tf32) {
-    extern __shared__ __align__(16) double sq[];
-    double* Sq = sq;                                   // [256][64]: S(i0 + il, k) at k * 64 + il
-    double* xc = sq + 256 * 64;                        // [16][257]
-    constexpr int XL = 257;
-    const int i0 = 64 * blockIdx.y;
-    for (int e = threadIdx.x; e < 256 * 64; e += 512) {
-        const int k = e >> 6, il = e & 63, i = i0 + il;
-        Sq[e] = (i < n && k < n) ? S[(size_t)k * n + i] : 0.0;
-    }
-    const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t ntile = (T + kSphTileQ - 1) / kSphTileQ;
-    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-        const int64_t t0 = tile * kSphTileQ;
-        __syncthreads();
-        for (int e = threadIdx.x; e < kSphTileQ * 256; e += 512) {
-            const int r = e >> 8, k = e & 255;
-            const int64_t t = t0 + r;
-            xc[r * XL + k] = (t < T && k < n) ? (double)x[t * n + k] - mean[k] : 0.0;
-        }
-        __syncthreads();
-        double acc0 = 0.0, acc1 = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < n; k++) {
-            const double xv = xc[s * XL + k];
-            acc0 = fma(Sq[k * 64 + lane], xv, acc0);
-            acc1 = fma(Sq[k * 64 + lane + 32], xv, acc1);
-        }
-        const int64_t t = t0 + s;
-        if (t < T) {
-            const double accs[2] = {acc0, acc1};
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int i = i0 + lane + 32 * u;
-                if (i < ldx) {
-                    const float v = (i < n) ? (float)accs[u] : 0.f;
-                    xo[t * ldx + i] = tf32 ? round_tf32(v) : v;
-                }
-            }
-        }
+// x_out[t][i] = sum_k S(i,k) (x[t][k] - mean[k]) in FP64 on the tensor cores
+// (mma.sync m8n8k4), rounded once to FP32 (padded channels zero).  A CTA keeps S
+// (all of it up to 128 channels; a slice of 64 output channels above, blockIdx.y)
+// in shared memory and walks sample tiles; a warp computes 16 samples x 16
+// channels, so that two loads of each operand feed four products; both operands
+// have a row stride of 4 doubles modulo 16 (fragment loads free of bank
+// conflicts).  Stages come as in k_cov_mma.  Bound by the FP64 pipe
+// (3.3e10 flop at n = 128, T = 1M, 0.9 ms at 36.7 TFLOP/s; 1.26 ms); the FMA form with 4
+// x 4 register blocks took 2.77 ms there, in 128 channels whatever n, and the
+// form above 128 channels 690 us at n = 160, T = 50k.
+struct SpherePlan {
+    int nt, mt, rows, kpad, yslices;   // 16-channel and 16-sample warp tiles, samples per tile, padded K
+    int threads;
+    size_t smem;
+};
+SpherePlan sphere_plan(int n) {
+    SpherePlan p;
+    const int nb = (n + 31) / 32;
+    p.kpad = 32 * nb;
+    p.nt = n <= 128 ? 2 * nb : 4;
+    p.yslices = n <= 128 ? 1 : (n + 63) / 64;
+    p.mt = n <= 128 ? 16 / p.nt : 2;                   // 16, 16, 12 and 16 warps; 8 above 128 channels
+    for (;; p.mt = 1) {                                // 4 warps above 208 channels
+        p.rows = 16 * p.mt;
+        p.threads = 32 * p.nt * p.mt;
+        p.smem = sizeof(double) * ((size_t)p.kpad * (16 * p.nt + 4) + 2 * (size_t)p.rows * (p.kpad + 4)) +
+                 sizeof(float) * (size_t)p.rows * n;
+        if (p.mt == 1 || p.smem + 4096 <= 232448) return p;
     }
 }
-
-// x_out[t][i] = sum_k S(i,k) (x[t][k] - mean[k]) in FP64, rounded once to FP32
-// (padded channels zero).  Persistent CTAs of 512 threads; S staged in shared
-// memory; a thread computes 4 channels x 4 samples of a 64-sample tile.
-constexpr int kSphTile = 64;
-__global__ void __launch_bounds__(512, 1) k_apply_sphere8(const float* __restrict__ x, int64_t T, int n,
-                                                          const double* __restrict__ mean,
-                                                          const double* __restrict__ S,
-                                                          float* __restrict__ xo, int ldx, int tf32) {
+__global__ void __launch_bounds__(512, 1) k_apply_sphere(const float* __restrict__ x, int64_t T, int n,
+                                                         const double* __restrict__ mean,
+                                                         const double* __restrict__ S, float* __restrict__ xo,
+                                                         int ldx, int tf32, int nt, int mt, int kpad, int* err) {
     extern __shared__ __align__(16) double ssm[];
-    double* Ss = ssm;
-    double* xc = ssm + 128 * 128;
-    constexpr int XL = 129;
-    for (int e = threadIdx.x; e < 128 * 128; e += 512) {
-        const int k = e >> 7, i = e & 127;
-        Ss[e] = (i < n && k < n) ? S[(size_t)k * n + i] : 0.0;
+    const int lds = 16 * nt + 4, ldk = kpad + 4, rows = 16 * mt, nb = kpad >> 5;
+    double* Ss = ssm;                                  // Ss[k * lds + i] = S(i0 + i, k)
+    double* xc = ssm + (size_t)kpad * lds;             // [2] tiles, xc[r * ldk + k]
+    float* raw = reinterpret_cast<float*>(xc + 2 * (size_t)rows * ldk);   // [rows][n]
+    __shared__ double mean_s[256];
+    __shared__ uint64_t bar;
+    __shared__ int abort_s;
+    volatile int* abort_flag = &abort_s;
+    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int i0 = 16 * nt * blockIdx.y;
+    const int wn = warp % nt, wm = warp / nt;
+    const int64_t ntile = (T + rows - 1) / rows;
+    if (tid == 0) {
+        abort_s = 0;
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (blockIdx.x < ntile) load_run(raw, x, (int64_t)blockIdx.x * rows, T, rows, n, &bar);
     }
-    const int ib = threadIdx.x & 31, tb = threadIdx.x >> 5;     // channels 4 ib.., samples 4 tb..
-    const int64_t ntile = (T + kSphTile - 1) / kSphTile;
-    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-        const int64_t t0 = tile * kSphTile;
-        __syncthreads();
-        for (int e = threadIdx.x; e < kSphTile * 128; e += 512) {
-            const int r = e >> 7, k = e & 127;
-            const int64_t t = t0 + r;
-            xc[r * XL + k] = (t < T && k < n) ? (double)x[t * n + k] - mean[k] : 0.0;
+    for (int k = warp; k < kpad; k += nw)
+        for (int il = lane; il < 16 * nt; il += 32) {
+            const int i = i0 + il;
+            Ss[k * lds + il] = (i < n && k < n) ? S[(size_t)k * n + i] : 0.0;
         }
+    for (int i = tid; i < 256; i += nthr) mean_s[i] = i < n ? mean[i] : 0.0;
+    __syncthreads();
+    uint32_t stage = 0;
+    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x, stage++) {
+        const int64_t t0 = tile * rows;
+        double* xb = xc + (size_t)(stage & 1) * rows * ldk;
+        mbar_wait(&bar, stage & 1, abort_flag, err);
+        each_element(rows, nb, nw, [&](int r, int k) {
+            xb[r * ldk + k] = (t0 + r < T && k < n) ? (double)raw[r * n + k] - mean_s[k] : 0.0;
+        });
         __syncthreads();
-        double acc[4][4];
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
+        if (tid == 0 && tile + gridDim.x < ntile) load_run(raw, x, (tile + gridDim.x) * rows, T, rows, n, &bar);
+        double acc[2][2][2] = {};
+        const double* pa = xb + (16 * wm + g) * ldk + q;
+        const double* pb = Ss + q * lds + 16 * wn + g;
+        const int ksteps = (n + 3) >> 2;
 #pragma unroll 4
-        for (int k = 0; k < n; k++) {
-            double s4[4], x4[4];
-#pragma unroll
-            for (int b = 0; b < 4; b += 2) {
-                const double2 v = *reinterpret_cast<const double2*>(&Ss[k * 128 + 4 * ib + b]);
-                s4[b] = v.x; s4[b + 1] = v.y;
-            }
-#pragma unroll
-            for (int a = 0; a < 4; a++) x4[a] = xc[(4 * tb + a) * XL + k];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fma(s4[b], x4[a], acc[a][b]);
+        for (int s = 0; s < ksteps; s++) {
+            const double a0 = pa[4 * s], a1 = pa[8 * ldk + 4 * s];
+            const double b0 = pb[4 * s * lds], b1 = pb[4 * s * lds + 8];
+            dmma884(acc[0][0][0], acc[0][0][1], a0, b0);
+            dmma884(acc[0][1][0], acc[0][1][1], a0, b1);
+            dmma884(acc[1][0][0], acc[1][0][1], a1, b0);
+            dmma884(acc[1][1][0], acc[1][1][1], a1, b1);
         }
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
-            const int64_t t = t0 + 4 * tb + a;
+        for (int a = 0; a < 2; a++) {
+            const int64_t t = t0 + 16 * wm + 8 * a + g;
             if (t >= T) continue;
 #pragma unroll
-            for (int b = 0; b < 4; b++) {
-                const int i = 4 * ib + b;
-                if (i < ldx) {
-                    const float v = (i < n) ? (float)acc[a][b] : 0.f;
-                    xo[t * ldx + i] = tf32 ? round_tf32(v) : v;
-                }
+            for (int c = 0; c < 2; c++) {
+                const int i = i0 + 16 * wn + 8 * c + 2 * q;   // even, and ldx a multiple of 32
+                if (i >= ldx) continue;
+                float2 v = make_float2((float)acc[a][c][0], (float)acc[a][c][1]);
+                if (tf32) v = make_float2(round_tf32(v.x), round_tf32(v.y));
+                *reinterpret_cast<float2*>(xo + t * ldx + i) = v;
             }
         }
+        // the last slice also owns the padding channels past it
+        if (blockIdx.y + 1 == gridDim.y)
+            for (int i = i0 + 16 * nt + 2 * lane; i < ldx; i += 64)
+                for (int r = warp; r < rows && t0 + r < T; r += nw)
+                    *reinterpret_cast<float2*>(xo + (t0 + r) * ldx + i) = make_float2(0.f, 0.f);
     }
 }
 
@@ -694,7 +773,7 @@ __global__ void k_convert(const double* __restrict__ xs, int64_t T, int n, float
 //   pp_scatter: sum_t (x_t - mean)(x_t - mean)^T / div (do_sphere 1 only);
 //   pp_finish:  the eigendecomposition of the covariance, S and ldetS, and
 //               the sphered data x = S (raw - mean) in the layout of the E-step.
-// part: scratch of pp_part_len doubles; evwork: >= 4 n^2 + 4 n doubles.
+// evwork: >= 4 n^2 + 4 n doubles.
 int sm_count() {
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
@@ -702,40 +781,50 @@ int sm_count() {
     return nsm;
 }
 
-size_t pp_part_len(int64_t T, int n) {
-    const size_t nblk = (size_t)((T + kChunk - 1) / kChunk);
-    const size_t a = nblk * n, b = (size_t)sm_count() * n * n;
-    return a > b ? a : b;
+// The steps' scratch: the partial sums and covariances, then the eigensolver's
+// state.  A shorter one gives fewer partials and CTAs.
+struct Scratch {
+    double* p;
+    size_t len;   // doubles, at least preprocess_min_ws(n)
+};
+constexpr int kJacCtas = 64;   // of the cooperative eigensolver
+
+// samples per CTA of the column sums: eight CTAs per SM
+int64_t colsum_chunk(int64_t T, int n, size_t len) {
+    const int64_t ctas = std::min<int64_t>(8 * (int64_t)sm_count(), (int64_t)(len / n));
+    return std::max<int64_t>((T + ctas - 1) / ctas, 64);
+}
+int cov_ranges(int n, size_t len) {
+    return (int)std::min<size_t>(sm_count() / cov_plan(n).ysplit, len / ((size_t)n * n));
 }
 
-cudaError_t pp_colsum(const float* raw, int64_t T, int n, double div, double* part, double* out,
+cudaError_t pp_colsum(const float* raw, int64_t T, int n, double div, Scratch ws, double* out,
                       cudaStream_t st) {
-    const int nblk = (int)((T + kChunk - 1) / kChunk);
-    k_colsum<<<nblk, 256, 0, st>>>(raw, T, n, part);
-    k_mean<<<1, 256, 0, st>>>(part, nblk, n, div, out);
+    const int64_t chunk = colsum_chunk(T, n, ws.len);
+    const int nblk = (int)((T + chunk - 1) / chunk);
+    k_colsum<<<nblk, kSumThreads, 0, st>>>(raw, T, n, chunk, ws.p);
+    k_mean<<<(n + 31) / 32, 32 * kFoldWarps, 0, st>>>(ws.p, nblk, n, div, out);
     return cudaGetLastError();
 }
 
 cudaError_t pp_scatter(const float* raw, int64_t T, int n, const double* means, double div,
-                       double* part, double* out, cudaStream_t st) {
-    const int ncov = sm_count();
-    const int64_t chunk = ((T + ncov - 1) / ncov + kCovRows - 1) / kCovRows * kCovRows;
-    if (n <= 128) {
-        k_cov8<<<ncov, 256, 0, st>>>(raw, T, n, chunk, means, part);
-    } else {
-        const size_t csmem = sizeof(double) * 2 * kCovRows * 128;
-        cudaError_t e = cudaFuncSetAttribute(k_cov8q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
-        if (e != cudaSuccess) return e;
-        k_cov8q<<<dim3(ncov, 4), 256, csmem, st>>>(raw, T, n, chunk, means, part);
-    }
-    k_cov_reduce<<<(n * n + 255) / 256, 256, 0, st>>>(part, ncov, n, div, out);
+                       Scratch ws, double* out, int* err, cudaStream_t st) {
+    const CovPlan p = cov_plan(n);
+    // a range is a whole number of stages; ranges past T are empty and leave zeros
+    const int ncov = cov_ranges(n, ws.len);
+    const int64_t chunk = ((T + ncov - 1) / ncov + p.rows - 1) / p.rows * p.rows;
+    cudaError_t e = cudaFuncSetAttribute(k_cov_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    if (e != cudaSuccess) return e;
+    k_cov_mma<<<dim3(ncov, p.ysplit), p.threads, p.smem, st>>>(raw, T, n, chunk, means, ws.p, p.nb, p.ntl, p.nrep,
+                                                             p.rows, err);
+    k_cov_reduce<<<(n * n + 31) / 32, 32 * kFoldWarps, 0, st>>>(ws.p, ncov, n, div, out);
     return cudaGetLastError();
 }
 
 // var_ready: evwork's variance slot already holds the do_sphere 2 variances
 cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const double* means,
                       const double* cov, double* sphere, double* evwork, double* ldetS_dev,
-                      float* x, int ldx, int tf32, int* err, double* part, bool var_ready,
+                      float* x, int ldx, int tf32, int* err, Scratch ws, bool var_ready,
                       cudaStream_t st, long long fault_wait_cycles) {
     const bool big = n > 128;
     const int nsm = sm_count();
@@ -761,8 +850,9 @@ cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const d
         int per_sm = 0;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jacobi_grid, kJacThreads, 0);
         if (e != cudaSuccess || per_sm < 1) return e ? e : cudaErrorInvalidValue;
-        const int nb = nsm < 64 ? nsm : 64;
+        const int nb = nsm < kJacCtas ? nsm : kJacCtas;
         const size_t np = (size_t)n * (n + 1) / 2;
+        double* part = ws.p;
         JacGlobal jg;
         jg.ap = part;
         jg.part = part + np;
@@ -780,21 +870,16 @@ cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const d
         k_var<<<n, 256, 0, st>>>(raw, T, n, means, var);
     }
     k_sphere<<<(n * n + 255) / 256, 256, 0, st>>>(V, ev, var, n, do_sphere, sphere, ldetS_dev);
-    if (big) {
-        const size_t smemq = sizeof(double) * (256 * 64 + kSphTileQ * 257);
-        e = cudaFuncSetAttribute(k_apply_sphere_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemq);
-        if (e != cudaSuccess) return e;
-        const int64_t ntq = (T + kSphTileQ - 1) / kSphTileQ;
-        const int gq = (int)(ntq < nsm ? ntq : nsm);
-        k_apply_sphere_q<<<dim3(gq, (ldx + 63) / 64), 512, smemq, st>>>(raw, T, n, means, sphere, x, ldx, tf32);
-        return cudaGetLastError();
-    }
-    const size_t smem2 = sizeof(double) * (128 * 128 + kSphTile * 129);
-    e = cudaFuncSetAttribute(k_apply_sphere8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    // the scratch is done with: the rows past T, which the kernel below leaves out
+    e = cudaMemsetAsync(x + (size_t)T * ldx, 0, sizeof(float) * 3 * ldx, st);
     if (e != cudaSuccess) return e;
-    const int64_t ntile = (T + kSphTile - 1) / kSphTile;
-    const int gsph = (int)(ntile < nsm ? ntile : nsm);
-    k_apply_sphere8<<<gsph, 512, smem2, st>>>(raw, T, n, means, sphere, x, ldx, tf32);
+    const SpherePlan p = sphere_plan(n);
+    e = cudaFuncSetAttribute(k_apply_sphere, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    if (e != cudaSuccess) return e;
+    const int64_t ntile = (T + p.rows - 1) / p.rows;
+    const int grid = (int)(ntile < nsm / p.yslices ? ntile : nsm / p.yslices);
+    k_apply_sphere<<<dim3(grid, p.yslices), p.threads, p.smem, st>>>(raw, T, n, means, sphere, x, ldx, tf32, p.nt,
+                                                                   p.mt, p.kpad, err);
     return cudaGetLastError();
 }
 
@@ -802,69 +887,77 @@ cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const d
 
 namespace amica {
 
+// least scratch (doubles): one partial covariance, or the cooperative
+// eigensolver's state
+size_t preprocess_min_ws(int n) {
+    const size_t nn = (size_t)n * n, jac = (size_t)n * (n + 1) / 2 + 2 * kJacCtas + 2;
+    return std::max(nn, jac);
+}
+
+// x holds (T + 3) x ldx floats, and at least 2 preprocess_min_ws(n): until the
+// sphered data are written to it, it serves as the scratch; the 3 rows past T
+// are left zero.
 // fault_wait_cycles > 0 arms the test hook of amica_test_arm_wait_fault for
 // this launch (cooperative eigensolver only: block 0 skips its first arrival,
 // every wait is bounded by fault_wait_cycles).
+static Scratch x_scratch(float* x, int64_t T, int n, int ldx) {
+    return Scratch{reinterpret_cast<double*>(x), std::max((size_t)(T + 3) * ldx / 2, preprocess_min_ws(n))};
+}
 cudaError_t launch_preprocess(const float* raw, int64_t T, int n, int do_sphere, double* means,
                               double* cov, double* sphere, double* evwork, double* ldetS_dev,
                               float* x, int ldx, int tf32, int* err, cudaStream_t st,
                               long long fault_wait_cycles) {
     if (n > 256 || ldx > 256) return cudaErrorInvalidValue;
-    double* part = nullptr;
-    cudaError_t e = cudaMallocAsync(&part, sizeof(double) * pp_part_len(T, n), st);
-    if (e != cudaSuccess) return e;
-    e = pp_colsum(raw, T, n, (double)T, part, means, st);
-    if (e == cudaSuccess && do_sphere == 1) e = pp_scatter(raw, T, n, means, (double)T, part, cov, st);
+    const Scratch ws = x_scratch(x, T, n, ldx);
+    cudaError_t e = pp_colsum(raw, T, n, (double)T, ws, means, st);
+    if (e == cudaSuccess && do_sphere == 1) e = pp_scatter(raw, T, n, means, (double)T, ws, cov, err, st);
     if (e == cudaSuccess)
-        e = pp_finish(raw, T, n, do_sphere, means, cov, sphere, evwork, ldetS_dev, x, ldx, tf32, err, part,
+        e = pp_finish(raw, T, n, do_sphere, means, cov, sphere, evwork, ldetS_dev, x, ldx, tf32, err, ws,
                       false, st, fault_wait_cycles);
-    cudaFreeAsync(part, st);
     return e;
 }
 
 // Sharded preprocessing: the column sums of this shard's raw data (n doubles).
+// (x may be in use: the scratch is its own.)
 cudaError_t launch_shard_colsum(const float* raw, int64_t T, int n, double* sums, cudaStream_t st) {
     if (n > 256) return cudaErrorInvalidValue;
-    double* part = nullptr;
-    cudaError_t e = cudaMallocAsync(&part, sizeof(double) * pp_part_len(T, n), st);
+    Scratch ws{nullptr, (size_t)8 * sm_count() * n};
+    cudaError_t e = cudaMallocAsync(&ws.p, sizeof(double) * ws.len, st);
     if (e != cudaSuccess) return e;
-    e = pp_colsum(raw, T, n, 1.0, part, sums, st);
-    cudaFreeAsync(part, st);
+    e = pp_colsum(raw, T, n, 1.0, ws, sums, st);
+    cudaFreeAsync(ws.p, st);
     return e;
 }
 
 // means = sums / T_total (the column sums of all shards), then the scatter of
 // this shard's raw data about them, n x n doubles.
 cudaError_t launch_shard_scatter(const float* raw, int64_t T, int n, const double* sums, int64_t T_total,
-                                 double* means, double* scatter, cudaStream_t st) {
+                                 double* means, double* scatter, int* err, cudaStream_t st) {
     if (n > 256 || T_total < 1) return cudaErrorInvalidValue;
-    double* part = nullptr;
-    cudaError_t e = cudaMallocAsync(&part, sizeof(double) * pp_part_len(T, n), st);
+    Scratch ws{nullptr, (size_t)sm_count() * n * n};
+    cudaError_t e = cudaMallocAsync(&ws.p, sizeof(double) * ws.len, st);
     if (e != cudaSuccess) return e;
-    k_mean<<<1, 256, 0, st>>>(sums, 1, n, (double)T_total, means);
-    e = pp_scatter(raw, T, n, means, 1.0, part, scatter, st);
-    cudaFreeAsync(part, st);
+    k_mean<<<(n + 31) / 32, 32 * kFoldWarps, 0, st>>>(sums, 1, n, (double)T_total, means);
+    e = pp_scatter(raw, T, n, means, 1.0, ws, scatter, err, st);
+    cudaFreeAsync(ws.p, st);
     return e;
 }
 
 // S and ldetS from the scatter of all shards (T_total samples; do_sphere 1 and
-// 2 read it, 0 ignores it), applied to this shard's samples.
+// 2 read it, 0 ignores it), applied to this shard's samples.  x as in
+// launch_preprocess.
 cudaError_t launch_shard_finish(const float* raw, int64_t T, int n, int do_sphere, const double* means,
                                 const double* scatter, int64_t T_total, double* cov, double* sphere,
                                 double* evwork, double* ldetS_dev, float* x, int ldx, int tf32, int* err,
                                 cudaStream_t st) {
     if (n > 256 || ldx > 256 || T_total < 2) return cudaErrorInvalidValue;
-    double* part = nullptr;
-    cudaError_t e = cudaMallocAsync(&part, sizeof(double) * pp_part_len(T, n), st);
-    if (e != cudaSuccess) return e;
     if (do_sphere != 0)
         k_scale_scatter<<<(n * n + 255) / 256, 256, 0, st>>>(scatter, n, (double)T_total, cov,
                                                              evwork + (size_t)n * n + n);
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
-        e = pp_finish(raw, T, n, do_sphere, means, cov, sphere, evwork, ldetS_dev, x, ldx, tf32, err, part,
-                      true, st, 0);
-    cudaFreeAsync(part, st);
+        e = pp_finish(raw, T, n, do_sphere, means, cov, sphere, evwork, ldetS_dev, x, ldx, tf32, err,
+                      x_scratch(x, T, n, ldx), true, st, 0);
     return e;
 }
 
