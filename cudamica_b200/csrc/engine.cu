@@ -50,6 +50,7 @@ int tc_tile_samples(int n, int shape);
 int tc_partial_groups(int n, int shape);
 int tc_psi_step(int shape);
 int tc_num_shapes();
+int tc_default_shape(int m, int M);
 int tc_cohort_encode_map(const EStepArgs& a, void* map);
 int tc_cohort_ctas();
 cudaError_t launch_estep_tc_cohort(const TcCohortSub* subs, const void* maps, const TcCohortItem* items,
@@ -413,7 +414,7 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     c->use_split = (cfg->precision == AMICA_PREC_MIXED) && !c->use_tc && split_form_supported((int)n) &&
                    T <= 0x7fffffff;
     if (cfg->tc_shape < 0 || cfg->tc_shape >= tc_num_shapes()) { amica_destroy(c); return AMICA_ERR_INVALIDPARAM; }
-    c->tc_shape = c->use_tc ? (int)cfg->tc_shape : 0;
+    c->tc_shape = !c->use_tc ? 0 : cfg->tc_shape ? (int)cfg->tc_shape : tc_default_shape((int)m, (int)M);
     c->S = c->use_tc ? tc_tile_samples((int)n, c->tc_shape) : plain_tile_samples();
     c->ntiles = (int)((T + c->S - 1) / c->S);
     int maxcl = c->use_tc      ? tc_max_clusters((int)n, (int)m, (int)M, c->tc_shape)
@@ -772,6 +773,7 @@ int amica_set_tile_shape(amica_ctx* c, int64_t shape) {
     if (!c->use_tc) return AMICA_ERR_UNSUPPORTED;
     if (c->pending >= 0) return AMICA_ERR_STATE;
     CK(cudaSetDevice(c->dev));
+    if (shape == 0) shape = tc_default_shape(c->m, c->M);
     const int S = tc_tile_samples(c->n, (int)shape);
     const int ntiles = (int)((c->T + S - 1) / S);
     const int mc = tc_max_clusters(c->n, c->m, c->M, (int)shape);
@@ -1197,7 +1199,7 @@ int amica_cohort_create(amica_ctx* const* ctxs, int64_t nsub, amica_cohort** out
         const amica_ctx* c = ctxs[s];
         if (!c || c->dev != c0->dev || c->m != c0->m) return AMICA_ERR_INVALIDPARAM;
         // the cohort kernel runs the default tile shape
-        if (!c->use_tc || c->M != 1 || c->tc_shape != 0) return AMICA_ERR_UNSUPPORTED;
+        if (!c->use_tc || c->M != 1 || c->tc_shape != tc_default_shape(c->m, 1)) return AMICA_ERR_UNSUPPORTED;
     }
     CK(cudaSetDevice(c0->dev));
     amica_cohort* co = new amica_cohort();
@@ -1240,7 +1242,7 @@ int amica_cohort_create(amica_ctx* const* ctxs, int64_t nsub, amica_cohort** out
             delete co;
             return AMICA_ERR_CUDA;
         }
-        co->nslots.push_back(nitem[s] * tc_partial_groups(c->n, 0));
+        co->nslots.push_back(nitem[s] * tc_partial_groups(c->n, c->tc_shape));
     }
     co->nitems = (int)items.size();
     int r = AMICA_OK;

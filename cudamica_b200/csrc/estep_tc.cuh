@@ -32,9 +32,10 @@
 // kErrWaitTimeout, stops waiting, frees its tensor memory and exits.
 //
 // This header holds the kernel template and its launchers; estep_tc.cu
-// instantiates the 3-warpgroup shape (and the cohort kernel, the self-test and
-// the host interface), estep_tc_wg2.cu the 2-warpgroup shapes, so that the two
-// compile in parallel.
+// instantiates the 3-warpgroup shape (and the self-test and the host interface),
+// estep_tc_wg2.cu the 2-warpgroup shapes, so that the two compile in parallel.
+// With one model (M = 1) the form without split correction is another kernel,
+// estep_tc_one.cuh.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -85,7 +86,7 @@ struct TcCfg {
                                   : 384u + (uint32_t)(kSub * (c - 2 * kGapChunks));
     }
 };
-using TcDef = TcCfg<3, 2>;               // the default shape (and the cohort kernel's)
+using TcDef = TcCfg<3, 2>;               // shape 0
 constexpr int kS = TcDef::kS;            // samples per tile (MMA1 N)
 constexpr int kWG = TcDef::kWG;          // density warpgroups
 constexpr int kDensWarps = TcDef::kDensWarps;

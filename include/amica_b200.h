@@ -66,8 +66,9 @@ typedef struct amica_cfg {
                                iteration after a Newton step changed every model's A by
                                less than phi_split_rel (relative, Frobenius) (new key) */
     int64_t tc_shape;       /* mixed form up to 128 channels: tile shape of the fused E-step,
-                               0 (default) 3 density warpgroups and 48-sample tiles with 2 x
-                               stages, 1 2 warpgroups and 32-sample tiles with 2 stages, 2 the
+                               0 the default for the model and mixture counts (3 density
+                               warpgroups and 48-sample tiles with 2 x stages; shape 1 with
+                               5 mixtures, or one model and 4), 1 2 warpgroups and 32-sample tiles with 2 stages, 2 the
                                same with 3 stages (cudamica_b200.autotune picks one by
                                measurement) (new key) */
     double lrate0, lratemax, lnatrate, lratefact, rho0, rholrate, rhomin, rhomax, rejsig;
