@@ -7,6 +7,9 @@ namespace amica {
 
 constexpr int kMaxModels = 8;     // thread-block cluster size limit (portable)
 constexpr int kMaxMix = 8;
+// rows of 128 floats past the sphered data that the tensor-core E-step reads and
+// that are zero (estep_tc.cuh: a tile of up to 48 rows)
+constexpr int kXTailRows = 48;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kTinyAbs = 1.17549435e-38f;  // FLT_MIN: |y| == 0 guard

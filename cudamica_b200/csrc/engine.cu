@@ -63,6 +63,7 @@ cudaError_t launch_preprocess(const float* raw, int64_t T, int n, int do_sphere,
                               float* x, int ldx, int tf32, int* err, cudaStream_t st,
                               long long fault_wait_cycles);
 size_t preprocess_min_ws(int n);
+size_t x_tail_len(int ldx);
 cudaError_t launch_convert_sphered(const double* xs, int64_t T, int n, float* x, int ldx, int tf32,
                                    cudaStream_t st);
 cudaError_t launch_shard_colsum(const float* raw, int64_t T, int n, double* sums, cudaStream_t st);
@@ -487,9 +488,9 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     AL(b.hist, b.hist_cap);
     AL(b.err, 1);
     AL(c->d_keep, T); AL(c->d_Lt, M * T); AL(c->d_P, T);
-    // 3 zero samples past T: the tensor-core form reads the data as rows of up
-    // to 4 samples
-    AL(c->d_x, std::max((size_t)(T + 3) * NP, 2 * preprocess_min_ws((int)n)));   // the sphering's scratch first
+    // zero rows past T: the tensor-core form reads the data as rows of 128 floats
+    // in segments of equal length; the buffer is the sphering's scratch first
+    AL(c->d_x, std::max((size_t)T * NP + x_tail_len(NP), 2 * preprocess_min_ws((int)n)));
     AL(c->d_means, n); AL(c->d_sphere, nn); AL(c->d_cov, nn); AL(c->d_evwork, 4 * nn + 4 * n);
     AL(c->d_ldetS, 1);
     c->backup_len = param_len(c) + (sizeof(Ctrl) + 7) / 8;

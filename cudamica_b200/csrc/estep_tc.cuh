@@ -94,6 +94,13 @@ constexpr int kThreads = TcDef::kThreads;
 constexpr int kCtlRegs = TcDef::kCtlRegs;
 constexpr int kDensRegs = TcDef::kDensRegs;
 constexpr int kSub = TcDef::kSub;
+// A tile's rows come kSegRows at a time from kS / kSegRows segments of the data
+// (tile t: rows t kSegRows .. of every segment), not as one run.  The models of
+// consecutive samples are mostly the same, and a model whose responsibility for
+// a pair of samples is exactly 0 skips its phase 2: with a run per tile one
+// model's CTA did all the work of a tile while the others waited for it at the
+// next exchange; this way every CTA of the cluster has its share in each tile.
+constexpr int kSegRows = 4;
 constexpr int kBcol = 64;               // TMEM column stride of the two b buffers
 constexpr int kPsiCol = 128;            // TMEM column of phi (N = NP columns)
 constexpr int kWloCol = 256;            // TMEM columns of W_lo, the A operand of the low MMA1 half
@@ -155,6 +162,7 @@ enum { BAR_FULL0 = 0, BAR_EMPTY0 = kMaxStages, BAR_BFULL0 = 2 * kMaxStages, BAR_
 struct TcArgs {
     EStepArgs e;
     int ngroups;   // partial slots per cluster: kWG per sample set, set-major
+    int64_t seg_rows;   // rows per segment
 };
 template <int NP, int MM, int R, bool SPLIT, int WG, int NST>
 __global__ void __launch_bounds__(TcCfg<WG, NST>::kThreads, 1)
@@ -269,7 +277,7 @@ __global__ void __launch_bounds__(TcCfg<WG, NST>::kThreads, 1)
     } else {
         // =========================== density warps =================================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDensRegs));
-        const int64_t item_tile0 = cid, item_stride = a.nclusters;
+        const int64_t item_tile0 = cid, item_stride = a.nclusters, seg_rows = ta.seg_rows;
         const int item_slot = cid, item_ngroups = ta.ngroups;
 #include "tc_density_item.inc"
     }
@@ -287,8 +295,9 @@ __global__ void __launch_bounds__(TcCfg<WG, NST>::kThreads, 1)
 inline int tc_np(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : 128); }
 inline int tc_pack(int n) { return 128 / tc_np(n); }
 
-// a.x holds at least ceil(T / R) * R samples of a.ldx = npc floats (samples at
-// and beyond T zero); it is read as ceil(T / R) rows of 128 floats.
+// a.x is read as rows of 128 floats (R samples of a.ldx = npc floats each) in
+// kS / kSegRows segments of ceil(rows / kS) kSegRows rows: up to kXTailRows rows
+// past the data, which are zero.
 template <int NP, int MM, int R, bool SPLIT, int WG, int NST>
 cudaError_t launch_tc(const EStepArgs& a, int nclusters, cudaStream_t st) {
     using Cf = TcCfg<WG, NST>;
@@ -299,12 +308,15 @@ cudaError_t launch_tc(const EStepArgs& a, int nclusters, cudaStream_t st) {
     if (a.ldx * R != NP) return cudaErrorInvalidValue;
     const int64_t rows = (a.T + R - 1) / R;
     if (a.ntiles != (int)((rows + kS - 1) / kS)) return cudaErrorInvalidValue;
+    constexpr int nseg = kS / kSegRows;
+    static_assert(kS % kSegRows == 0 && kS <= kXTailRows, "segments");
+    const int64_t seg_rows = (int64_t)a.ntiles * kSegRows;
     CUtensorMap map;
-    cuuint64_t dims[2] = {(cuuint64_t)NP, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)NP * 4};
-    cuuint32_t box[2] = {32, (cuuint32_t)kS};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)a.x, dims, strides, box, estr,
+    cuuint64_t dims[3] = {(cuuint64_t)NP, (cuuint64_t)seg_rows, (cuuint64_t)nseg};
+    cuuint64_t strides[2] = {(cuuint64_t)NP * 4, (cuuint64_t)seg_rows * NP * 4};
+    cuuint32_t box[3] = {32, (cuuint32_t)kSegRows, (cuuint32_t)nseg};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)a.x, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
@@ -321,6 +333,7 @@ cudaError_t launch_tc(const EStepArgs& a, int nclusters, cudaStream_t st) {
     TcArgs ta;
     ta.e = a;
     ta.ngroups = kWG * R;
+    ta.seg_rows = seg_rows;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nclusters * a.M);
     cfg.blockDim = dim3(kThreads);

@@ -20,6 +20,10 @@
 #include "tc_ptx.cuh"
 
 namespace amica {
+// Zero floats past the T x ldx sphered data: up to three samples that fill the
+// last row of 128 floats, then kXTailRows rows (256 channels: 3 rows for the
+// contraction of the split form).
+size_t x_tail_len(int ldx) { return ldx <= 128 ? 128 + (size_t)kXTailRows * 128 : 3 * (size_t)ldx; }
 // sphere_eig.cu
 cudaError_t launch_eig_cluster(const double* C, double* V, double* evals, int n, int* done, cudaStream_t st);
 }  // namespace amica
@@ -871,7 +875,7 @@ cudaError_t pp_finish(const float* raw, int64_t T, int n, int do_sphere, const d
     }
     k_sphere<<<(n * n + 255) / 256, 256, 0, st>>>(V, ev, var, n, do_sphere, sphere, ldetS_dev);
     // the scratch is done with: the rows past T, which the kernel below leaves out
-    e = cudaMemsetAsync(x + (size_t)T * ldx, 0, sizeof(float) * 3 * ldx, st);
+    e = cudaMemsetAsync(x + (size_t)T * ldx, 0, sizeof(float) * amica::x_tail_len(ldx), st);
     if (e != cudaSuccess) return e;
     const SpherePlan p = sphere_plan(n);
     e = cudaFuncSetAttribute(k_apply_sphere, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
@@ -894,14 +898,14 @@ size_t preprocess_min_ws(int n) {
     return std::max(nn, jac);
 }
 
-// x holds (T + 3) x ldx floats, and at least 2 preprocess_min_ws(n): until the
-// sphered data are written to it, it serves as the scratch; the 3 rows past T
-// are left zero.
+// x holds T x ldx + x_tail_len(ldx) floats, and at least 2 preprocess_min_ws(n):
+// until the sphered data are written to it, it serves as the scratch; the floats
+// past T x ldx are left zero.
 // fault_wait_cycles > 0 arms the test hook of amica_test_arm_wait_fault for
 // this launch (cooperative eigensolver only: block 0 skips its first arrival,
 // every wait is bounded by fault_wait_cycles).
 static Scratch x_scratch(float* x, int64_t T, int n, int ldx) {
-    return Scratch{reinterpret_cast<double*>(x), std::max((size_t)(T + 3) * ldx / 2, preprocess_min_ws(n))};
+    return Scratch{reinterpret_cast<double*>(x), std::max((size_t)T * ldx / 2, preprocess_min_ws(n))};
 }
 cudaError_t launch_preprocess(const float* raw, int64_t T, int n, int do_sphere, double* means,
                               double* cov, double* sphere, double* evwork, double* ldetS_dev,
