@@ -290,6 +290,11 @@ __device__ __forceinline__ float tf32_rna_alu(float x) {
     return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
 
+// Half of TF32's last place added, so that the tensor core, which reads the top
+// 19 bits of an operand, sees the value rounded to nearest, ties away from zero
+// (tf32_rna_alu without clearing the bits that are not read).
+__device__ __forceinline__ float tf32_half_up(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
+
 // The seven per-(channel, mixture) sums A0..A6 of dens_acc mapped to the
 // reference's statistics (usum, kappa num, lambda num, mu num, mu den, beta den,
 // rho num; src/kernels.cu:495-827), with f' = rho p / y:

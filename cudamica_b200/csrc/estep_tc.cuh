@@ -231,6 +231,9 @@ __global__ void __launch_bounds__(TcCfg<WG, NST>::kThreads, 1)
             *reinterpret_cast<float4*>((uint8_t*)Wsm + sw128_off(i, k, 128)) = v;
         }
     }
+    // the b tile's columns of skipped samples must be finite from the start
+    for (uint32_t o = 16u * tid; o < Sh::G_BYTES; o += 16u * kThreads)
+        *reinterpret_cast<float4*>(sm + Sh::OFF_BT + o) = make_float4(0.f, 0.f, 0.f, 0.f);
     if (warp == kDensWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(tmem_holder)), "r"(Sh::TMEM_COLS) : "memory");

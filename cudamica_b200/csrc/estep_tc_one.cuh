@@ -181,11 +181,6 @@ __device__ __forceinline__ void one_control(uint8_t* sm, uint64_t* bar, volatile
     mbar_wait(&bar[ONE_DRAIN], 0u, abort_flag, err, false, false);
 }
 
-// Half of TF32's last place added, so that the tensor core, which reads the top
-// 19 bits of an operand, sees the value rounded to nearest, ties away from zero
-// (tf32_rna_alu without clearing the bits that are not read).
-__device__ __forceinline__ float tf32_half_up(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
