@@ -24,8 +24,8 @@ namespace amica {
 cudaError_t launch_estep_plain(const EStepArgs& a, int NP, int nclusters, cudaStream_t st);
 cudaError_t launch_estep_tc(const EStepArgs& a, int NP, int nclusters, cudaStream_t st, int split, int shape);
 // mstep.cu
-cudaError_t launch_reduce(const double* partial, double* raw, double* stats, int nslots, int M, int n, int m,
-                          int psi_step, int psi_is_phi, cudaStream_t st);
+cudaError_t launch_reduce(const double* partial, double* raw, int nslots, int M, int n, int m, int psi_step,
+                          cudaStream_t st);
 cudaError_t launch_adjoint_dw(const double* raw, const double* A, double* out, int n, int m, int M,
                               cudaStream_t st);
 }
@@ -104,7 +104,7 @@ cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int
                                     int m, int M, const double* A, const double* c,
                                     const double* beta, const double* rho, double* out,
                                     int psi_is_phi, cudaStream_t st) {
-    cudaError_t e = launch_reduce(grad_partial, raw, nullptr, nslots, M, n, m, psi_step, 0, st);
+    cudaError_t e = launch_reduce(grad_partial, raw, nslots, M, n, m, psi_step, st);
     if (e != cudaSuccess) return e;
     const int len = psi_is_phi ? m * n : n * n;
     k_adjoint_finalize<<<dim3((len + 255) / 256, M), 256, 0, st>>>(raw, A, c, beta, rho, out, n, m, M, psi_is_phi);

@@ -37,12 +37,10 @@ struct Ctrl {
     int64_t iter, numdec, nkeep, nrej_total, rej_passes;
     int64_t newton, ll_decreased, no_newt, last_rejected;
     double rej_mean, rej_std;
-    // split correction of phi (tensor-core form): the largest relative change
-    // ||A_new - A|| / ||A|| of this iteration's A update (bits of a
-    // non-negative double, so that an integer max orders them), the M-step
-    // CTAs that have reported it, and the flag the E-step reads
-    uint64_t newton_rel_bits;
-    int64_t reparm_done, phi_split;
+    // CTAs of the two M-step kernels that are done (zero between iterations)
+    int64_t mstep_done, reparm_done;
+    // split correction of phi (tensor-core form): the flag the E-step reads
+    int64_t phi_split;
 };
 
 // One history record per iteration (read back by the host after a run).
@@ -143,7 +141,7 @@ struct MStepBuffers {
     double *A, *Anew, *c, *alpha, *mu, *beta, *rho, *gm, *W, *ldet, *ltc64;
     double *partial, *raw, *stats, *work, *chunk;
     double* gj;        // n > 128: M n^2 working matrices + M n pivot logs of the inverse
-    int64_t* bflag;          // M: Newton-condition violations of the last M-step
+    int64_t* bflag;          // M: Newton-condition violations found so far (zero between M-steps)
     int* use_newton;         // M: 1 Newton step, 0 natural gradient, -1 frozen model (no update)
     float *Wf, *wcf;
     MixParam* mp;

@@ -6,8 +6,8 @@
 //   -> fused E-step (plain FP32 or tcgen05 TF32; above 128 channels the
 //      mixed form is the split one: b = W x as TF32 tensor-core GEMMs, the
 //      density-only E-step, then Psi = sum g x^T as TF32 GEMMs)
-//   -> k_reduce + k_finalize (deterministic FP64 reduction of per-CTA sums)
-//   -> k_mstep_params -> k_ctrl -> k_gemm64 (A update) -> k_reparm
+//   -> k_reduce (deterministic FP64 reduction of per-CTA sums)
+//   -> k_mstep (parameters, control block) -> k_gemm64 (A update) -> k_reparm
 //   (-> k_reject on schedule)
 // with no host synchronisation, so amica_run() replays one captured CUDA graph
 // per iteration.  This replaces runamica()'s iteration body
@@ -83,9 +83,9 @@ cudaError_t launch_adjoint_finalize(const double* grad_partial, double* raw, int
 
 size_t reject_ws_len(int64_t T);
 cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream_t st);
-cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nclusters,
+cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nslots, bool with_cn,
                                    cudaStream_t st);
-cudaError_t launch_mstep(const MStepBuffers& b, const MStepCfgHost& h, const float* P_rel,
+cudaError_t launch_mstep(const MStepBuffers& b, const MStepCfgHost& h, bool cn_from_raw, const float* P_rel,
                          uint8_t* keep, int64_t T, cudaStream_t st);
 cudaError_t launch_reject_now(const MStepBuffers& b, const MStepCfgHost& h, const float* P_rel,
                               uint8_t* keep, int64_t T, cudaStream_t st);
@@ -258,29 +258,33 @@ int x_ready(amica_ctx* c) {
     return AMICA_OK;
 }
 
-int enqueue_estep(amica_ctx* c) {
+// full_stats: the whole statistics vector (an iteration's M-step takes cnew from
+// the raw sums)
+int enqueue_estep(amica_ctx* c, bool full_stats) {
     CK(launch_prep(c->b, c->hc, c->st));
     EStepArgs a = estep_args(c);
     if (c->use_split) TRY(enqueue_split_estep(c, a));
     else if (c->use_tc) CK(launch_estep_tc(a, c->NP, c->nclusters, c->st, c->hc.phi_split, c->tc_shape));
     else CK(launch_estep_plain(a, c->NP, c->nclusters, c->st));
-    CK(launch_reduce_finalize(c->b, c->hc, c->nslots, c->st));
+    CK(launch_reduce_finalize(c->b, c->hc, c->nslots, full_stats, c->st));
     return AMICA_OK;
 }
 
-// Kernels one iteration launches: inverse/derive, E-step, reduce, finalize
-// (+ phi from Psi in the plain form), params, ctrl, A update (when A is
-// updated), reparametrisation, the finiteness check (+ three for rejection when
-// enabled).
+// Kernels one iteration launches: inverse/derive (two above 128 channels), E-step
+// (with phi_split = 2 its second form, which returns at once, too), reduction
+// (+ phi from Psi in the plain form), parameters and control, A update (when A is
+// updated), reparametrisation with the finiteness check (+ three for rejection
+// when enabled).
 int launches_per_iteration(const amica_ctx* c) {
     // the split form adds the W split and its two tensor-core contractions
     const int split = c->use_split ? 3 : 0;
-    return 8 + split + (c->hc.psi_is_phi ? 0 : 1) + (c->hc.update_A ? 1 : 0) + (c->hc.do_reject ? 3 : 0);
+    return 5 + (c->n > 128 ? 1 : 0) + (c->hc.phi_split == 2 ? 1 : 0) + split + (c->hc.psi_is_phi ? 0 : 1) +
+           (c->hc.update_A ? 1 : 0) + (c->hc.do_reject ? 3 : 0);
 }
 
 int enqueue_iteration(amica_ctx* c) {
-    TRY(enqueue_estep(c));
-    CK(launch_mstep(c->b, c->hc, c->d_P, c->d_keep, c->T, c->st));
+    TRY(enqueue_estep(c, false));
+    CK(launch_mstep(c->b, c->hc, true, c->d_P, c->d_keep, c->T, c->st));
     return AMICA_OK;
 }
 
@@ -837,7 +841,7 @@ int amica_estep_stats(amica_ctx* c, double* stats) {
     if (!c) return AMICA_ERR_INVALIDPARAM;
     if (!c->have_x || !c->have_init) return AMICA_ERR_STATE;
     CK(cudaSetDevice(c->dev));
-    TRY(enqueue_estep(c));
+    TRY(enqueue_estep(c, true));
     c->have_estep = true;
     TRY(check_device_error(c));
     if (stats)
@@ -1033,7 +1037,7 @@ int amica_shard_estep(amica_ctx* c, double* d_stats) {
     CK(cudaSetDevice(c->dev));
     TRY(snapshot_params(c, false));
     CK(cudaEventRecord(c->ev0, c->st));
-    TRY(enqueue_estep(c));
+    TRY(enqueue_estep(c, true));
     CK(cudaMemcpyAsync(d_stats, c->b.stats, sizeof(double) * amica_stats_len(c->n, c->M, c->m),
                        cudaMemcpyDeviceToDevice, c->st));
     // stream-ordered: the all-reduce that follows is queued behind it on this
@@ -1057,7 +1061,7 @@ int amica_shard_mstep(amica_ctx* c, const double* d_stats, int64_t nkeep_total, 
     // the M-step normalises by the samples of every shard (LL, gm); the next
     // E-step of this shard counts its own again
     k_set_nkeep<<<1, 1, 0, c->st>>>(c->b.ctrl, nkeep_total);
-    CK(launch_mstep(c->b, c->hc, c->d_P, c->d_keep, c->T, c->st));
+    CK(launch_mstep(c->b, c->hc, false, c->d_P, c->d_keep, c->T, c->st));
     k_set_nkeep<<<1, 1, 0, c->st>>>(c->b.ctrl, c->T);
     CK(cudaEventRecord(c->ev1, c->st));
     CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
@@ -1300,8 +1304,8 @@ static int cohort_capture(amica_cohort* co) {
         for (int s = 0; s < ns; s++) {
             amica_ctx* c = co->subs[s];
             CK(cudaStreamWaitEvent(c->st, co->mid, 0));
-            CK(launch_reduce_finalize(c->b, c->hc, co->nslots[s], c->st));
-            CK(launch_mstep(c->b, c->hc, c->d_P, c->d_keep, c->T, c->st));
+            CK(launch_reduce_finalize(c->b, c->hc, co->nslots[s], false, c->st));
+            CK(launch_mstep(c->b, c->hc, true, c->d_P, c->d_keep, c->T, c->st));
             CK(cudaEventRecord(co->evs[2 * s + 1], c->st));
             CK(cudaStreamWaitEvent(co->st, co->evs[2 * s + 1], 0));
         }

@@ -22,7 +22,7 @@ int plain_max_clusters(int n, int m, int M);
 int plain_tile_samples();
 cudaError_t launch_estep_plain(const EStepArgs& a, int NP, int nclusters, cudaStream_t st);
 cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream_t st);
-cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nclusters,
+cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nslots, bool with_cn,
                                    cudaStream_t st);
 }  // namespace amica
 
@@ -147,7 +147,7 @@ extern "C" int amica_estep_stats_noalloc(const float* x, int64_t ldx, int64_t n,
     a.T = T; a.ldx = (int)ldx; a.n = (int)n; a.M = (int)M; a.m = (int)m;
     a.ntiles = ntiles; a.nclusters = ncl; a.update_rho = (int)update_rho; a.grad_mode = 0;
     if (launch_estep_plain(a, NP, ncl, st) != cudaSuccess) return AMICA_ERR_CUDA;
-    if (launch_reduce_finalize(b, h, ncl * groups, st) != cudaSuccess) return AMICA_ERR_CUDA;
+    if (launch_reduce_finalize(b, h, ncl * groups, true, st) != cudaSuccess) return AMICA_ERR_CUDA;
     int herr = 0;
     if (cudaMemcpyAsync(&herr, b.err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         return AMICA_ERR_CUDA;

@@ -19,21 +19,6 @@ namespace {
 
 constexpr int kT = 256;
 
-__device__ double block_sum(double v, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-    __syncthreads();
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < (int)(blockDim.x / 32); i++) s += sh[i];
-        sh[32] = s;
-    }
-    __syncthreads();
-    return sh[32];
-}
-
 // ---------------------------------------------------------------------------
 // k_inverse_derive: W_h = A_h^{-1}, ldet_h = -log|det A_h| and the FP32 E-step
 // constants, one CTA of 512 threads per model (n <= 128).  Replaces pinv() and
@@ -745,110 +730,148 @@ __global__ void __launch_bounds__(256) k_gemm64(GemmArgs g) {
 }
 
 // Reparametrisation and c update after the A update (src/amica.cu:2367-2512):
-// unit columns of A, mu *= norm, beta /= norm^2, mu -= W_old (cnew - c), c = cnew.
-// One CTA of 1024 threads per model (n <= 256).
-// With phi_split = 2, every CTA also reports ||A_new - A||_F / ||A||_F of its
-// model (frozen models report nothing), and the last CTA to finish switches the
-// split correction of phi on for good once a Newton iteration changed no
+// unit columns of A, mu *= norm, beta /= norm^2, mu -= W_old (cnew - c), c = cnew;
+// and the finiteness check of everything the M-step wrote (the host then rolls
+// the iteration back; the next E-step would otherwise carry NaN into the LL).
+//
+// A CTA of 8 warps owns 8 channels of one model: a warp its column of A (norm,
+// scaled copy) and that channel's mu and beta; the CTA's rows of W (cnew - c) are
+// summed by all its threads, 64 contiguous bytes of W per column.  The last CTA
+// of the grid writes c (which the others read).  Bound by the latency of two
+// passes over a column; with one CTA per model it took 36 us at n = 128 and 72 at
+// n = 256 (and the check was a launch of its own).
+// With phi_split = 2, ||A_new - A||_F / ||A||_F of each model (frozen models report
+// nothing) is summed from the columns in order by the last CTA, which switches
+// the split correction of phi on for good once a Newton iteration changed no
 // model's A by more than phi_split_rel.
-__global__ void __launch_bounds__(1024) k_reparm(int update_A, int do_reparm, double* A,
-                                                 const double* __restrict__ Anew,
-                                                 const double* __restrict__ W, double* c,
-                                                 double* mu, double* beta,
-                                                 const double* __restrict__ work,
-                                                 const int* __restrict__ use_newton, int n, int m,
-                                                 int phi_split, double phi_split_rel, Ctrl* ctrl) {
-    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    auto report = [&](double rel, bool frozen) {
-        if (phi_split != 2 || tid != 0) return;
-        if (!frozen) atomicMax((unsigned long long*)&ctrl->newton_rel_bits,
-                               (unsigned long long)__double_as_longlong(rel));
-        __threadfence();
-        if (atomicAdd((unsigned long long*)&ctrl->reparm_done, 1ull) == (unsigned long long)(gridDim.x - 1)) {
-            __threadfence();
-            const double mx = __longlong_as_double((long long)atomicMax(
-                (unsigned long long*)&ctrl->newton_rel_bits, 0ull));
-            if (update_A && ctrl->newton && mx < phi_split_rel) ctrl->phi_split = 1;
+constexpr int kRepCh = 8;
+struct ReparmArgs {
+    int update_A, do_reparm, n, m, M, phi_split;
+    double phi_split_rel;
+    double *A, *c, *mu, *beta, *work;
+    const double *Anew, *W, *alpha, *rho, *gm;
+    const int* use_newton;
+    Ctrl* ctrl;
+    int* err;
+};
+__global__ void __launch_bounds__(32 * kRepCh) k_reparm(ReparmArgs a) {
+    const int n = a.n, m = a.m, h = blockIdx.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int i0 = kRepCh * blockIdx.x, i = i0 + warp;
+    double* work = a.work + (size_t)h * 4 * n;         // kappa, lambda (read by the A update before): per-column sums
+    const double* cnew = work + 3 * n;
+    const double* ch = a.c + (size_t)h * n;
+    const bool frozen = a.use_newton[h] < 0;           // A, c, mu, beta unchanged
+    bool bad = false;
+    __shared__ double shift_s[8][kRepCh];
+    __shared__ int last_s;
+    const bool full = a.update_A && !frozen && a.do_reparm;
+    if (full) {
+        // shift(i) = sum_k W(i, k) (cnew - c)(k): thread (k % 32, channel)
+        const int ic = tid & (kRepCh - 1);
+        double s = 0.0;
+        if (i0 + ic < n) {
+            const double* Wi = a.W + (size_t)h * n * n + i0 + ic;
+#pragma unroll 4
+            for (int k = tid >> 3; k < n; k += 32) s = fma(Wi[(size_t)k * n], cnew[k] - ch[k], s);
         }
-    };
-    if (use_newton[h] < 0) {                          // frozen model: A, c, mu, beta unchanged
-        report(0.0, true);
-        return;
+        s += __shfl_xor_sync(0xffffffffu, s, 8);
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+        if (lane < kRepCh) shift_s[warp][lane] = s;
     }
-    const double* cnew = work + (size_t)h * 4 * n + 3 * n;
-    double* ch = c + (size_t)h * n;
-    __shared__ double norms[kMaxN], shift[kMaxN], dc[kMaxN];
-    __shared__ double red[2][32];
-    double rel = 0.0;
-    if (update_A) {
-        double* Ah = A + (size_t)h * n * n;
-        const double* An = Anew + (size_t)h * n * n;
-        if (phi_split == 2) {
-            double dd = 0.0, aa = 0.0;
-            for (int e = tid; e < n * n; e += blockDim.x) {
-                const double d = An[e] - Ah[e];
-                dd += d * d;
-                aa += Ah[e] * Ah[e];
+    __syncthreads();
+    if (i < n) {
+        double* Ai = a.A + (size_t)h * n * n + (size_t)i * n;
+        double nrm = 1.0;
+        if (a.update_A && !frozen) {
+            const double* Ani = a.Anew + (size_t)h * n * n + (size_t)i * n;
+            double s = 0.0, dd = 0.0, aa = 0.0;
+            double v[8];                               // n <= 256: the column in registers
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int r = lane + 32 * u;
+                v[u] = 0.0;
+                if (r < n) {
+                    v[u] = Ani[r];
+                    const double o = Ai[r], d = v[u] - o;
+                    s = fma(v[u], v[u], s);
+                    dd = fma(d, d, dd);
+                    aa = fma(o, o, aa);
+                }
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+                dd += __shfl_xor_sync(0xffffffffu, dd, o);
+                aa += __shfl_xor_sync(0xffffffffu, aa, o);
+            }
+            if (a.do_reparm) nrm = sqrt(s);
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int r = lane + 32 * u;
+                if (r < n) {
+                    const double w = a.do_reparm ? v[u] / nrm : v[u];
+                    Ai[r] = w;
+                    bad |= !isfinite(w);
+                }
+            }
+            if (lane == 0) { work[i] = dd; work[n + i] = aa; }
+        } else {
+            for (int r = lane; r < n; r += 32) bad |= !isfinite(Ai[r]);
+        }
+        if (lane < m) {
+            const size_t idx = ((size_t)h * m + lane) * n + i;
+            double mv = a.mu[idx], bv = a.beta[idx];
+            if (full) {
+                double shift = 0.0;
+#pragma unroll
+                for (int w = 0; w < 8; w++) shift += shift_s[w][warp];
+                mv = mv * nrm - shift;
+                bv /= nrm * nrm;
+                a.mu[idx] = mv;
+                a.beta[idx] = bv;
+            }
+            bad |= !isfinite(mv) || !isfinite(bv) || !isfinite(a.alpha[idx]) || !isfinite(a.rho[idx]);
+        }
+        if (lane == 0) bad |= !isfinite(frozen ? ch[i] : cnew[i]);
+    }
+    if (blockIdx.x == 0 && tid == 0) bad |= !isfinite(a.gm[h]);
+    if (__syncthreads_or(bad) && tid == 0) atomicOr(a.err, kErrNonFinite);
+    // ---- the last CTA: c, and the relative change of A
+    if (tid == 0) {
+        __threadfence();
+        last_s = atomicAdd((unsigned long long*)&a.ctrl->reparm_done, 1ull) ==
+                 (unsigned long long)gridDim.x * gridDim.y - 1;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    double mx = 0.0;
+    for (int q = 0; q < a.M; q++) {
+        if (a.use_newton[q] < 0) continue;
+        const double* wq = a.work + (size_t)q * 4 * n;
+        for (int r = tid; r < n; r += blockDim.x) a.c[(size_t)q * n + r] = wq[3 * n + r];   // src/amica.cu:2456-2462
+        if (a.phi_split == 2 && a.update_A && warp == 0) {
+            double dd = 0.0, aa = 0.0;
+            for (int r = lane; r < n; r += 32) { dd += __ldcg(wq + r); aa += __ldcg(wq + n + r); }
             for (int o = 16; o > 0; o >>= 1) {
                 dd += __shfl_xor_sync(0xffffffffu, dd, o);
                 aa += __shfl_xor_sync(0xffffffffu, aa, o);
             }
-            if (lane == 0) { red[0][warp] = dd; red[1][warp] = aa; }
-            __syncthreads();
-            if (tid == 0) {
-                double sd = 0.0, sa = 0.0;
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) { sd += red[0][w]; sa += red[1][w]; }
-                rel = sa > 0.0 ? sqrt(sd / sa) : 0.0;
-            }
-            __syncthreads();
+            if (aa > 0.0) mx = fmax(mx, sqrt(dd / aa));
         }
-        if (do_reparm) {
-            for (int cc = warp; cc < n; cc += 32) {
-                double s = 0.0;
-                for (int r = lane; r < n; r += 32) s += An[(size_t)cc * n + r] * An[(size_t)cc * n + r];
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (lane == 0) norms[cc] = sqrt(s);
-            }
-            if (tid < n) dc[tid] = cnew[tid] - ch[tid];
-            __syncthreads();
-            for (int ib = 0; ib < n; ib += 128) {
-                const int i = ib + (tid >> 3), part = tid & 7;
-                const double* Wh = W + (size_t)h * n * n;
-                double acc = 0.0;
-                if (i < n)
-                    for (int k = part; k < n; k += 8) acc += Wh[(size_t)k * n + i] * dc[k];
-                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-                if (part == 0 && i < n) shift[i] = acc;
-            }
-            __syncthreads();
-            for (int cc = tid >> 7; cc < n; cc += 8)
-                for (int r = tid & 127; r < n; r += 128)
-                    Ah[(size_t)cc * n + r] = An[(size_t)cc * n + r] / norms[cc];
-            for (int e = tid; e < m * n; e += blockDim.x) {
-                const int i = e % n;
-                const size_t idx = (size_t)h * m * n + e;
-                double mv = mu[idx] * norms[i];
-                beta[idx] /= (norms[i] * norms[i]);
-                mu[idx] = mv - shift[i];
-            }
-        } else {
-            for (int e = tid; e < n * n; e += blockDim.x) Ah[e] = An[e];
-        }
-        __syncthreads();
     }
-    for (int i = tid; i < n; i += blockDim.x) ch[i] = cnew[i];   // src/amica.cu:2456-2462
-    report(rel, false);
+    if (tid == 0 && a.phi_split == 2 && a.update_A && a.ctrl->newton && mx < a.phi_split_rel) a.ctrl->phi_split = 1;
 }
 
 // ---------------------------------------------------------------------------
 // k_reduce: raw[h][e] = sum over slots of partial[q][h][e], fixed order.  The
 // n x n block is carried only by every psi_step-th slot (the tensor-core E-step
 // keeps phi in one slot per cluster); when it already is phi it also goes
-// straight into the statistics vector.  Replaces the block/device reductions of
-// src/amica.cu:1618-1920.
+// straight into the statistics vector (oracle layout), as do the entries that a
+// factor finishes: kappa * beta (src/kernels.cu:616), mu_denom * sqrt(beta) (:745)
+// and rho * beta_denom (:748-750).  cnew is a product with A (finish_cn).  Replaces
+// the block/device reductions of src/amica.cu:1618-1920.
 //
 // A CTA owns 32 consecutive entries; warp w adds slots w, w + nwarps, ... (one
 // 256-byte row of each) and the warps' sums are added in order.  Bound by the
@@ -856,8 +879,13 @@ __global__ void __launch_bounds__(1024) k_reparm(int update_A, int do_reparm, do
 // one thread per entry the 1776 slots of a 32-channel fit took 259 us, and the
 // 888 of a 64-channel one 133 us.
 constexpr int kReduceMaxWarps = 32;
+struct ReduceStats {             // stats null: raw sums only
+    double* stats;
+    const double *beta, *rho, *ltc64;
+    const Ctrl* ctrl;
+};
 __global__ void __launch_bounds__(32 * kReduceMaxWarps) k_reduce(
-    const double* __restrict__ partial, double* __restrict__ raw, double* __restrict__ stats, int nslots,
+    const double* __restrict__ partial, double* __restrict__ raw, ReduceStats rs, int nslots,
     int M, int n, int m, int psi_step, int psi_is_phi) {
     __shared__ double sh[kReduceMaxWarps][32];
     PartLayout PL{n, m};
@@ -881,45 +909,58 @@ __global__ void __launch_bounds__(32 * kReduceMaxWarps) k_reduce(
     if (warp != 0 || e >= total) return;
     for (int w = 1; w < nw; w++) s += sh[w][lane];
     raw[e] = s;
-    if (in_psi && psi_is_phi) stats[SL.base(h) + SL.phi() + (off - psi0)] = s;
+    if (!rs.stats) return;
+    double* S = rs.stats + SL.base(h);
+    if (in_psi) {
+        if (psi_is_phi) S[SL.phi() + (off - psi0)] = s;
+    } else if (off >= PL.mix(0)) {
+        const int k = (off - PL.mix(0)) / (m * n), q = off - PL.mix(k);
+        const size_t idx = (size_t)h * m * n + q;
+        if (k == kKn) s *= rs.beta[idx];
+        else if (k == kMd) s *= sqrt(rs.beta[idx]);
+        else if (k == kBd) s *= rs.rho[idx] > 2.0 ? rs.rho[idx] : 1.0;
+        S[SL.mix(k) + q] = s;
+    } else if (off >= PL.s2() && off < PL.gs()) {
+        S[SL.s2() + (off - PL.s2())] = s;
+    } else if (off == 1) {
+        S[SL.vs()] = s;
+    } else if (off == 0 && h == 0) {
+        rs.stats[0] = s + (double)rs.ctrl->nkeep * rs.ltc64[0];
+    }
 }
 
-// ---------------------------------------------------------------------------
-// k_finalize: raw per-model sums -> the flat statistics vector (oracle layout):
-// phi = (Psi - gsum c^T) W^T, and the per-block factors of src/kernels.cu:616
-// (kappa * beta), :745 (mu_denom * sqrt(beta)), :748-750 (rho * beta_denom).
-__global__ void __launch_bounds__(kT) k_finalize(
-    const double* __restrict__ raw, const double* __restrict__ W, const double* __restrict__ A,
-    const double* __restrict__ c,
-    const double* __restrict__ beta, const double* __restrict__ rho,
-    const double* __restrict__ ltc64, const Ctrl* __restrict__ ctrl, double* __restrict__ stats,
-    int n, int m, int psi_is_phi) {
-    const int h = blockIdx.x, tid = threadIdx.x;
+// cnew's numerator sum_t v x_i = (A sum_t v b)_i + vsum c_i (x - c = A b) for channel
+// i = i0 + (thread % 32) of model h: the CTA's warps (of 256 or 1024 threads) share
+// the columns of A; the result in warp 0.  sh: 32 x 32 doubles.
+__device__ __forceinline__ double finish_cn(const double* __restrict__ R, const double* __restrict__ Ah,
+                                            const double* __restrict__ c, int h, int n, int m, int i0,
+                                            double (*sh)[32]) {
+    PartLayout PL{n, m};
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int i = i0 + lane;
+    double s = 0.0;
+    if (i < n) {
+#pragma unroll 4
+        for (int k = warp; k < n; k += nw) s = fma(Ah[(size_t)k * n + i], R[PL.cn() + k], s);
+    }
+    __syncthreads();
+    sh[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < n) {
+        s = R[1] * c[(size_t)h * n + i];
+        for (int w = 0; w < nw; w++) s += sh[w][lane];
+    }
+    return s;
+}
+// the statistics' cnew entries; blockIdx = (32-channel block, model)
+__global__ void __launch_bounds__(kT) k_cn(const double* __restrict__ raw, const double* __restrict__ A,
+                                           const double* __restrict__ c, double* __restrict__ stats, int n, int m) {
+    __shared__ double sh[kT / 32][32];
+    const int h = blockIdx.y, i = 32 * blockIdx.x + threadIdx.x;
     PartLayout PL{n, m};
     StatLayout SL{n, m};
-    const double* R = raw + (size_t)h * PL.stride();
-    double* S = stats + SL.base(h);
-    if (h == 0 && tid == 0) stats[0] = R[0] + (double)ctrl->nkeep * ltc64[0];
-    if (tid == 0) S[SL.vs()] = R[1];
-    const double* Ah = A + (size_t)h * n * n;
-    for (int i = tid; i < n; i += kT) {
-        // sum_t v x_i = (A sum_t v b)_i + vsum c_i, since x - c = A b
-        double acc = R[1] * c[(size_t)h * n + i];
-        for (int k = 0; k < n; k++) acc += Ah[(size_t)k * n + i] * R[PL.cn() + k];
-        S[SL.cn() + i] = acc;
-        S[SL.s2() + i] = R[PL.s2() + i];
-    }
-    for (int e = tid; e < m * n; e += kT) {
-        const size_t idx = (size_t)h * m * n + e;
-        const double bt = beta[idx], r = rho[idx];
-        S[SL.mix(kUs) + e] = R[PL.mix(kUs) + e];
-        S[SL.mix(kKn) + e] = R[PL.mix(kKn) + e] * bt;
-        S[SL.mix(kLn) + e] = R[PL.mix(kLn) + e];
-        S[SL.mix(kMn) + e] = R[PL.mix(kMn) + e];
-        S[SL.mix(kMd) + e] = R[PL.mix(kMd) + e] * sqrt(bt);
-        S[SL.mix(kBd) + e] = R[PL.mix(kBd) + e] * (r > 2.0 ? r : 1.0);
-        S[SL.mix(kRn) + e] = R[PL.mix(kRn) + e];
-    }
+    const double s = finish_cn(raw + (size_t)h * PL.stride(), A + (size_t)h * n * n, c, h, n, m, 32 * blockIdx.x, sh);
+    if (threadIdx.x < 32 && i < n) stats[SL.base(h) + SL.cn() + i] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -947,95 +988,10 @@ __device__ double psi_series(double x) {
     return r;
 }
 
-// Per-model parameter updates (src/amica.cu:1995-2154) and the Newton
-// condition bflag (src/amica.cu:2155-2230).  One CTA of 1024 threads per model;
-// kappa, lambda, sigma2 and cnew go to `work` for the A update.
-constexpr int kMT = 1024;
-__global__ void __launch_bounds__(kMT) k_mstep_params(
-    MCfg cf, const double* __restrict__ stats, Ctrl* ctrl, double* gm, double* alpha, double* mu,
-    double* beta, double* rho, double* work, int64_t* bflag, int* use_newton) {
-    const int h = blockIdx.x, tid = threadIdx.x;
-    const int n = cf.n, m = cf.m, mn = m * n;
-    StatLayout SL{n, m};
-    const double* S = stats + SL.base(h);
-    const int64_t iter = ctrl->iter + 1;
-    const double Tk = (double)ctrl->nkeep;
-    double* kappa = work + (size_t)h * 4 * n;
-    double* lambda = kappa + n;
-    double* sig2 = kappa + 2 * n;
-    double* cnew = kappa + 3 * n;
-    __shared__ double sh[33];
-    __shared__ double ks[kMaxN];
-    const double vsum = S[SL.vs()];
-    const double ivs = 1.0 / vsum;
-    if (!(vsum >= kMinModelVsum)) {                   // a model that explains no data: frozen
-        if (tid == 0) {
-            if (cf.update_gm) gm[h] = fmax(vsum / Tk, kMinGm);
-            bflag[h] = 0;
-            use_newton[h] = -1;
-        }
-        return;
-    }
-    if (tid == 0 && cf.update_gm) gm[h] = vsum / Tk;
-    if (tid == 0 && !cf.update_A) use_newton[h] = 0;
-    // alpha = usum / vsum; then kappa / lambda with the new alpha and old mu
-    for (int i = tid; i < n; i += kMT) {
-        const double s2 = S[SL.s2() + i] * ivs;
-        sig2[i] = s2;
-        cnew[i] = S[SL.cn() + i] * ivs;
-        double kap = 0.0, lam = 0.0;
-        for (int j = 0; j < m; j++) {
-            const int mi = j * n + i;
-            const size_t idx = (size_t)h * mn + mi;
-            const double us = S[SL.mix(kUs) + mi];
-            if (cf.update_alpha) alpha[idx] = us * ivs;
-            if (!(us > 0.0)) continue;                // a component with no responsibility
-            const double dk = S[SL.mix(kKn) + mi] / us;
-            const double a = alpha[idx];
-            kap += dk * a;
-            const double muv = mu[idx];
-            lam += (muv * muv * dk + S[SL.mix(kLn) + mi] / us) * a;
-        }
-        kappa[i] = kap;
-        lambda[i] = lam;
-        ks[i] = kap * s2;
-    }
-    __syncthreads();
-    for (int mi = tid; mi < mn; mi += kMT) {
-        const size_t idx = (size_t)h * mn + mi;
-        if (!(S[SL.mix(kUs) + mi] > 0.0)) continue;  // no responsibility: mu, beta, rho kept
-        if (cf.update_mu) mu[idx] += S[SL.mix(kMn) + mi] / S[SL.mix(kMd) + mi];
-        if (cf.update_beta) {
-            const double bnum = (rho[idx] > 2.0) ? 0.0 : S[SL.mix(kUs) + mi];
-            beta[idx] *= bnum / S[SL.mix(kBd) + mi];
-        }
-        if (cf.update_rho && iter >= cf.rho_start_iter) {
-            double r = rho[idx];
-            const double ps = psi_series(1.0 + 1.0 / r);
-            const double d = 1.0 - (r / ps) * S[SL.mix(kRn) + mi] / S[SL.mix(kUs) + mi];
-            r = r + cf.rholrate * d;
-            if (r > cf.rhomax) r = cf.rhomax;
-            else if (r < cf.rhomin) r = cf.rhomin;
-            rho[idx] = r;
-        }
-    }
-    if (!cf.update_A) return;
-    // bflag: entries of (kappa sigma2)(kappa sigma2)^T that are <= 1, diagonal included
-    double cnt = 0.0;
-    for (int r = tid & 127; r < n; r += 128)
-        for (int cc = tid >> 7; cc < n; cc += kMT / 128)
-            if (ks[r] * ks[cc] <= 1.0) cnt += 1.0;
-    cnt = block_sum(cnt, sh);
-    const int64_t bf = (int64_t)cnt;
-    const int newton = (bf == 0 && cf.do_newton && iter >= cf.newt_start_iter);
-    if (tid == 0) { bflag[h] = bf; use_newton[h] = newton; }
-}
-
 // LL bookkeeping and the learning-rate schedule (src/amica.cu:1981-1993,
-// :2281-2285).  One thread.
-__global__ void k_ctrl(MCfg cf, const double* __restrict__ stats, Ctrl* ctrl,
-                       const int64_t* __restrict__ bflag, IterRec* hist, int64_t hist_cap) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// :2281-2285).  One thread; no_newt: some model fails the Newton condition.
+__device__ void update_ctrl(const MCfg& cf, const double* __restrict__ stats, Ctrl* ctrl, int no_newt,
+                            IterRec* hist, int64_t hist_cap) {
     Ctrl c = *ctrl;
     const int64_t iter = c.iter + 1;
     const double ll = stats[0] / ((double)cf.n * (double)c.nkeep);
@@ -1054,8 +1010,6 @@ __global__ void k_ctrl(MCfg cf, const double* __restrict__ stats, Ctrl* ctrl,
     c.ll_prev = ll;
     c.newton = 0;
     if (cf.update_A) {
-        int no_newt = 0;
-        for (int h = 0; h < cf.M; h++) no_newt |= (bflag[h] > 0);
         const double step = c.lrate < 0.1 ? c.lrate : 0.1;
         if (iter >= cf.newt_start_iter && cf.do_newton && !no_newt) {
             c.lrate = fmin(cf.lratemax, c.lrate + step);
@@ -1067,8 +1021,7 @@ __global__ void k_ctrl(MCfg cf, const double* __restrict__ stats, Ctrl* ctrl,
     }
     c.iter = iter;
     c.last_rejected = 0;
-    // the A update of this iteration reports its relative change (k_reparm)
-    c.newton_rel_bits = 0;
+    c.mstep_done = 0;
     c.reparm_done = 0;
     if (cf.phi_split != 2) c.phi_split = cf.phi_split;
     *ctrl = c;
@@ -1084,6 +1037,107 @@ __global__ void k_ctrl(MCfg cf, const double* __restrict__ stats, Ctrl* ctrl,
         r.phi_split = c.phi_split;          // the form this iteration's E-step ran
         hist[iter - 1] = r;
     }
+}
+
+// Parameter updates (src/amica.cu:1995-2154), the Newton condition
+// (src/amica.cu:2155-2230) and the control block.  A CTA owns 32 channels of one
+// model: lane = channel, warp = mixture; kappa, lambda, sigma2 and cnew go to
+// `work` for the A update.  Everything is per channel but the Newton condition:
+// (kappa sigma2)(kappa sigma2)^T has an entry <= 1 iff some kappa sigma2 (they are
+// not negative) is <= 1 itself, the diagonal being part of it.  The last CTA of
+// the grid combines the channels' findings and advances the control block.
+// Bound by the latency of one chain of loads, divisions and a digamma; with one
+// CTA per model walking all channels and the n^2 products, and the control block
+// in a launch of its own, the two took 16 us at n = 32 and 17 at n = 128.
+// raw not null: cnew's numerator comes from the E-step's raw sums (finish_cn), the
+// statistics' own entries for it are not read.
+constexpr int kMT = 256;
+__global__ void __launch_bounds__(kMT) k_mstep(
+    MCfg cf, const double* __restrict__ stats, const double* __restrict__ raw, const double* __restrict__ A,
+    const double* __restrict__ c, Ctrl* ctrl, double* gm, double* alpha, double* mu, double* beta, double* rho,
+    double* work, int64_t* bflag, int* use_newton, IterRec* hist, int64_t hist_cap) {
+    __shared__ double sh[kMT / 32][32], kap_s[5][32], lam_s[5][32];
+    __shared__ int last_s;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, j = tid >> 5;
+    const int n = cf.n, m = cf.m, mn = m * n;
+    const int i = 32 * blockIdx.x + lane;
+    StatLayout SL{n, m};
+    PartLayout PL{n, m};
+    const double* S = stats + SL.base(h);
+    const int64_t iter = ctrl->iter + 1;
+    const double Tk = (double)ctrl->nkeep;
+    const double vsum = S[SL.vs()];
+    const double ivs = 1.0 / vsum;
+    const bool frozen = !(vsum >= kMinModelVsum);      // a model that explains no data
+    if (blockIdx.x == 0 && tid == 0 && cf.update_gm) gm[h] = frozen ? fmax(vsum / Tk, kMinGm) : vsum / Tk;
+    if (!frozen) {
+        double* kappa = work + (size_t)h * 4 * n;
+        double cn = 0.0;
+        if (raw) cn = finish_cn(raw + (size_t)h * PL.stride(), A + (size_t)h * n * n, c, h, n, m, 32 * blockIdx.x, sh);
+        if (j < m) {
+            double kap = 0.0, lam = 0.0;
+            if (i < n) {
+                const int mi = j * n + i;
+                const size_t idx = (size_t)h * mn + mi;
+                const double us = S[SL.mix(kUs) + mi], kn = S[SL.mix(kKn) + mi], ln = S[SL.mix(kLn) + mi];
+                const double muv = mu[idx], bv = beta[idx], rv = rho[idx];
+                // alpha = usum / vsum; kappa / lambda with the new alpha and old mu
+                const double al = cf.update_alpha ? us * ivs : alpha[idx];
+                if (cf.update_alpha) alpha[idx] = al;
+                if (us > 0.0) {                        // else a component with no responsibility: mu, beta, rho kept
+                    const double dk = kn / us;
+                    kap = dk * al;
+                    lam = (muv * muv * dk + ln / us) * al;
+                    if (cf.update_mu) mu[idx] = muv + S[SL.mix(kMn) + mi] / S[SL.mix(kMd) + mi];
+                    if (cf.update_beta) beta[idx] = bv * ((rv > 2.0 ? 0.0 : us) / S[SL.mix(kBd) + mi]);
+                    if (cf.update_rho && iter >= cf.rho_start_iter) {
+                        const double ps = psi_series(1.0 + 1.0 / rv);
+                        const double d = 1.0 - (rv / ps) * S[SL.mix(kRn) + mi] / us;
+                        double r = rv + cf.rholrate * d;
+                        if (r > cf.rhomax) r = cf.rhomax;
+                        else if (r < cf.rhomin) r = cf.rhomin;
+                        rho[idx] = r;
+                    }
+                }
+            }
+            kap_s[j][lane] = kap;
+            lam_s[j][lane] = lam;
+        }
+        __syncthreads();
+        if (j == 0) {
+            bool low = false;
+            if (i < n) {
+                const double s2 = S[SL.s2() + i] * ivs;
+                if (!raw) cn = S[SL.cn() + i];
+                double kap = 0.0, lam = 0.0;
+                for (int q = 0; q < m; q++) { kap += kap_s[q][lane]; lam += lam_s[q][lane]; }
+                kappa[i] = kap;
+                kappa[n + i] = lam;
+                kappa[2 * n + i] = s2;
+                kappa[3 * n + i] = cn * ivs;
+                low = kap * s2 <= 1.0;
+            }
+            if (__any_sync(0xffffffffu, low) && lane == 0)
+                atomicOr((unsigned long long*)&bflag[h], 1ull);
+        }
+    }
+    // ---- the last CTA
+    __threadfence();
+    __syncthreads();
+    if (tid == 0)
+        last_s = atomicAdd((unsigned long long*)&ctrl->mstep_done, 1ull) ==
+                 (unsigned long long)gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (!last_s || tid != 0) return;
+    __threadfence();
+    int no_newt = 0;
+    for (int q = 0; q < cf.M; q++) {
+        const bool fz = !(stats[SL.base(q) + SL.vs()] >= kMinModelVsum);
+        const int low = (int)atomicExch((unsigned long long*)&bflag[q], 0ull);   // zero for the next iteration
+        no_newt |= low;
+        use_newton[q] = fz ? -1 : cf.update_A && !low && cf.do_newton && iter >= cf.newt_start_iter;
+    }
+    update_ctrl(cf, stats, ctrl, no_newt, hist, hist_cap);
 }
 
 // Rejection pass (engine-defined; the reference has none): over kept samples,
@@ -1280,28 +1334,36 @@ cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream
     return cudaGetLastError();
 }
 
-// stats receives the n x n block when psi_is_phi (else it may be null).  Warps
-// per CTA: about 16 slots each, so that a warp's loop is two batches of eight
+// Warps per CTA: about 16 slots each, so that a warp's loop is two batches of eight
 // independent loads (4 warps at the least, to fill the SMs' load queues).
-cudaError_t launch_reduce(const double* partial, double* raw, double* stats, int nslots, int M, int n, int m,
-                          int psi_step, int psi_is_phi, cudaStream_t st) {
+static cudaError_t reduce_slots(const double* partial, double* raw, const ReduceStats& rs, int nslots, int M, int n,
+                                int m, int psi_step, int psi_is_phi, cudaStream_t st) {
     PartLayout PL{n, m};
     const int64_t total = (int64_t)M * PL.stride();
     int nw = 4;
     while (nw < kReduceMaxWarps && nw * 16 < nslots) nw *= 2;
-    k_reduce<<<(unsigned)((total + 31) / 32), 32 * nw, 0, st>>>(partial, raw, stats, nslots, M, n, m, psi_step,
+    k_reduce<<<(unsigned)((total + 31) / 32), 32 * nw, 0, st>>>(partial, raw, rs, nslots, M, n, m, psi_step,
                                                                 psi_is_phi);
     return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nclusters,
+// the slot sums alone (adjoint.cu)
+cudaError_t launch_reduce(const double* partial, double* raw, int nslots, int M, int n, int m, int psi_step,
+                          cudaStream_t st) {
+    return reduce_slots(partial, raw, ReduceStats{}, nslots, M, n, m, psi_step, 0, st);
+}
+
+// The statistics from the partial slots.  with_cn = false leaves their cnew
+// entries to launch_mstep(cn_from_raw).
+cudaError_t launch_reduce_finalize(const MStepBuffers& b, const MStepCfgHost& h, int nslots, bool with_cn,
                                    cudaStream_t st) {
     PartLayout PL{h.n, h.m};
     StatLayout SL{h.n, h.m};
-    launch_reduce(b.partial, b.raw, b.stats, nclusters, h.M, h.n, h.m, h.psi_step > 0 ? h.psi_step : 1,
-                  h.psi_is_phi, st);
-    k_finalize<<<h.M, kT, 0, st>>>(b.raw, b.W, b.A, b.c, b.beta, b.rho, b.ltc64, b.ctrl, b.stats,
-                                   h.n, h.m, h.psi_is_phi);
+    const ReduceStats rs{b.stats, b.beta, b.rho, b.ltc64, b.ctrl};
+    cudaError_t e = reduce_slots(b.partial, b.raw, rs, nslots, h.M, h.n, h.m, h.psi_step > 0 ? h.psi_step : 1,
+                                 h.psi_is_phi, st);
+    if (e != cudaSuccess) return e;
+    if (with_cn) k_cn<<<dim3((h.n + 31) / 32, h.M), kT, 0, st>>>(b.raw, b.A, b.c, b.stats, h.n, h.m);
     if (!h.psi_is_phi) {
         dim3 g((h.n + 31) / 32, (h.n + 31) / 32, h.M);
         GemmArgs ga{};
@@ -1331,30 +1393,13 @@ cudaError_t launch_adjoint_dw(const double* raw, const double* A, double* out, i
     return cudaGetLastError();
 }
 
-// Flags a non-finite parameter after the M-step, so that the host rolls the
-// iteration back (the next E-step would otherwise carry NaN into the LL).
-__global__ void k_check_finite(const double* __restrict__ A, const double* __restrict__ c,
-                               const double* __restrict__ alpha, const double* __restrict__ mu,
-                               const double* __restrict__ beta, const double* __restrict__ rho,
-                               const double* __restrict__ gm, int64_t nA, int64_t nc, int64_t nmix,
-                               int M, int* err) {
-    bool bad = false;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    for (int64_t e = t0; e < nA; e += stride) bad |= !isfinite(A[e]);
-    for (int64_t e = t0; e < nc; e += stride) bad |= !isfinite(c[e]);
-    for (int64_t e = t0; e < nmix; e += stride)
-        bad |= !isfinite(alpha[e]) || !isfinite(mu[e]) || !isfinite(beta[e]) || !isfinite(rho[e]);
-    for (int64_t e = t0; e < M; e += stride) bad |= !isfinite(gm[e]);
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(err, kErrNonFinite);
-}
-
-cudaError_t launch_mstep(const MStepBuffers& b, const MStepCfgHost& h, const float* P_rel,
+// The M-step from b.stats; cn_from_raw: cnew's numerator from b.raw instead.
+cudaError_t launch_mstep(const MStepBuffers& b, const MStepCfgHost& h, bool cn_from_raw, const float* P_rel,
                          uint8_t* keep, int64_t T, cudaStream_t st) {
     const MCfg cf = to_mcfg(h);
-    k_mstep_params<<<h.M, kMT, 0, st>>>(cf, b.stats, b.ctrl, b.gm, b.alpha, b.mu, b.beta, b.rho,
-                                        b.work, b.bflag, b.use_newton);
-    k_ctrl<<<1, 32, 0, st>>>(cf, b.stats, b.ctrl, b.bflag, b.hist, b.hist_cap);
+    k_mstep<<<dim3((h.n + 31) / 32, h.M), kMT, 0, st>>>(cf, b.stats, cn_from_raw ? b.raw : nullptr, b.A, b.c, b.ctrl,
+                                                        b.gm, b.alpha, b.mu, b.beta, b.rho, b.work, b.bflag,
+                                                        b.use_newton, b.hist, b.hist_cap);
     if (h.update_A) {
         dim3 g((h.n + 31) / 32, (h.n + 31) / 32, h.M);
         GemmArgs ga{};
@@ -1365,14 +1410,9 @@ cudaError_t launch_mstep(const MStepBuffers& b, const MStepCfgHost& h, const flo
         ga.stats = b.stats; ga.work = b.work;
         k_gemm64<<<g, 256, 0, st>>>(ga);
     }
-    k_reparm<<<h.M, 1024, 0, st>>>(h.update_A, h.do_reparm, b.A, b.Anew, b.W, b.c, b.mu, b.beta,
-                                  b.work, b.use_newton, h.n, h.m, h.phi_split, h.phi_split_rel, b.ctrl);
-    {
-        const int64_t nA = (int64_t)h.M * h.n * h.n, nmix = (int64_t)h.M * h.m * h.n;
-        const int grid = (int)std::min<int64_t>((nA + 255) / 256, 148);
-        k_check_finite<<<grid, 256, 0, st>>>(b.A, b.c, b.alpha, b.mu, b.beta, b.rho, b.gm, nA,
-                                             (int64_t)h.M * h.n, nmix, h.M, b.err);
-    }
+    ReparmArgs ra{h.update_A, h.do_reparm, h.n, h.m, h.M, h.phi_split, h.phi_split_rel,
+                  b.A, b.c, b.mu, b.beta, b.work, b.Anew, b.W, b.alpha, b.rho, b.gm, b.use_newton, b.ctrl, b.err};
+    k_reparm<<<dim3((h.n + kRepCh - 1) / kRepCh, h.M), 32 * kRepCh, 0, st>>>(ra);
     if (h.do_reject && P_rel && keep)
         reject_pass(cf, b.ctrl, P_rel, keep, T, b.chunk, b.hist, b.hist_cap, 0, st);
     return cudaGetLastError();
