@@ -93,6 +93,13 @@ cudaError_t launch_reject_now(const MStepBuffers& b, const MStepCfgHost& h, cons
 
 using namespace amica;
 
+// What the host reads after an iteration, in one piece of device memory.
+struct Status {
+    Ctrl ctrl;
+    int64_t err;       // the kernels' error bits (an int)
+    double ldetS;
+};
+
 struct amica_ctx {
     amica_cfg cfg{};
     int dev = 0;
@@ -117,7 +124,7 @@ struct amica_ctx {
     float* d_rawx = nullptr;     // T x n raw input (float)
     float* d_x = nullptr;        // T x NP sphered (float)
     double *d_means = nullptr, *d_sphere = nullptr, *d_cov = nullptr, *d_evwork = nullptr,
-           *d_ldetS = nullptr;
+           *d_ldetS = nullptr;   // d_ldetS in *d_status
     double ldetS = 0.0;
     std::vector<double> h_means, h_sphere;
 
@@ -125,14 +132,23 @@ struct amica_ctx {
     MStepCfgHost hc{};
     uint8_t* d_keep = nullptr;
     float *d_Lt = nullptr, *d_P = nullptr;
-    double* d_backup = nullptr;   // parameter snapshot for NaN rollback
-    size_t backup_len = 0;
+    // A, c, alpha, mu, beta, rho, gm (param_len doubles), *d_status, W: one block, so
+    // that a snapshot for the NaN rollback (parameters and ctrl), and parameters
+    // in and out, are one copy each
+    double* d_block = nullptr;
+    Status* d_status = nullptr;
+    double* d_backup = nullptr;
+    size_t backup_len = 0;        // bytes
+    int64_t iter = 0;             // ctrl->iter as of the last call
+    double* h_stage = nullptr;    // pinned: the block's parameters, and W
+    bool stage_busy = false;      // a copy out of h_stage may be in flight
+    IterRec* h_recs = nullptr;    // pinned: kPinnedRecs history records, then a single one
     double* d_gradp = nullptr;    // adjoint partials
     double* d_grad = nullptr;
 
-    Ctrl* h_ctrl = nullptr;       // pinned
+    Status* h_status = nullptr;   // pinned
+    Ctrl* h_ctrl = nullptr;       // its ctrl
     long long fault_wait_cycles = 0;   // amica_test_arm_wait_fault: armed for the next preprocess
-    int* h_err = nullptr;         // pinned
     std::vector<IterRec> hist;    // host copy of the iteration history
 
     cudaGraphExec_t graph = nullptr;
@@ -188,20 +204,19 @@ int64_t param_len(const amica_ctx* c) {
     return M * n * n + M * n + 4 * M * m * n + M;
 }
 
+constexpr int64_t kPinnedRecs = 256;
+
+// parameters and control block, to or from the backup
 int snapshot_params(amica_ctx* c, bool restore) {
-    const int64_t n = c->n, M = c->M, m = c->m;
-    double* p = c->d_backup;
-    struct Seg { double* d; int64_t len; } segs[] = {
-        {c->b.A, M * n * n}, {c->b.c, M * n}, {c->b.alpha, M * m * n}, {c->b.mu, M * m * n},
-        {c->b.beta, M * m * n}, {c->b.rho, M * m * n}, {c->b.gm, M}};
-    for (auto& s : segs) {
-        if (restore) CK(cudaMemcpyAsync(s.d, p, sizeof(double) * s.len, cudaMemcpyDeviceToDevice, c->st));
-        else CK(cudaMemcpyAsync(p, s.d, sizeof(double) * s.len, cudaMemcpyDeviceToDevice, c->st));
-        p += s.len;
-    }
-    Ctrl* cb = reinterpret_cast<Ctrl*>(p);
-    if (restore) CK(cudaMemcpyAsync(c->b.ctrl, cb, sizeof(Ctrl), cudaMemcpyDeviceToDevice, c->st));
-    else CK(cudaMemcpyAsync(cb, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToDevice, c->st));
+    if (restore) CK(cudaMemcpyAsync(c->d_block, c->d_backup, c->backup_len, cudaMemcpyDeviceToDevice, c->st));
+    else CK(cudaMemcpyAsync(c->d_backup, c->d_block, c->backup_len, cudaMemcpyDeviceToDevice, c->st));
+    return AMICA_OK;
+}
+
+// the pinned staging area, once no copy reads it any more
+int stage(amica_ctx* c) {
+    if (c->stage_busy) CK(cudaStreamSynchronize(c->st));
+    c->stage_busy = false;
     return AMICA_OK;
 }
 
@@ -288,10 +303,13 @@ int enqueue_iteration(amica_ctx* c) {
     return AMICA_OK;
 }
 
-int check_device_error(amica_ctx* c) {
-    CK(cudaMemcpyAsync(c->h_err, c->b.err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    int e = *c->h_err;
+int enqueue_status(amica_ctx* c) {
+    CK(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(Status), cudaMemcpyDeviceToHost, c->st));
+    return AMICA_OK;
+}
+// the error bits of a status that has arrived (cleared on the device)
+int status_error(amica_ctx* c) {
+    const int e = (int)c->h_status->err;
     if (e) {
         CK(cudaMemsetAsync(c->b.err, 0, sizeof(int), c->st));
         if (e & kErrWaitTimeout) return AMICA_ERR_TIMEOUT;
@@ -300,6 +318,43 @@ int check_device_error(amica_ctx* c) {
         if (e & kErrNonFinite) return AMICA_ERR_NUMERIC;
         return AMICA_ERR_CUDA;
     }
+    return AMICA_OK;
+}
+int check_device_error(amica_ctx* c) {
+    TRY(enqueue_status(c));
+    CK(cudaStreamSynchronize(c->st));
+    return status_error(c);
+}
+// history records [it0, it0 + count): into the pinned buffer behind the status
+// where they fit (read after the next synchronisation), else after it
+int enqueue_recs(amica_ctx* c, int64_t it0, int64_t count) {
+    if (count > 0 && count <= kPinnedRecs)
+        CK(cudaMemcpyAsync(c->h_recs, c->b.hist + it0, sizeof(IterRec) * count, cudaMemcpyDeviceToHost, c->st));
+    return AMICA_OK;
+}
+// The record of the single iteration after c->iter, in a slot of its own (a batch of
+// amica_run_async may be outstanding).  Past the end of the device's history it is
+// made from the control block.
+int enqueue_last_rec(amica_ctx* c) {
+    if (c->iter < c->b.hist_cap)
+        CK(cudaMemcpyAsync(c->h_recs + kPinnedRecs, c->b.hist + c->iter, sizeof(IterRec), cudaMemcpyDeviceToHost,
+                           c->st));
+    return AMICA_OK;
+}
+IterRec last_rec(const amica_ctx* c) {
+    if (c->iter < c->b.hist_cap) return c->h_recs[kPinnedRecs];
+    const Ctrl& t = *c->h_ctrl;
+    IterRec r{};
+    r.ll = t.ll; r.lrate = t.lrate; r.iter = t.iter; r.newton = t.newton; r.ll_decreased = t.ll_decreased;
+    r.nkeep = t.nkeep; r.nrejected = t.last_rejected; r.phi_split = t.phi_split;
+    return r;
+}
+int fetch_recs(amica_ctx* c, int64_t it0, std::vector<IterRec>& recs) {
+    const int64_t count = (int64_t)recs.size();
+    if (count > kPinnedRecs)
+        CK(cudaMemcpy(recs.data(), c->b.hist + it0, sizeof(IterRec) * count, cudaMemcpyDeviceToHost));
+    else
+        std::copy(c->h_recs, c->h_recs + count, recs.begin());
     return AMICA_OK;
 }
 
@@ -461,9 +516,21 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     const size_t nn = (size_t)n * n, mn = (size_t)m * n;
     int r = AMICA_OK;
 #define AL(p, cnt) if ((r = dalloc(&(p), (cnt))) != AMICA_OK) { amica_destroy(c); return r; }
-    AL(b.A, M * nn); AL(b.Anew, M * nn); AL(b.c, M * n); AL(b.alpha, M * mn); AL(b.mu, M * mn);
-    AL(b.beta, M * mn); AL(b.rho, M * mn); AL(b.gm, M); AL(b.W, M * nn); AL(b.ldet, M);
-    AL(b.ltc64, M);
+    const size_t plen = (size_t)param_len(c), slen = sizeof(Status) / sizeof(double);
+    AL(c->d_block, plen + slen + M * nn);
+    {
+        double* p = c->d_block;
+        auto take = [&](double** q, size_t len) { *q = p; p += len; };
+        take(&b.A, M * nn); take(&b.c, M * n); take(&b.alpha, M * mn); take(&b.mu, M * mn);
+        take(&b.beta, M * mn); take(&b.rho, M * mn); take(&b.gm, M);
+        c->d_status = reinterpret_cast<Status*>(p);
+        p += slen;
+        take(&b.W, M * nn);
+        b.ctrl = &c->d_status->ctrl;
+        b.err = reinterpret_cast<int*>(&c->d_status->err);
+        c->d_ldetS = &c->d_status->ldetS;
+    }
+    AL(b.Anew, M * nn); AL(b.ldet, M); AL(b.ltc64, M);
     PartLayout PL{(int)n, (int)m};
     const int groups = c->use_tc ? tc_partial_groups((int)n, c->tc_shape) : c->use_split ? 1 : plain_partial_groups((int)n);
     c->nslots = c->nclusters * groups;
@@ -486,19 +553,16 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     if (n > 128) AL(b.gj, (size_t)M * nn + (size_t)M * n);
     AL(b.bflag, M); AL(b.use_newton, M);
     AL(b.Wf, (size_t)M * NP * NP); AL(b.wcf, (size_t)M * NP); AL(b.mp, (size_t)M * m * NP);
-    AL(b.ctrl, 1);
     b.hist_cap = cfg->maxiter > 0 ? cfg->maxiter : 200;
     if (b.hist_cap < 1000) b.hist_cap = 1000;
     AL(b.hist, b.hist_cap);
-    AL(b.err, 1);
     AL(c->d_keep, T); AL(c->d_Lt, M * T); AL(c->d_P, T);
     // zero rows past T: the tensor-core form reads the data as rows of 128 floats
     // in segments of equal length; the buffer is the sphering's scratch first
     AL(c->d_x, std::max((size_t)T * NP + x_tail_len(NP), 2 * preprocess_min_ws((int)n)));
     AL(c->d_means, n); AL(c->d_sphere, nn); AL(c->d_cov, nn); AL(c->d_evwork, 4 * nn + 4 * n);
-    AL(c->d_ldetS, 1);
-    c->backup_len = param_len(c) + (sizeof(Ctrl) + 7) / 8;
-    AL(c->d_backup, c->backup_len);
+    c->backup_len = sizeof(double) * plen + sizeof(Ctrl);
+    AL(c->d_backup, plen + slen);
     if (c->use_split) {
         // g is written per 64-sample tile as the Psi operand image
         AL(c->d_B, (size_t)T * M * NP); AL(c->d_G, (size_t)((T + 63) / 64) * 64 * M * NP);
@@ -507,8 +571,16 @@ int amica_create(const amica_cfg* cfg, amica_ctx** out) {
     }
 #undef AL
     CK(cudaMemsetAsync(c->d_keep, 1, T, c->st));
-    CK(cudaMallocHost(&c->h_ctrl, sizeof(Ctrl)));
-    CK(cudaMallocHost(&c->h_err, sizeof(int)));
+    {
+        // one pinned allocation: the status, the records, the parameters and W
+        const size_t recs = sizeof(IterRec) * (kPinnedRecs + 1);
+        char* hp = nullptr;
+        CK(cudaMallocHost(&hp, sizeof(Status) + recs + sizeof(double) * (plen + M * nn)));
+        c->h_status = reinterpret_cast<Status*>(hp);
+        c->h_ctrl = &c->h_status->ctrl;
+        c->h_recs = reinterpret_cast<IterRec*>(hp + sizeof(Status));
+        c->h_stage = reinterpret_cast<double*>(hp + sizeof(Status) + recs);
+    }
     CK(cudaStreamSynchronize(c->st));
     *out = c;
     return AMICA_OK;
@@ -519,16 +591,14 @@ int amica_destroy(amica_ctx* c) {
     cudaSetDevice(c->dev);
     if (c->st) cudaStreamSynchronize(c->st);
     if (c->graph) cudaGraphExecDestroy(c->graph);
-    void* ptrs[] = {c->b.A, c->b.Anew, c->b.c, c->b.alpha, c->b.mu, c->b.beta, c->b.rho, c->b.gm,
-                    c->b.W, c->b.ldet, c->b.ltc64, c->b.partial, c->b.raw, c->b.stats,
+    void* ptrs[] = {c->d_block, c->b.Anew, c->b.ldet, c->b.ltc64, c->b.partial, c->b.raw, c->b.stats,
                     c->b.work, c->b.chunk, c->b.gj, c->b.bflag, c->b.use_newton, c->b.Wf, c->b.wcf,
-                    c->b.mp, c->b.ctrl, c->b.hist, c->b.err, c->d_keep, c->d_Lt, c->d_P, c->d_x,
-                    c->d_rawx, c->d_means, c->d_sphere, c->d_cov, c->d_evwork, c->d_ldetS,
+                    c->b.mp, c->b.hist, c->d_keep, c->d_Lt, c->d_P, c->d_x,
+                    c->d_rawx, c->d_means, c->d_sphere, c->d_cov, c->d_evwork,
                     c->d_backup, c->d_gradp, c->d_grad, c->d_B, c->d_G, c->d_Whi, c->d_Wlo, c->d_xT};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    if (c->h_ctrl) cudaFreeHost(c->h_ctrl);
-    if (c->h_err) cudaFreeHost(c->h_err);
+    if (c->h_status) cudaFreeHost(c->h_status);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->st) cudaStreamDestroy(c->st);
@@ -570,12 +640,8 @@ int amica_preprocess(amica_ctx* c) {
     CK(launch_preprocess(c->d_rawx, c->T, c->n, (int)c->cfg.do_sphere, c->d_means, c->d_cov,
                          c->d_sphere, c->d_evwork, c->d_ldetS, c->d_x, c->NP, (c->use_tc || c->use_split) ? 1 : 0,
                          c->b.err, c->st, fault));
-    double ld = 0.0;
-    CK(cudaMemcpyAsync(&ld, c->d_ldetS, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
     TRY(check_device_error(c));
-    c->ldetS = ld;
-    c->hc.ldetS = ld;
+    c->ldetS = c->hc.ldetS = c->h_status->ldetS;
     TRY(x_ready(c));
     return AMICA_OK;
 }
@@ -603,18 +669,23 @@ int amica_init(amica_ctx* c, const double* A0, const double* c0) {
     if (!c) return AMICA_ERR_INVALIDPARAM;
     CK(cudaSetDevice(c->dev));
     const int n = c->n, M = c->M, m = c->m;
-    std::vector<double> A((size_t)M * n * n), cc((size_t)M * n), alpha((size_t)M * m * n),
-        mu((size_t)M * m * n), beta((size_t)M * m * n), rho((size_t)M * m * n), gm(M);
+    // built in the staging area, in the block's order
+    TRY(stage(c));
+    const size_t nnM = (size_t)M * n * n, mnM = (size_t)M * m * n;
+    double* A = c->h_stage;
+    double *cc = A + nnM, *alpha = cc + (size_t)M * n, *mu = alpha + mnM, *beta = mu + mnM, *rho = beta + mnM,
+           *gm = rho + mnM;
+    std::fill(cc, cc + (size_t)M * n, 0.0);
     std::mt19937_64 rng((uint64_t)c->cfg.seed);
     std::uniform_real_distribution<double> U(0.0, 1.0);
     std::normal_distribution<double> N01(0.0, 1.0);
     if (A0) {
-        memcpy(A.data(), A0, sizeof(double) * A.size());
-        if (c0) memcpy(cc.data(), c0, sizeof(double) * cc.size());
+        memcpy(A, A0, sizeof(double) * nnM);
+        if (c0) memcpy(cc, c0, sizeof(double) * M * n);
     } else {
         // A = I + 0.05 (U - 0.5), unit columns; c ~ N(0, 1) (src/amica.cu:272-312)
         for (int h = 0; h < M; h++) {
-            double* Ah = A.data() + (size_t)h * n * n;
+            double* Ah = A + (size_t)h * n * n;
             for (int e = 0; e < n * n; e++) Ah[e] = (U(rng) - 0.5) * 0.05 + ((e % n) == (e / n) ? 1.0 : 0.0);
             for (int col = 0; col < n; col++) {
                 double s = 0.0;
@@ -641,13 +712,7 @@ int amica_init(amica_ctx* c, const double* A0, const double* c0) {
                 rho[idx] = c->cfg.rho0;                // :389-394
             }
     }
-    CK(cudaMemcpyAsync(c->b.A, A.data(), sizeof(double) * A.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->b.c, cc.data(), sizeof(double) * cc.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->b.alpha, alpha.data(), sizeof(double) * alpha.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->b.mu, mu.data(), sizeof(double) * mu.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->b.beta, beta.data(), sizeof(double) * beta.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->b.rho, rho.data(), sizeof(double) * rho.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->b.gm, gm.data(), sizeof(double) * gm.size(), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->d_block, c->h_stage, sizeof(double) * param_len(c), cudaMemcpyHostToDevice, c->st));
     Ctrl ctl{};
     ctl.lrate = c->cfg.lrate0;
     ctl.lratemax = c->cfg.lratemax;
@@ -658,6 +723,7 @@ int amica_init(amica_ctx* c, const double* A0, const double* c0) {
     CK(cudaMemcpyAsync(c->b.ctrl, c->h_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemsetAsync(c->d_keep, 1, c->T, c->st));
     CK(cudaStreamSynchronize(c->st));
+    c->iter = 0;
     c->hist.clear();
     c->have_init = true;
     if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
@@ -672,10 +738,11 @@ int amica_em_step(amica_ctx* c, amica_iter_out* out) {
     CK(cudaEventRecord(c->ev0, c->st));
     TRY(enqueue_iteration(c));
     CK(cudaEventRecord(c->ev1, c->st));
-    CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
+    TRY(enqueue_status(c));
+    TRY(enqueue_last_rec(c));
     CK(cudaStreamSynchronize(c->st));
     c->have_estep = true;
-    int e = check_device_error(c);
+    int e = status_error(c);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     const Ctrl ctl = *c->h_ctrl;
@@ -685,8 +752,8 @@ int amica_em_step(amica_ctx* c, amica_iter_out* out) {
         cudaStreamSynchronize(c->st);
         return e;
     }
-    IterRec r{};
-    CK(cudaMemcpy(&r, c->b.hist + (ctl.iter - 1), sizeof(IterRec), cudaMemcpyDeviceToHost));
+    const IterRec r = last_rec(c);
+    c->iter = ctl.iter;
     c->hist.push_back(r);
     print_iter(c, r);
     fill_out(r, ctl, ms, out);
@@ -709,15 +776,14 @@ int amica_run_async(amica_ctx* c, int64_t maxiter) {
         CK(cudaGraphInstantiate(&c->graph, g, 0));
         CK(cudaGraphDestroy(g));
     }
-    CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    const int64_t it0 = c->h_ctrl->iter;
+    const int64_t it0 = c->iter;
     if (it0 + maxiter > c->b.hist_cap) return AMICA_ERR_INVALIDPARAM;
     TRY(snapshot_params(c, false));
     CK(cudaEventRecord(c->ev0, c->st));
     for (int64_t k = 0; k < maxiter; k++) CK(cudaGraphLaunch(c->graph, c->st));
     CK(cudaEventRecord(c->ev1, c->st));
-    CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
+    TRY(enqueue_status(c));
+    TRY(enqueue_recs(c, it0, maxiter));
     c->pending = maxiter;
     c->pending_it0 = it0;
     return AMICA_OK;
@@ -731,12 +797,12 @@ int amica_run_wait(amica_ctx* c, amica_iter_out* hist) {
     c->pending = -1;
     CK(cudaStreamSynchronize(c->st));
     c->have_estep = maxiter > 0 || c->have_estep;
-    int e = check_device_error(c);
+    int e = status_error(c);
+    c->iter = c->h_ctrl->iter;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     std::vector<IterRec> recs(maxiter);
-    if (maxiter > 0)
-        CK(cudaMemcpy(recs.data(), c->b.hist + it0, sizeof(IterRec) * maxiter, cudaMemcpyDeviceToHost));
+    TRY(fetch_recs(c, it0, recs));
     for (int64_t k = 0; k < maxiter; k++) {
         if (e == AMICA_OK && !std::isfinite(recs[k].ll)) e = AMICA_ERR_NUMERIC;
         c->hist.push_back(recs[k]);
@@ -746,6 +812,7 @@ int amica_run_wait(amica_ctx* c, amica_iter_out* hist) {
     if (e == AMICA_ERR_NUMERIC) {
         snapshot_params(c, true);
         cudaStreamSynchronize(c->st);
+        c->iter = it0;
     }
     return e;
 }
@@ -804,19 +871,33 @@ int amica_run(amica_ctx* c, int64_t maxiter, amica_iter_out* hist) {
     return amica_run_wait(c, hist);
 }
 
+// Parameters in and out go through the pinned staging area in one copy up to this
+// size; above it the arrays are copied one by one from and to the caller's memory.
+constexpr size_t kStageBytes = 2u << 20;
+
 int amica_get_params(amica_ctx* c, double* A, double* W, double* cc, double* gm, double* alpha,
                      double* mu, double* beta, double* rho) {
     if (!c) return AMICA_ERR_INVALIDPARAM;
     CK(cudaSetDevice(c->dev));
-    const size_t nn = (size_t)c->n * c->n * c->M, mn = (size_t)c->m * c->n * c->M;
-    if (A) CK(cudaMemcpyAsync(A, c->b.A, sizeof(double) * nn, cudaMemcpyDeviceToHost, c->st));
-    if (W) CK(cudaMemcpyAsync(W, c->b.W, sizeof(double) * nn, cudaMemcpyDeviceToHost, c->st));
-    if (cc) CK(cudaMemcpyAsync(cc, c->b.c, sizeof(double) * c->n * c->M, cudaMemcpyDeviceToHost, c->st));
-    if (gm) CK(cudaMemcpyAsync(gm, c->b.gm, sizeof(double) * c->M, cudaMemcpyDeviceToHost, c->st));
-    if (alpha) CK(cudaMemcpyAsync(alpha, c->b.alpha, sizeof(double) * mn, cudaMemcpyDeviceToHost, c->st));
-    if (mu) CK(cudaMemcpyAsync(mu, c->b.mu, sizeof(double) * mn, cudaMemcpyDeviceToHost, c->st));
-    if (beta) CK(cudaMemcpyAsync(beta, c->b.beta, sizeof(double) * mn, cudaMemcpyDeviceToHost, c->st));
-    if (rho) CK(cudaMemcpyAsync(rho, c->b.rho, sizeof(double) * mn, cudaMemcpyDeviceToHost, c->st));
+    const size_t nn = (size_t)c->n * c->n * c->M, mn = (size_t)c->m * c->n * c->M, nM = (size_t)c->n * c->M;
+    struct Seg { double* host; const double* dev; size_t len; } segs[] = {
+        {A, c->b.A, nn}, {cc, c->b.c, nM}, {alpha, c->b.alpha, mn}, {mu, c->b.mu, mn}, {beta, c->b.beta, mn},
+        {rho, c->b.rho, mn}, {gm, c->b.gm, (size_t)c->M}, {W, c->b.W, nn}};
+    const size_t plen = (size_t)param_len(c);
+    if (sizeof(double) * (plen + nn) <= kStageBytes) {
+        TRY(stage(c));
+        CK(cudaMemcpyAsync(c->h_stage, c->d_block, sizeof(double) * plen, cudaMemcpyDeviceToHost, c->st));
+        if (W) CK(cudaMemcpyAsync(c->h_stage + plen, c->b.W, sizeof(double) * nn, cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        const double* p = c->h_stage;
+        for (const auto& s : segs) {
+            if (s.host) memcpy(s.host, p, sizeof(double) * s.len);
+            p += s.len;
+        }
+        return AMICA_OK;
+    }
+    for (const auto& s : segs)
+        if (s.host) CK(cudaMemcpyAsync(s.host, s.dev, sizeof(double) * s.len, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     return AMICA_OK;
 }
@@ -825,14 +906,37 @@ int amica_set_params(amica_ctx* c, const double* A, const double* cc, const doub
                      const double* alpha, const double* mu, const double* beta, const double* rho) {
     if (!c) return AMICA_ERR_INVALIDPARAM;
     CK(cudaSetDevice(c->dev));
-    const size_t nn = (size_t)c->n * c->n * c->M, mn = (size_t)c->m * c->n * c->M;
-    if (A) CK(cudaMemcpyAsync(c->b.A, A, sizeof(double) * nn, cudaMemcpyHostToDevice, c->st));
-    if (cc) CK(cudaMemcpyAsync(c->b.c, cc, sizeof(double) * c->n * c->M, cudaMemcpyHostToDevice, c->st));
-    if (gm) CK(cudaMemcpyAsync(c->b.gm, gm, sizeof(double) * c->M, cudaMemcpyHostToDevice, c->st));
-    if (alpha) CK(cudaMemcpyAsync(c->b.alpha, alpha, sizeof(double) * mn, cudaMemcpyHostToDevice, c->st));
-    if (mu) CK(cudaMemcpyAsync(c->b.mu, mu, sizeof(double) * mn, cudaMemcpyHostToDevice, c->st));
-    if (beta) CK(cudaMemcpyAsync(c->b.beta, beta, sizeof(double) * mn, cudaMemcpyHostToDevice, c->st));
-    if (rho) CK(cudaMemcpyAsync(c->b.rho, rho, sizeof(double) * mn, cudaMemcpyHostToDevice, c->st));
+    const size_t nn = (size_t)c->n * c->n * c->M, mn = (size_t)c->m * c->n * c->M, nM = (size_t)c->n * c->M;
+    struct Seg { const double* host; double* dev; size_t len; } segs[] = {
+        {A, c->b.A, nn}, {cc, c->b.c, nM}, {alpha, c->b.alpha, mn}, {mu, c->b.mu, mn}, {beta, c->b.beta, mn},
+        {rho, c->b.rho, mn}, {gm, c->b.gm, (size_t)c->M}};
+    const size_t plen = (size_t)param_len(c);
+    if (sizeof(double) * plen <= kStageBytes) {
+        TRY(stage(c));
+        // consecutive arrays that are given go in one copy; the caller's memory has
+        // been read when this returns
+        size_t off = 0, from = 0;
+        auto send = [&](size_t to) -> int {
+            if (to > from)
+                CK(cudaMemcpyAsync(c->d_block + from, c->h_stage + from, sizeof(double) * (to - from),
+                                   cudaMemcpyHostToDevice, c->st));
+            return AMICA_OK;
+        };
+        for (const auto& s : segs) {
+            if (s.host) {
+                memcpy(c->h_stage + off, s.host, sizeof(double) * s.len);
+            } else {
+                TRY(send(off));
+                from = off + s.len;
+            }
+            off += s.len;
+        }
+        TRY(send(off));
+        c->stage_busy = true;
+        return AMICA_OK;
+    }
+    for (const auto& s : segs)
+        if (s.host) CK(cudaMemcpyAsync(s.dev, s.host, sizeof(double) * s.len, cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
     return AMICA_OK;
 }
@@ -1064,9 +1168,10 @@ int amica_shard_mstep(amica_ctx* c, const double* d_stats, int64_t nkeep_total, 
     CK(launch_mstep(c->b, c->hc, false, c->d_P, c->d_keep, c->T, c->st));
     k_set_nkeep<<<1, 1, 0, c->st>>>(c->b.ctrl, c->T);
     CK(cudaEventRecord(c->ev1, c->st));
-    CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
+    TRY(enqueue_status(c));
+    TRY(enqueue_last_rec(c));
     CK(cudaStreamSynchronize(c->st));
-    int e = check_device_error(c);
+    int e = status_error(c);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     const Ctrl ctl = *c->h_ctrl;
@@ -1076,8 +1181,8 @@ int amica_shard_mstep(amica_ctx* c, const double* d_stats, int64_t nkeep_total, 
         cudaStreamSynchronize(c->st);
         return e;
     }
-    IterRec r{};
-    CK(cudaMemcpy(&r, c->b.hist + (ctl.iter - 1), sizeof(IterRec), cudaMemcpyDeviceToHost));
+    IterRec r = last_rec(c);
+    c->iter = ctl.iter;
     r.nkeep = nkeep_total;
     c->hist.push_back(r);
     print_iter(c, r);
@@ -1114,12 +1219,8 @@ int amica_shard_sphere(amica_ctx* c, const double* d_scatter_total, int64_t T_to
     CK(launch_shard_finish(c->d_rawx, c->T, c->n, (int)c->cfg.do_sphere, c->d_means, d_scatter_total, T_total,
                            c->d_cov, c->d_sphere, c->d_evwork, c->d_ldetS, c->d_x, c->NP,
                            (c->use_tc || c->use_split) ? 1 : 0, c->b.err, c->st));
-    double ld = 0.0;
-    CK(cudaMemcpyAsync(&ld, c->d_ldetS, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
     TRY(check_device_error(c));
-    c->ldetS = ld;
-    c->hc.ldetS = ld;
+    c->ldetS = c->hc.ldetS = c->h_status->ldetS;
     TRY(x_ready(c));
     c->have_shard_mean = false;
     return AMICA_OK;
@@ -1143,17 +1244,19 @@ int amica_selftest_umma(int mode, int N, int K, const float* A, const float* B, 
     return tc_selftest(mode, N, K, A, B, D, device_err);
 }
 
+__global__ void k_set_iter_state(Ctrl* ctrl, int64_t iter, double lrate, double ll_prev) {
+    ctrl->iter = iter;
+    ctrl->lrate = lrate;
+    ctrl->ll_prev = ll_prev;
+}
+
 int amica_set_iter_state(amica_ctx* c, int64_t iter, double lrate, double ll_prev) {
     if (!c || iter < 0 || !(lrate > 0.0)) return AMICA_ERR_INVALIDPARAM;
     if (!c->have_init) return AMICA_ERR_STATE;
     CK(cudaSetDevice(c->dev));
-    CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    c->h_ctrl->iter = iter;
-    c->h_ctrl->lrate = lrate;
-    c->h_ctrl->ll_prev = ll_prev;
-    CK(cudaMemcpyAsync(c->b.ctrl, c->h_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    k_set_iter_state<<<1, 1, 0, c->st>>>(c->b.ctrl, iter, lrate, ll_prev);
+    CK(cudaGetLastError());
+    c->iter = iter;
     return AMICA_OK;
 }
 
@@ -1329,9 +1432,7 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
         amica_ctx* c = co->subs[s];
         if (!c->have_x || !c->have_init) return AMICA_ERR_STATE;
         if (c->pending >= 0) return AMICA_ERR_STATE;
-        CK(cudaMemcpyAsync(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
-        it0[s] = c->h_ctrl->iter;
+        it0[s] = c->iter;
         if (it0[s] + iters > c->b.hist_cap) return AMICA_ERR_INVALIDPARAM;
     }
     if (!co->graph) TRY(cohort_capture(co));
@@ -1344,6 +1445,13 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
     CK(cudaEventRecord(co->ev0, co->st));
     for (int64_t k = 0; k < iters; k++) CK(cudaGraphLaunch(co->graph, co->st));
     CK(cudaEventRecord(co->ev1, co->st));
+    // each subject's status and records on its own stream, behind the graphs
+    for (int s = 0; s < ns; s++) {
+        amica_ctx* c = co->subs[s];
+        CK(cudaStreamWaitEvent(c->st, co->ev1, 0));
+        TRY(enqueue_status(c));
+        TRY(enqueue_recs(c, it0[s], iters));
+    }
     CK(cudaStreamSynchronize(co->st));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, co->ev0, co->ev1));
@@ -1352,11 +1460,11 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
     for (int s = 0; s < ns; s++) {
         amica_ctx* c = co->subs[s];
         c->have_estep = c->have_estep || iters > 0;
-        int e = check_device_error(c);
-        CK(cudaMemcpy(c->h_ctrl, c->b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost));
+        CK(cudaStreamSynchronize(c->st));
+        int e = status_error(c);
+        c->iter = c->h_ctrl->iter;
         std::vector<IterRec> recs(iters);
-        if (iters > 0)
-            CK(cudaMemcpy(recs.data(), c->b.hist + it0[s], sizeof(IterRec) * iters, cudaMemcpyDeviceToHost));
+        TRY(fetch_recs(c, it0[s], recs));
         for (int64_t k = 0; k < iters; k++) {
             if (e == AMICA_OK && !std::isfinite(recs[k].ll)) e = AMICA_ERR_NUMERIC;
             c->hist.push_back(recs[k]);
@@ -1366,6 +1474,7 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
         if (e == AMICA_ERR_NUMERIC) {
             snapshot_params(c, true);
             cudaStreamSynchronize(c->st);
+            c->iter = it0[s];
         }
         if (first_err == AMICA_OK) first_err = e;
     }
