@@ -31,7 +31,6 @@ using namespace amica;
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = 5u << 20;     // 5 MiB per device
-constexpr int kNoAllocMaxClusters = 8;                // largest E-step grid in this mode
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -98,12 +97,13 @@ extern "C" int amica_estep_stats_noalloc(const float* x, int64_t ldx, int64_t n,
     const int ntiles = (int)((T + plain_tile_samples() - 1) / plain_tile_samples());
     int ncl = plain_max_clusters((int)n, (int)m, (int)M);
     if (ncl <= 0) return AMICA_ERR_UNSUPPORTED;
-    if (ncl > kNoAllocMaxClusters) ncl = kNoAllocMaxClusters;
     if (ncl > ntiles) ncl = ntiles;
     // above 128 channels each cluster has one slot per channel block
     const int groups = plain_partial_groups((int)n);
-    // every cluster writes its own partial slots: use fewer clusters (down to
-    // one, which runs every tile) until the layout fits the fixed array
+    // every cluster writes its own partial slots: as many clusters as tiles and
+    // SMs, fewer (down to one, which runs every tile) until the layout fits the
+    // fixed array.  (64 clusters against 8 at n = 32, T = 4096: the E-step kernel
+    // takes 14 us instead of 60.)
     MStepBuffers b;
     while (ncl > 1 && carve(nullptr, (int)n, (int)M, (int)m, NP, ncl * groups, &b) > kNoAllocScratchBytes)
         ncl--;

@@ -120,10 +120,14 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
     __shared__ double s_lgm;
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const double* Ah = A + (size_t)h * n * n;
-    for (int e = tid; e < kInvN * kInvN; e += kInvThreads) {
-        const int j = e >> 7, r = e & (kInvN - 1);
-        As[r * kLdA + j] = (r < n && j < n) ? Ah[(size_t)j * n + r] : 0.0;
-    }
+    // columns of whole panels, and all rows that panel threads hold
+    const int np16 = (n + kPanel - 1) & ~(kPanel - 1), nct = np16 / 8;
+    for (int j = warp; j < np16; j += kInvThreads / 32)
+#pragma unroll
+        for (int u = 0; u < kInvN / 32; u++) {
+            const int r = lane + 32 * u;
+            As[r * kLdA + j] = (r < n && j < n) ? Ah[(size_t)j * n + r] : 0.0;
+        }
     if (tid < kInvN) pinv[tid] = 0x7fffffff;
     if (tid == 0) s_bad = 0;
     // panel threads (tid < 64): rows r0 = tid and r1 = tid + 64, not yet pivot rows
@@ -244,18 +248,20 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
             const int kp = k0 - kPanel;
             const double* Xp = Xs + ((b - 1) & 1) * kInvN * kLdX;
             const int w0 = b == npan ? 0 : 4, nw = b == npan ? 16 : 12;
-            for (int ct = warp - w0; ct < kInvN / 8; ct += nw) {
+            for (int ct = warp - w0; ct < nct; ct += nw) {
                 const int j0 = 8 * ct;
                 if ((unsigned)(j0 - kp) < (unsigned)kPanel || (unsigned)(j0 - k0) < (unsigned)kPanel) continue;
-                block_sweep_strip(As, Xp, Pt, pinv, kp, ct, 0, 8, lane);
-                block_sweep_strip(As, Xp, Pt, pinv, kp, ct, 8, 8, lane);
+                // (constant tile counts: a runtime one doubled the kernel's time)
+                int rt = 0;
+                for (; rt + 8 <= nct; rt += 8) block_sweep_strip(As, Xp, Pt, pinv, kp, ct, rt, 8, lane);
+                for (; rt < nct; rt += 2) block_sweep_strip(As, Xp, Pt, pinv, kp, ct, rt, 2, lane);
             }
         }
         __syncthreads();
         if (s_bad || b == npan) break;
         // Pt for this panel: its pivot rows' entries outside it, now final up to it
         const int w = min(kPanel, n - k0);
-        for (int e = tid; e < kPanel * kInvN; e += kInvThreads) {
+        for (int e = tid; e < kPanel * np16; e += kInvThreads) {
             const int j = e >> 4, t = e & (kPanel - 1);
             if ((unsigned)(j - k0) < (unsigned)kPanel) continue;
             Pt[j * kLdX + t] = t < w ? As[perm[k0 + t] * kLdA + j] : 0.0;
@@ -264,7 +270,8 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
         if (b + 1 < npan) {
             // the next panel's 16 columns: 2 strips x 16 row tiles, 2 tiles per warp
             const double* Xb = Xs + (b & 1) * kInvN * kLdX;
-            block_sweep_strip(As, Xb, Pt, pinv, k0, 2 * (b + 1) + (warp & 1), 2 * (warp >> 1), 2, lane);
+            const int rt0 = 2 * (warp >> 1);
+            if (rt0 < nct) block_sweep_strip(As, Xb, Pt, pinv, k0, 2 * (b + 1) + (warp & 1), rt0, 2, lane);
         }
         __syncthreads();
     }
@@ -575,52 +582,69 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_big(const double* __
 }
 
 // k_derive: log|det W_h|, the Lt constant and the FP32 E-step constants from a
-// column-major W (the tail of k_inverse_derive for the n > 128 path).  One CTA
-// of 256 threads per model.
+// column-major W (the tail of k_inverse_derive for the n > 128 path).  A CTA of 8
+// warps owns 32 channels of one model: w_c = W c (warps share the columns), its
+// rows of W in FP32 (32 x 32 tiles turned in shared memory) and its channels'
+// mixture constants.  (One CTA per model, walking rows of the column-major W and
+// adding the pivots' logarithms in one thread, took 166 us at n = 256.)
 __global__ void __launch_bounds__(256) k_derive(
     const double* __restrict__ W, const double* __restrict__ pivlog, const double* __restrict__ c,
     const double* __restrict__ alpha, const double* __restrict__ mu, const double* __restrict__ beta,
     const double* __restrict__ rho, const double* __restrict__ gm, double ldetS,
     double* __restrict__ ldet, double* __restrict__ ltc64, float* __restrict__ Wf,
     float* __restrict__ wcf, MixParam* __restrict__ mp, int n, int m, int NP) {
-    const int h = blockIdx.x, tid = threadIdx.x;
+    __shared__ double part[8][32];
+    __shared__ float tile[32][33];
+    const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int i0 = 32 * blockIdx.x, i = i0 + lane;
     const double* Wh = W + (size_t)h * n * n;
-    __shared__ double wcs[kMaxN];
-    if (tid == 0) {
+    if (blockIdx.x == 0 && warp == 0) {
         double ld = 0.0;
-        for (int k = 0; k < n; k++) ld += pivlog[(size_t)h * n + k];
-        ldet[h] = -ld;
-        ltc64[h] = log(gm[h]) - ld + ldetS;           // src/amica.cu:1009
+        for (int k = lane; k < n; k += 32) ld += pivlog[(size_t)h * n + k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, o);
+        if (lane == 0) {
+            ldet[h] = -ld;
+            ltc64[h] = log(gm[h]) - ld + ldetS;        // src/amica.cu:1009
+        }
     }
-    for (int i = tid; i < NP; i += blockDim.x) {
-        double wc = 0.0;
-        if (i < n)
-            for (int k = 0; k < n; k++) wc += Wh[(size_t)k * n + i] * c[(size_t)h * n + k];
-        wcs[i] = wc;
-        wcf[(size_t)h * NP + i] = (float)wc;
+    double wc = 0.0;
+    if (i < n) {
+#pragma unroll 8
+        for (int k = warp; k < n; k += 8) wc = fma(Wh[(size_t)k * n + i], c[(size_t)h * n + k], wc);
     }
+    part[warp][lane] = wc;
     float* Wfh = Wf + (size_t)h * NP * NP;
-    for (int e = tid; e < NP * NP; e += blockDim.x) {
-        const int i = e / NP, k = e - i * NP;
-        Wfh[e] = (i < n && k < n) ? (float)Wh[(size_t)k * n + i] : 0.f;
+    for (int k0 = 0; k0 < NP; k0 += 32) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = k0 + warp + 8 * q;           // column k of W, rows i0 ..
+            tile[lane][warp + 8 * q] = (i < n && k < n) ? (float)Wh[(size_t)k * n + i] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) Wfh[(size_t)(i0 + warp + 8 * q) * NP + k0 + lane] = tile[warp + 8 * q][lane];
     }
-    __syncthreads();
-    for (int e = tid; e < m * NP; e += blockDim.x) {
-        const int j = e / NP, i = e - j * NP;
+    wc = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) wc += part[w][lane];   // in every warp
+    if (warp == 0) wcf[(size_t)h * NP + i] = (float)wc;
+    if (warp < m) {
         MixParam q;
         if (i < n) {
-            const size_t idx = ((size_t)h * m + j) * n + i;
+            const size_t idx = ((size_t)h * m + warp) * n + i;
             const double s = sqrt(beta[idx]);
             const double r = rho[idx];
             q.s = (float)s;
-            q.off = (float)(s * (mu[idx] + wcs[i]));
+            q.off = (float)(s * (mu[idx] + wc));
             q.cl2 = (float)((log(alpha[idx]) + 0.5 * log(beta[idx]) - M_LN2 - lgamma(1.0 + 1.0 / r)) *
                             1.4426950408889634);
             q.rho = (float)r;
         } else {
             q.s = 0.f; q.off = 0.f; q.cl2 = 0.f; q.rho = 1.f;
         }
-        mp[((size_t)h * m + j) * NP + i] = q;
+        mp[((size_t)h * m + warp) * NP + i] = q;
     }
 }
 
@@ -1320,7 +1344,7 @@ cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream
                                              (int)kBigSmem);
         if (e != cudaSuccess) return e;
         k_inverse_big<<<h.M, kInvThreads, kBigSmem, st>>>(b.A, b.gj, b.W, pivlog, h.n, b.err);
-        k_derive<<<h.M, 256, 0, st>>>(b.W, pivlog, b.c, b.alpha, b.mu, b.beta, b.rho, b.gm, h.ldetS,
+        k_derive<<<dim3(h.NP / 32, h.M), 256, 0, st>>>(b.W, pivlog, b.c, b.alpha, b.mu, b.beta, b.rho, b.gm, h.ldetS,
                                       b.ldet, b.ltc64, b.Wf, b.wcf, b.mp, h.n, h.m, h.NP);
         return cudaGetLastError();
     }
