@@ -22,6 +22,13 @@ enum : int {
     kErrNonFinite = 8,        // the M-step produced a non-finite parameter
 };
 
+// The split form's tiles of 32 samples: sample s of tile `tile` of ntiles =
+// ceil(T / 32) is sample s % 4 of the tile's four in segment s / 4 of eight (each
+// of 4 ntiles samples); indices at and beyond T are padding.
+__host__ __device__ inline int64_t split_sample(int64_t tile, int s, int64_t ntiles) {
+    return (int64_t)(s >> 2) * 4 * ntiles + 4 * tile + (s & 3);
+}
+
 // Per-(model, mixture, channel) E-step constants, derived in FP64 from the
 // parameters once per iteration and rounded to FP32:
 //   y  = s * (W x)_i - off          (s = sqrt(beta), off = s * (mu + (W c)_i))

@@ -7,6 +7,12 @@
 // score function and the per-(channel, mixture) sums) and writes g as the
 // Psi contraction's operand image.
 //
+// A tile's samples are four consecutive ones from each of eight segments of the
+// data (common.cuh, split_sample): the models of consecutive samples are mostly
+// the same, and a model skips the second phase of samples it has no
+// responsibility for, so with 32 consecutive samples one CTA of the cluster
+// worked while the others waited.  n = 256, T = 400k, M = 4, m = 5: FIGURE.
+//
 // Layout: one thread-block cluster of M CTAs (CTA h = model h) per tile
 // stream, 256 threads per CTA (thread = channel, all 32 samples of a tile),
 // 128 registers, two CTAs per SM: clusters of M place on any SM pair, so the
@@ -53,10 +59,10 @@ struct DensShape {
     static constexpr size_t off_b = 0;                                          // [2][kDS][kDNP] float
     static constexpr size_t off_lse = off_b + 2 * (size_t)kDS * kDNP * 4;       // [kDS][kDLL] float
     static constexpr size_t off_slot = off_lse + (size_t)kDS * kDLL * 4;        // [2][kDS] float
-    static constexpr size_t off_v = off_slot + 2 * kDS * 4;                     // [kDS] float
+    static constexpr size_t off_v = off_slot + 2 * kDS * 4;                     // [kDS] float, 16-byte aligned
     static constexpr size_t off_bar = off_v + kDS * 4;                          // 2 mbarriers, abort flag
     static constexpr size_t bytes = off_bar + 32;
-    static_assert(off_b % 16 == 0 && off_bar % 8 == 0, "alignment");
+    static_assert(off_b % 16 == 0 && off_v % 16 == 0 && off_bar % 8 == 0, "alignment");
 };
 
 // Per-mixture constants of one channel for two mixtures at once.
@@ -162,16 +168,15 @@ __device__ __forceinline__ void da_one(const MixQ1& P, float bx, float nlse, flo
 
 // The b rows of one tile of model h into the b buffer: one 1 KB bulk copy per
 // sample (rows past T are not copied; phase 1 reads them as 0).  Warp 0.
-__device__ __forceinline__ void issue_b_tile(const EStepArgs& a, int h, int tile, float* bs, uint64_t* bar,
-                                             int lane) {
-    const int64_t t0 = (int64_t)tile * kDS;
-    const int64_t left = a.T - t0;
-    const int rows = left < kDS ? (int)left : kDS;
+__device__ __forceinline__ void issue_b_tile(const EStepArgs& a, int h, int tile, int ntiles, float* bs,
+                                             uint64_t* bar, int lane) {
+    const int64_t t = split_sample(tile, lane, ntiles);
+    const bool in = t < a.T;
+    const int rows = __popc(__ballot_sync(0xffffffffu, in));
     if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * kDNP * 4);
     __syncwarp();
-    if (lane < rows)
-        bulk_load(smem_u32(bs + lane * kDNP), a.bext + (size_t)(t0 + lane) * a.ldb + (size_t)h * kDNP,
-                  kDNP * 4, bar);
+    if (in)
+        bulk_load(smem_u32(bs + lane * kDNP), a.bext + (size_t)t * a.ldb + (size_t)h * kDNP, kDNP * 4, bar);
 }
 
 template <int MM>
@@ -239,7 +244,7 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
     const float wci = a.wc[(size_t)h * kDNP + ch];
     const float ltch = (float)(a.ltc64[h] - a.ltc64[0]);
     __syncthreads();
-    if (tid < 32 && cid < ntiles) issue_b_tile(a, h, cid, bs, &bar[0], lane);
+    if (tid < 32 && cid < ntiles) issue_b_tile(a, h, cid, ntiles, bs, &bar[0], lane);
 
     float2 fP[NPRA][7];
     float fS1[7];
@@ -280,8 +285,8 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
 
     int it = 0;
     for (int tile = cid; tile < ntiles; tile += a.nclusters, ++it) {
-        const int64_t t0 = (int64_t)tile * kDS;
         const int par = it & 1, stg = it & 1;
+        auto in_tile = [&](int t) { return split_sample(tile, t, ntiles) < T; };
         const float* bst = bs + stg * (kDS * kDNP);
         if (mbar_wait(&bar[stg], (uint32_t)(it >> 1) & 1u, abort_flag, a.err) && tid < 32) pend &= ~(1u << stg);
         // ---- the other stage was last read before the previous tile's final
@@ -289,16 +294,17 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
         const int next = tile + a.nclusters;
         if (tid < 32) {
             const int go = __shfl_sync(0xffffffffu, (next < ntiles && !abort_get(abort_flag)) ? 1 : 0, 0);
-            if (go) issue_b_tile(a, h, next, bs + (stg ^ 1) * (kDS * kDNP), &bar[stg ^ 1], lane);
+            if (go) issue_b_tile(a, h, next, ntiles, bs + (stg ^ 1) * (kDS * kDNP), &bar[stg ^ 1], lane);
             if (go) {
                 pend |= 1u << (stg ^ 1);
                 pendpar = (pendpar & ~(1u << (stg ^ 1))) | ((((uint32_t)(it + 1) >> 1) & 1u) << (stg ^ 1));
             }
         }
+        const bool all_in = in_tile(kDS - 1);          // the tile's largest sample index
         // ---- phase 1: log-sum-exp over mixtures per (channel, sample), log2 units
 #pragma unroll 4
         for (int t = 0; t < kDS; t++) {
-            const float bx = (t0 + t < T) ? bst[t * kDNP + ch] : 0.f;
+            const float bx = all_in || in_tile(t) ? bst[t * kDNP + ch] : 0.f;
             float q[MM];
 #pragma unroll
             for (int qq = 0; qq < NPR; qq++) {
@@ -345,7 +351,7 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
             const float P = lmax + kLn2 * ptx_lg2(se);
             const float Lh = myslot[tid];
             const float vh = ptx_ex2((Lh - P) * kLog2e);
-            const int64_t tg = t0 + tid;
+            const int64_t tg = split_sample(tile, tid, ntiles);
             const bool valid = tg < T && (a.keep == nullptr || a.keep[tg]);
             vS[tid] = valid ? vh : 0.f;
             if (valid) {
@@ -368,7 +374,9 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
             float* gblk = a.gout + (((size_t)tile * M + h) * 2 + hc) * 4096;
 #pragma unroll 1
             for (int r4 = 0; r4 < kDS; r4 += 4) {
-                float gq[4];
+                float gq[4] = {0.f, 0.f, 0.f, 0.f};
+                const float4 v4 = *reinterpret_cast<const float4*>(vS + r4);
+                if (v4.x != 0.f || v4.y != 0.f || v4.z != 0.f || v4.w != 0.f)   // the same for every thread
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int t = r4 + q;
@@ -376,7 +384,7 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
                     float g = 0.f;
                     if (v != 0.f) {   // the same for every thread of the warp
                         const float nl = -lse[t * kDLL + ch];
-                        const float bx = bst[t * kDNP + ch];   // v != 0: t0 + t < T
+                        const float bx = bst[t * kDNP + ch];   // v != 0: the sample is before T
                         float2 g2 = make_float2(0.f, 0.f);
                         float g1 = 0.f;
 #pragma unroll
@@ -388,7 +396,7 @@ __global__ void __launch_bounds__(kDT, 2) estep_dens_kernel(EStepArgs a) {
                         fS2 = fmaf(v * bb, bb, fS2);
                         fGs += ch_ok ? g : 0.f;
                     }
-                    gq[q] = (ch_ok && t0 + t < T) ? tf32_rna_alu(g) : 0.f;
+                    gq[q] = ch_ok ? tf32_rna_alu(g) : 0.f;   // past T: v = 0, g = 0
                 }
                 *reinterpret_cast<float4*>(gblk + sw128_off(rr, r4, 128) / 4) =
                     make_float4(gq[0], gq[1], gq[2], gq[3]);

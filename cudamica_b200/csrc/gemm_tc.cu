@@ -408,8 +408,9 @@ __global__ void __launch_bounds__(kGxThreads, 1) k_gx_tc(GxArgs a) {
     }
 }
 
-// The x^T operand image: block q holds samples [32 q, 32 q + 32) as a 256 x 32
-// K-major swizzled tile (row = channel); samples past T are zero.
+// The x^T operand image: block q holds the samples of tile q of the density kernel
+// (split_sample) as a 256 x 32 K-major swizzled tile (row = channel); samples past
+// T are zero.
 __global__ void __launch_bounds__(256) k_xt_image(const float* __restrict__ x, int64_t T, int64_t nblocks,
                                                   float* __restrict__ ximg) {
     const int k = threadIdx.x;
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(256) k_xt_image(const float* __restrict__ x, i
             float v[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const int64_t t = q * 32 + c4 * 4 + e;
+                const int64_t t = split_sample(q, c4 * 4 + e, nblocks);
                 v[e] = t < T ? x[(size_t)t * kNP + k] : 0.f;
             }
             *reinterpret_cast<float4*>(ximg + (size_t)q * 8192 + sw128_off(k, c4 * 4, 256) / 4) =
