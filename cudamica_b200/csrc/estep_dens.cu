@@ -11,7 +11,8 @@
 // data (common.cuh, split_sample): the models of consecutive samples are mostly
 // the same, and a model skips the second phase of samples it has no
 // responsibility for, so with 32 consecutive samples one CTA of the cluster
-// worked while the others waited.  n = 256, T = 400k, M = 4, m = 5: FIGURE.
+// worked while the others waited.  E-step at n = 256, T = 400k, M = 4, m = 5: 5.36 ->
+// 4.79 ms.
 //
 // Layout: one thread-block cluster of M CTAs (CTA h = model h) per tile
 // stream, 256 threads per CTA (thread = channel, all 32 samples of a tile),
