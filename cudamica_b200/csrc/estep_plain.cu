@@ -15,6 +15,13 @@
 //      src/amica.cu:1535-1550, with phi formed from Psi in the FP64 M-step).
 // Partial sums go to a per-CTA slot of `partial`; a separate kernel reduces
 // the slots in a fixed order, so results are deterministic.
+//
+// Bound by the FP32 pipe and shared-memory loads of the two products and by MUFU
+// latency with 8 to 12 warps per SM.  E-step, with lanes for 32, 64 or 128 channels,
+// K always the padded count and runs of consecutive samples -> now: n = 71, T =
+// 200k, M = 2, m = 3: 1039 -> 668 us; n = 128, T = 300k, M = 3: 2.51 -> 2.36 ms; n =
+// 256, T = 50k, M = 2, m = 5: 1.27 -> 1.22 ms; n = 100, T = 200k, M = 1: 564 -> 534 us;
+// n = 32, T = 300k, M = 1: 199 -> 205 us.
 #include <cooperative_groups.h>
 #include <cstdio>
 
@@ -28,46 +35,67 @@ using namespace amica;
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kS = 64;  // samples per tile
+// A tile's samples are four consecutive ones from each of 16 segments of the data
+// (sample t of tile: segment t / 4): the models of consecutive samples are mostly
+// the same, and a model skips the second phase of samples it has no
+// responsibility for, so that with a run of samples one CTA of the cluster works
+// while the others wait.
+__device__ __forceinline__ int64_t plain_sample(int64_t tile, int t, int64_t ntiles) {
+    return (int64_t)(t >> 2) * 4 * ntiles + 4 * tile + (t & 3);
+}
 
-// NP: channels padded (32, 64, 128 or 256).  Up to 128 channels one CTA per
-// model holds them all; at 256 the Q = 4 CTAs of a model each own NPL = 64
-// channels (their rows of W, their densities, their rows of Psi) and read the
-// full x tile; their per-sample channel sums are added in the cluster.
-template <int NP>
+// NP: channels as laid out (32, 64, 128 or 256); NA: channels worked on (96 for
+// 65 to 96 of 128).  Up to 128 channels one CTA per model holds them all; at 256
+// the Q = 4 CTAs of a model each own NPL = 64 channels (their rows of W, their
+// densities, their rows of Psi) and read the full x tile; their per-sample channel
+// sums are added in the cluster.
+// 8 warps, 12 with NA = 96.  (16 warps at NA = 128 and 256, with half the register
+// block each, are bound by shared-memory loads in the products: 2.47 against 2.36
+// ms at n = 128, T = 300k, M = 3, and 1.58 against 1.26 at n = 256, T = 50k, M = 2.)
+template <int NP, int NA, int MM>
 struct PlainShape {
-    static constexpr int NPL = NP <= 128 ? NP : 64; // channels of this CTA
-    static constexpr int Q = NP / NPL;              // CTAs per model
-    static constexpr int SPLIT = kThreads / NPL;    // sample groups per channel
+    static constexpr int NPL = NP <= 128 ? NA : 64; // channels of this CTA
+    static constexpr int Q = NP <= 128 ? 1 : NP / NPL;   // CTAs per model
+    static constexpr int THREADS = NPL == 96 ? 384 : 256;
+    static constexpr int SPLIT = THREADS / NPL;     // sample groups per channel
     static constexpr int SUB = kS / SPLIT;          // samples per thread per tile
+    static constexpr int NK = NP <= 128 ? NA : NP;  // columns of W and x held
     static constexpr int WLD = NPL + 4;             // padded row of W^T in smem
-    static constexpr int XLD = NP + 4;              // padded row of the x tile
+    static constexpr int XLD = NK + 4;              // padded row of the x tile
     // GEMM b = W x: each thread 4 channels x CT samples
     static constexpr int NTI = NPL / 4;
-    static constexpr int NTT = kThreads / NTI;
+    static constexpr int NTT = THREADS / NTI;
     static constexpr int CT = kS / NTT;
-    static_assert(NTI * NTT == kThreads && NTT * CT == kS, "b = W x tiling");
-    // Psi update: each thread RI x RK block
+    static_assert(NTI * NTT == THREADS && NTT * CT == kS, "b = W x tiling");
+    // Psi update: each thread RI x RK block, RI in two runs of RI / 2 channels
     static constexpr int RI = NPL / 16;
-    static constexpr int RK = NP / 16;
-    static constexpr int LLD = NPL + 1;             // padded row of the lse tile
-    static constexpr size_t smem_floats =
-        (size_t)NP * WLD + (size_t)kS * XLD + (size_t)kS * NPL + (size_t)kS * LLD +
-                  (size_t)kS * LLD + 2 * kS + 2 * kS;
+    static constexpr int RK = NK / (THREADS / 16);
+    static_assert(RK * (THREADS / 16) == NK && RI % 2 == 0, "Psi tiling");
+    static constexpr int LLD = NPL + 8;             // padded row of the lse tile (8 lanes per sample)
+    static constexpr int NACC = 7 * MM + 3;
+    static constexpr size_t tile_floats = (size_t)kS * (XLD + NPL + NPL + LLD);
+    // FP64 running sums: with 256 threads each keeps those of its own channel and
+    // sample group in registers; with more the groups' FP32 sums are folded through
+    // shared memory (the tile's place) into FP64 sums spread over the threads
+    static constexpr bool REG64 = THREADS == 256;
+    static constexpr size_t fold_floats = (size_t)NACC * THREADS * (REG64 ? 2 : 1);
+    static constexpr size_t work_floats = tile_floats > fold_floats ? tile_floats : fold_floats;
+    static constexpr size_t smem_floats = (size_t)NK * WLD + work_floats + 2 * kS + kS;
+    static constexpr int NFOLD = REG64 ? NACC : (NACC * NPL + THREADS - 1) / THREADS;   // FP64 sums per thread
 };
 
-template <int NP, int MM>
-__global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
-    using Sh = PlainShape<NP>;
-    constexpr int NPL = Sh::NPL, Q = Sh::Q;
+template <int NP, int NA, int MM>
+__global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, 1) estep_plain_kernel(EStepArgs a) {
+    using Sh = PlainShape<NP, NA, MM>;
+    constexpr int NPL = Sh::NPL, Q = Sh::Q, THREADS = Sh::THREADS, NK = Sh::NK, NACC = Sh::NACC;
     extern __shared__ __align__(16) float sm[];
-    float* Wt = sm;                                   // [NP][WLD]  Wt[k][i] = W[i0 + i][k]
-    float* xs = Wt + NP * Sh::WLD;                   // [S][XLD]
-    float* bs = xs + kS * Sh::XLD;                   // [S][NPL]   (W x)_i per sample
-    float* gs = bs + kS * NPL;                        // [S][NPL] g; its region is [S][LLD]
-    float* lse = gs + kS * Sh::LLD;                 // [S][LLD]   log-sum-exp over mixtures
-    float* slot = lse + kS * Sh::LLD;                 // [2][S]     cluster-visible L_h(t)
+    float* Wt = sm;                                   // [NK][WLD]  Wt[k][i] = W[i0 + i][k]
+    float* xs = Wt + NK * Sh::WLD;                    // [S][XLD]
+    float* bs = xs + kS * Sh::XLD;                    // [S][NPL]   (W x)_i per sample
+    float* gs = bs + kS * NPL;                        // [S][NPL]   g
+    float* lse = gs + kS * NPL;                       // [S][LLD]   log-sum-exp over mixtures
+    float* slot = Wt + NK * Sh::WLD + Sh::work_floats;   // [2][S]  cluster-visible L_h(t)
     float* vS = slot + 2 * kS;                        // [S]        v_h(t) (0 if not used)
 
     cg::cluster_group cluster = cg::this_cluster();
@@ -77,16 +105,16 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
     const int cid = blockIdx.x / (a.M * Q);
     const int tid = threadIdx.x;
     const int n = a.n, M = a.M;
-    if (a.m != MM || n > NP) {
+    if (a.m != MM || n > NP || (NP <= 128 && n > NA)) {
         if (tid == 0) atomicOr(a.err, kErrShape);
     }
 
     // ---- resident per-CTA data: W_h^T and this thread's mixture constants
     {
         const float* Wh = a.Wf + ((size_t)h * NP + i0c) * NP;
-        for (int e = tid; e < NPL * NP; e += kThreads) {
-            int i = e / NP, k = e % NP;
-            Wt[k * Sh::WLD + i] = Wh[e];
+        for (int e = tid; e < NPL * NK; e += THREADS) {
+            int i = e / NK, k = e % NK;
+            Wt[k * Sh::WLD + i] = Wh[(size_t)i * NP + k];
         }
     }
     const int ch = tid % NPL;           // density-phase channel (of this CTA)
@@ -97,13 +125,11 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
     constexpr int NPR = MM / 2;
     constexpr bool kOdd = (MM & 1) != 0;
     constexpr int NPRA = NPR > 0 ? NPR : 1;
-    float pr[MM];
     MixV<float2> P2[NPRA];
     MixV<float> P1;
 #pragma unroll
     for (int j = 0; j < MM; j++) {
         const MixParam q = a.mp[((size_t)h * MM + j) * NP + gch];
-        pr[j] = q.rho;
         if (j < 2 * NPR) {
             float2* f[5] = {&P2[j / 2].s, &P2[j / 2].npo, &P2[j / 2].pc, &P2[j / 2].pr, &P2[j / 2].sr};
             const float vals[5] = {q.s, -q.off, q.cl2, q.rho, q.s * q.rho};
@@ -117,17 +143,71 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
         }
     }
     const float wci = a.wc[(size_t)h * NP + gch];
-    float ltc[kMaxModels];
-#pragma unroll
-    for (int q = 0; q < kMaxModels; q++) ltc[q] = (q < M) ? (float)(a.ltc64[q] - a.ltc64[0]) : 0.f;
+    // this model's offset of Lt (with Q > 1 the per-sample threads add every model's;
+    // eight more registers for them measured 4% slower at n = 256)
+    const float ltch = (float)(a.ltc64[h] - a.ltc64[0]);
 
-    // FP64 running sums for this thread's channel: A0..A6 of dens_acc per mixture
-    double dA[7][MM];
+    // FP32 sums of this thread's channel and sample group: A0..A6 of dens_acc per
+    // mixture, sum v b, sum v b^2, sum g
+    float2 fP[NPRA][7];
+    float fS1[7], fCn, fS2, fGs;
+    auto zero_sums = [&]() {
 #pragma unroll
-    for (int k = 0; k < 7; k++)
+        for (int k = 0; k < 7; k++) {
 #pragma unroll
-        for (int j = 0; j < MM; j++) dA[k][j] = 0.0;
-    double dCn = 0.0, dS2 = 0.0, dGs = 0.0;
+            for (int qq = 0; qq < NPRA; qq++) fP[qq][k] = make_float2(0.f, 0.f);
+            fS1[k] = 0.f;
+        }
+        fCn = fS2 = fGs = 0.f;
+    };
+    zero_sums();
+    // FP64 running sums: REG64, this thread's NACC; else thread e owns the (sum, channel)
+    // pairs e, e + THREADS, ... of NACC x NPL, the groups added in order
+    double dF[Sh::NFOLD];
+#pragma unroll
+    for (int u = 0; u < Sh::NFOLD; u++) dF[u] = 0.0;
+    auto fold = [&]() {                               // not REG64: between two barriers
+        if constexpr (Sh::REG64) {
+#pragma unroll
+            for (int k = 0; k < 7; k++) {
+#pragma unroll
+                for (int qq = 0; qq < NPR; qq++) {
+                    dF[k * MM + 2 * qq] += fP[qq][k].x;
+                    dF[k * MM + 2 * qq + 1] += fP[qq][k].y;
+                }
+                if constexpr (kOdd) dF[k * MM + MM - 1] += fS1[k];
+            }
+            dF[7 * MM + 0] += fCn;
+            dF[7 * MM + 1] += fS2;
+            dF[7 * MM + 2] += fGs;
+            zero_sums();
+            return;
+        }
+        float* fb = xs;
+#pragma unroll
+        for (int k = 0; k < 7; k++) {
+#pragma unroll
+            for (int qq = 0; qq < NPR; qq++) {
+                fb[(k * MM + 2 * qq) * THREADS + tid] = fP[qq][k].x;
+                fb[(k * MM + 2 * qq + 1) * THREADS + tid] = fP[qq][k].y;
+            }
+            if constexpr (kOdd) fb[(k * MM + MM - 1) * THREADS + tid] = fS1[k];
+        }
+        fb[(7 * MM + 0) * THREADS + tid] = fCn;
+        fb[(7 * MM + 1) * THREADS + tid] = fS2;
+        fb[(7 * MM + 2) * THREADS + tid] = fGs;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < Sh::NFOLD; u++) {
+            const int e = tid + u * THREADS;
+            if (e < NACC * NPL) {
+                const int k = e / NPL, c = e - k * NPL;
+#pragma unroll
+                for (int g = 0; g < Sh::SPLIT; g++) dF[u] += (double)fb[k * THREADS + g * NPL + c];
+            }
+        }
+        zero_sums();
+    };
     double dLL = 0.0, dVs = 0.0;   // per-sample threads (tid < S)
     constexpr int PRI = Sh::RI, PRK = Sh::RK;
     float psi[PRI][PRK];
@@ -135,16 +215,18 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
     for (int r = 0; r < PRI; r++)
 #pragma unroll
         for (int c = 0; c < PRK; c++) psi[r][c] = 0.f;
+    const int kend = NK < ((n + 3) & ~3) ? NK : ((n + 3) & ~3);   // W and x are zero beyond n
 
-    int par = 0;
-    for (int tile = cid; tile < a.ntiles; tile += a.nclusters, par ^= 1) {
-        const int64_t t0 = (int64_t)tile * kS;
-        {
-        // ---- stage the x tile (float4, coalesced; rows past T are zero)
-        for (int e = tid; e < kS * (NP / 4); e += kThreads) {
-            int t = e / (NP / 4), k4 = e % (NP / 4);
+    int it = 0;
+    for (int tile = cid; tile < a.ntiles; tile += a.nclusters, it++) {
+        const int par = it & 1;
+        __syncthreads();                              // the last tile's (or fold's) readers are done
+        // ---- stage the x tile (float4, coalesced; samples past T are zero)
+        for (int e = tid; e < kS * (NK / 4); e += THREADS) {
+            const int t = e / (NK / 4), k4 = e % (NK / 4);
+            const int64_t ts = plain_sample(tile, t, a.ntiles);
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t0 + t < a.T) v = reinterpret_cast<const float4*>(a.x + (t0 + t) * a.ldx)[k4];
+            if (ts < a.T) v = reinterpret_cast<const float4*>(a.x + ts * a.ldx)[k4];
             *reinterpret_cast<float4*>(xs + t * Sh::XLD + 4 * k4) = v;
         }
         __syncthreads();
@@ -157,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
 #pragma unroll
                 for (int q = 0; q < 4; q++) acc[c][q] = 0.f;
 #pragma unroll 2
-            for (int k = 0; k < NP; k += 4) {
+            for (int k = 0; k < kend; k += 4) {
                 float4 w0 = *reinterpret_cast<const float4*>(Wt + (k + 0) * Sh::WLD + 4 * ti);
                 float4 w1 = *reinterpret_cast<const float4*>(Wt + (k + 1) * Sh::WLD + 4 * ti);
                 float4 w2 = *reinterpret_cast<const float4*>(Wt + (k + 2) * Sh::WLD + 4 * ti);
@@ -180,7 +262,6 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
                 *reinterpret_cast<float4*>(bs + (tt * Sh::CT + c) * NPL + 4 * ti) =
                     make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
         }
-        }
         __syncthreads();
         // ---- phase 1: per (channel, sample) log-sum-exp over mixtures (log2 units)
 #pragma unroll 4
@@ -201,17 +282,21 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
             lse[t * Sh::LLD + ch] = ch_ok ? lse2<MM>(q) : 0.f;
         }
         __syncthreads();
-        // ---- Lt_h(t): channel sum in fixed order, published for the cluster
-        // (with Q > 1, this CTA's channels only; the blocks are added below)
+        // ---- Lt_h(t): the channel sum by 8 lanes per sample in a fixed
+        // order, published for the cluster (with Q > 1, this CTA's channels only; the
+        // blocks are added below)
         float* myslot = slot + par * kS;
-        if (tid < kS) {
-            float s = 0.f;
-            if constexpr (Q == 1) {
-                for (int i = 0; i < n; i++) s += lse[tid * Sh::LLD + i];
-                myslot[tid] = ltc[h] + kLn2 * s;
-            } else {
-                for (int i = 0; i < NPL; i++) s += lse[tid * Sh::LLD + i];
-                myslot[tid] = s;
+        if (tid < 256) {                              // two rounds of 32 samples
+#pragma unroll
+            for (int t0r = 0; t0r < kS; t0r += 32) {
+                const int t = t0r + (tid >> 3), j = tid & 7;
+                float s = 0.f;
+#pragma unroll
+                for (int i = 0; i < NPL / 8; i++) s += lse[t * Sh::LLD + 8 * i + j];
+                s += __shfl_xor_sync(0xffffffffu, s, 4);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                if (j == 0) myslot[t] = Q == 1 ? ltch + kLn2 * s : s;
             }
         }
         cluster.sync();
@@ -229,18 +314,21 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
                         float s = 0.f;
 #pragma unroll
                         for (int b = 0; b < Q; b++) s += cluster.map_shared_rank(myslot, q * Q + b)[tid];
-                        L[q] = ltc[q] + kLn2 * s;
+                        L[q] = (float)(a.ltc64[q] - a.ltc64[0]) + kLn2 * s;
                     }
                     lmax = fmaxf(lmax, L[q]);
                 }
             }
-            float se = 0.f;
+            float se = 0.f, Lh = 0.f;
 #pragma unroll
             for (int q = 0; q < kMaxModels; q++)
-                if (q < M) se += ptx_ex2((L[q] - lmax) * kLog2e);
+                if (q < M) {
+                    se += ptx_ex2((L[q] - lmax) * kLog2e);
+                    if (q == h) Lh = L[q];
+                }
             const float P = lmax + kLn2 * ptx_lg2(se);
-            const float vh = ptx_ex2((L[h] - P) * kLog2e);
-            const int64_t tg = t0 + tid;
+            const float vh = ptx_ex2((Lh - P) * kLog2e);
+            const int64_t tg = plain_sample(tile, tid, a.ntiles);
             const bool valid = tg < a.T && (a.keep == nullptr || a.keep[tg]);
             vS[tid] = valid ? vh : 0.f;
             if (valid && cq == 0) {
@@ -248,22 +336,13 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
                 if (h == 0) dLL += (double)P;
             }
             if (tg < a.T && cq == 0) {
-                if (a.Lt_out) a.Lt_out[(size_t)h * a.T + tg] = L[h];
+                if (a.Lt_out) a.Lt_out[(size_t)h * a.T + tg] = Lh;
                 if (a.P_out && h == 0) a.P_out[tg] = P;
             }
         }
         __syncthreads();
         // ---- phase 2: responsibilities, score function and sufficient statistics
         {
-            float2 fP[NPRA][7];
-            float fS1[7];
-#pragma unroll
-            for (int k = 0; k < 7; k++) {
-#pragma unroll
-                for (int qq = 0; qq < NPRA; qq++) fP[qq][k] = make_float2(0.f, 0.f);
-                fS1[k] = 0.f;
-            }
-            float fCn = 0.f, fS2 = 0.f, fGs = 0.f;
             // the densities, responsibilities and sums of tile sample t; returns g
             auto sample = [&](int t) -> float {
                 const float v = vS[t];
@@ -285,98 +364,113 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
                 fGs += ch_ok ? g : 0.f;
                 return g;
             };
-            {
 #pragma unroll 2
-                for (int r = 0; r < Sh::SUB; r++) {
-                    const int t = grp * Sh::SUB + r;
-                    const float g = sample(t);
-                    gs[t * NPL + ch] = ch_ok ? g : 0.f;
-                }
-            }
-            if (ch_ok) {
-#pragma unroll
-                for (int k = 0; k < 7; k++) {
-#pragma unroll
-                    for (int qq = 0; qq < NPR; qq++) {
-                        dA[k][2 * qq] += fP[qq][k].x;
-                        dA[k][2 * qq + 1] += fP[qq][k].y;
-                    }
-                    if constexpr (kOdd) dA[k][MM - 1] += fS1[k];
-                }
-                dCn += fCn; dS2 += fS2; dGs += fGs;
+            for (int r = 0; r < Sh::SUB; r++) {
+                const int t = grp * Sh::SUB + r;
+                const float g = sample(t);
+                gs[t * NPL + ch] = ch_ok ? g : 0.f;
             }
         }
+        if constexpr (Sh::REG64) fold();
         __syncthreads();
-        // ---- Psi_h += g x^T over the tile (thread: RI x RK block)
+        // ---- Psi_h += g x^T over the tile (thread: RI x RK block, its channels in two
+        // runs NPL / 2 apart, so that a warp's loads of g are free of bank conflicts)
         {
             const int pi = tid % 16, pk = tid / 16;
-            const int i0 = pi * Sh::RI, k0 = pk * Sh::RK;
+            const int i0 = pi * (PRI / 2), k0 = pk * PRK;
+            if (k0 < kend) {
 #pragma unroll 4
-            for (int t = 0; t < kS; t++) {
-                float gv[Sh::RI], xv[Sh::RK];
+                for (int t = 0; t < kS; t++) {
+                    float gv[PRI], xv[PRK];
 #pragma unroll
-                for (int r = 0; r < Sh::RI; r++) gv[r] = gs[t * NPL + i0 + r];
+                    for (int r = 0; r < PRI; r++) gv[r] = gs[t * NPL + (r >= PRI / 2 ? NPL / 2 - PRI / 2 : 0) + i0 + r];
 #pragma unroll
-                for (int c = 0; c < Sh::RK; c++) xv[c] = xs[t * Sh::XLD + k0 + c];
+                    for (int c = 0; c < PRK; c++) xv[c] = xs[t * Sh::XLD + k0 + c];
 #pragma unroll
-                for (int r = 0; r < Sh::RI; r++)
+                    for (int r = 0; r < PRI; r++)
 #pragma unroll
-                    for (int c = 0; c < Sh::RK; c++) psi[r][c] = fmaf(gv[r], xv[c], psi[r][c]);
+                        for (int c = 0; c < PRK; c++) psi[r][c] = fmaf(gv[r], xv[c], psi[r][c]);
+                }
             }
         }
-        __syncthreads();
+        // FP32 sums cover at most 32 samples of a thread before they go to FP64
+        if (!Sh::REG64 && par == 1) {
+            __syncthreads();
+            fold();
+        }
     }
+    __syncthreads();
+    if constexpr (!Sh::REG64) fold();
 
-    // ---- write this CTA's partial sums (fixed-order combination of groups)
+    // ---- write this CTA's partial sums
     PartLayout L{n, MM};
     // one slot per (cluster, channel block); entries of the other blocks stay zero
     double* out = a.partial + ((size_t)(cid * Q + cq) * M + h) * L.stride();
-    double* red = reinterpret_cast<double*>(xs);   // [SPLIT][NPL] doubles, one statistic at a time
-    constexpr int NACC = 7 * MM + 3;
-    double vals[NACC];
+    // the FP64 sums of a channel side by side, then mapped to the statistics
+    double* red = reinterpret_cast<double*>(xs);      // [NACC][NPL]
+    static_assert((size_t)NACC * NPL * 2 <= Sh::work_floats, "final sums");
+    __syncthreads();
+    if constexpr (Sh::REG64) {
 #pragma unroll
-    for (int j = 0; j < MM; j++) {
-        mix_stats_from_sums(dA[0][j], dA[1][j], dA[2][j], dA[3][j], dA[4][j], dA[5][j], dA[6][j],
-                            pr[j], a.grad_mode, a.update_rho, vals[kUs * MM + j], vals[kKn * MM + j],
-                            vals[kLn * MM + j], vals[kMn * MM + j], vals[kMd * MM + j],
-                            vals[kBd * MM + j], vals[kRn * MM + j]);
-    }
-    vals[7 * MM + 0] = dCn; vals[7 * MM + 1] = dS2; vals[7 * MM + 2] = dGs;
-#pragma unroll
-    for (int k = 0; k < NACC; k++) {
-        red[grp * NPL + ch] = vals[k];
+        for (int k = 0; k < NACC; k++) red[k * THREADS + tid] = dF[k];
         __syncthreads();
-        if (tid < NPL && i0c + tid < n) {
-            double s = 0.0;
-            for (int g2 = 0; g2 < Sh::SPLIT; g2++) s += red[g2 * NPL + tid];
-            const int gi = i0c + tid;
-            int dst;
-            if (k < 7 * MM) dst = L.mix(k / MM) + (k % MM) * n + gi;
-            else if (k == 7 * MM) dst = L.cn() + gi;
-            else if (k == 7 * MM + 1) dst = L.s2() + gi;
-            else dst = L.gs() + gi;
-            out[dst] = s;
+        double s[(NACC * NPL + THREADS - 1) / THREADS];   // the groups added in order
+#pragma unroll
+        for (int u = 0; u * THREADS < NACC * NPL; u++) {
+            const int e = tid + u * THREADS;
+            s[u] = 0.0;
+            if (e < NACC * NPL)
+#pragma unroll
+                for (int g = 0; g < Sh::SPLIT; g++) s[u] += red[(e / NPL) * THREADS + g * NPL + e % NPL];
         }
         __syncthreads();
+#pragma unroll
+        for (int u = 0; u * THREADS < NACC * NPL; u++)
+            if (tid + u * THREADS < NACC * NPL) red[tid + u * THREADS] = s[u];
+    } else {
+#pragma unroll
+        for (int u = 0; u < Sh::NFOLD; u++) {
+            const int e = tid + u * THREADS;
+            if (e < NACC * NPL) red[e] = dF[u];
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < MM * NPL; e += THREADS) {
+        const int j = e / NPL, c = e - j * NPL, gi = i0c + c;
+        if (gi >= n) continue;
+        const float rho = a.mp[((size_t)h * MM + j) * NP + gi].rho;
+        auto A = [&](int k) { return red[(k * MM + j) * NPL + c]; };
+        double v[7];
+        mix_stats_from_sums(A(0), A(1), A(2), A(3), A(4), A(5), A(6), rho, a.grad_mode, a.update_rho, v[kUs],
+                            v[kKn], v[kLn], v[kMn], v[kMd], v[kBd], v[kRn]);
+#pragma unroll
+        for (int k = 0; k < 7; k++) out[L.mix(k) + j * n + gi] = v[k];
+    }
+    for (int c = tid; c < NPL; c += THREADS) {
+        const int gi = i0c + c;
+        if (gi >= n) continue;
+        out[L.cn() + gi] = red[(7 * MM + 0) * NPL + c];
+        out[L.s2() + gi] = red[(7 * MM + 1) * NPL + c];
+        out[L.gs() + gi] = red[(7 * MM + 2) * NPL + c];
     }
     // LL numerator and vsum: per-sample threads, combined in fixed order
-    double* red2 = red;
-    if (tid < kS) { red2[tid] = dLL; red2[kS + tid] = dVs; }
+    __syncthreads();
+    if (tid < kS) { red[tid] = dLL; red[kS + tid] = dVs; }
     __syncthreads();
     if (tid == 0 && cq == 0) {
         double s0 = 0.0, s1 = 0.0;
-        for (int t = 0; t < kS; t++) { s0 += red2[t]; s1 += red2[kS + t]; }
+        for (int t = 0; t < kS; t++) { s0 += red[t]; s1 += red[kS + t]; }
         out[0] = s0;
         out[1] = s1;
     }
     {
         const int pi = tid % 16, pk = tid / 16;
-        const int i0 = pi * Sh::RI, k0 = pk * Sh::RK;
+        const int i0 = pi * (PRI / 2), k0 = pk * PRK;
 #pragma unroll
-        for (int r = 0; r < Sh::RI; r++)
+        for (int r = 0; r < PRI; r++)
 #pragma unroll
-            for (int c = 0; c < Sh::RK; c++) {
-                const int i = i0c + i0 + r, k = k0 + c;
+            for (int c = 0; c < PRK; c++) {
+                const int i = i0c + (r >= PRI / 2 ? NPL / 2 - PRI / 2 : 0) + i0 + r, k = k0 + c;
                 if (i < n && k < n) out[L.psi() + (size_t)k * n + i] = (double)psi[r][c];
             }
     }
@@ -384,31 +478,59 @@ __global__ void __launch_bounds__(kThreads, 1) estep_plain_kernel(EStepArgs a) {
     cluster.sync();
 }
 
-template <int NP, int MM>
-cudaError_t launch_plain(const EStepArgs& a, int nclusters, cudaStream_t st) {
-    using Sh = PlainShape<NP>;
+// The launch of a shape, ready but for its grid.
+template <int NP, int NA, int MM>
+cudaError_t plain_config(int M, int nclusters, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+    using Sh = PlainShape<NP, NA, MM>;
+    auto kern = estep_plain_kernel<NP, NA, MM>;
     const size_t smem = Sh::smem_floats * sizeof(float);
-    auto kern = estep_plain_kernel<NP, MM>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    if (a.M * Sh::Q > 1) {
+    const int csize = M * Sh::Q;
+    if (csize > 8) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nclusters * a.M * Sh::Q);
-    cfg.blockDim = dim3(kThreads);
+    cfg = {};
+    cfg.gridDim = dim3(nclusters * csize);
+    cfg.blockDim = dim3(Sh::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.M * Sh::Q;
+    attr[0].val.clusterDim.x = csize;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, a);
+    return cudaSuccess;
 }
+
+template <int NP, int NA, int MM>
+cudaError_t launch_plain(const EStepArgs& a, int nclusters, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    const cudaError_t e = plain_config<NP, NA, MM>(a.M, nclusters, st, cfg, attr);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&cfg, estep_plain_kernel<NP, NA, MM>, a);
+}
+
+// Largest cluster count whose clusters can all be resident at once (the grid
+// is persistent: every cluster loops over its share of the tiles).
+template <int NP, int NA, int MM>
+int max_active_clusters(int M) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    if (plain_config<NP, NA, MM>(M, 64, nullptr, cfg, attr) != cudaSuccess) return -1;
+    int num = 0;
+    if (cudaOccupancyMaxActiveClusters(&num, estep_plain_kernel<NP, NA, MM>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    return num;
+}
+
+// channels worked on: 65 to 96 of 128 take three quarters of the lanes
+int plain_work_channels(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 96 ? 96 : n <= 128 ? 128 : 256; }
 
 }  // namespace
 
@@ -420,71 +542,35 @@ int plain_pad_channels(int n) {
     return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : (n <= 256 ? 256 : -1)));
 }
 // Partial-sum slots per cluster: one per channel block.
-int plain_partial_groups(int n) { return plain_pad_channels(n) == 256 ? PlainShape<256>::Q : 1; }
+int plain_partial_groups(int n) { return plain_pad_channels(n) == 256 ? PlainShape<256, 256, 1>::Q : 1; }
 
-// Largest cluster count whose clusters can all be resident at once (the grid
-// is persistent: every cluster loops over its share of the tiles).
-template <int NP, int MM>
-int max_active_clusters(int M) {
-    using Sh = PlainShape<NP>;
-    const size_t smem = Sh::smem_floats * sizeof(float);
-    auto kern = estep_plain_kernel<NP, MM>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return -1;
-    const int csize = M * Sh::Q;
-    if (csize > 8 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return -1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(csize * 64);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csize;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, kern, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return -1;
-    }
-    return num;
-}
+#define AMICA_PLAIN_EACH_M(NPV, NAV) \
+    AMICA_PLAIN_CASE(NPV, NAV, 1) AMICA_PLAIN_CASE(NPV, NAV, 2) AMICA_PLAIN_CASE(NPV, NAV, 3) \
+    AMICA_PLAIN_CASE(NPV, NAV, 4) AMICA_PLAIN_CASE(NPV, NAV, 5)
+#define AMICA_PLAIN_EACH \
+    AMICA_PLAIN_EACH_M(32, 32) AMICA_PLAIN_EACH_M(64, 64) AMICA_PLAIN_EACH_M(128, 96) \
+    AMICA_PLAIN_EACH_M(128, 128) AMICA_PLAIN_EACH_M(256, 256)
 
 int plain_max_clusters(int n, int m, int M) {
-    const int NP = plain_pad_channels(n);
-    if (NP < 0 || m < 1 || m > 5 || M < 1 || M > kMaxModels) return -1;
-#define AMICA_PLAIN_OCC(NPV, MMV) \
-    if (NP == NPV && m == MMV) return max_active_clusters<NPV, MMV>(M);
-#define AMICA_PLAIN_OCC_NP(NPV) \
-    AMICA_PLAIN_OCC(NPV, 1) AMICA_PLAIN_OCC(NPV, 2) AMICA_PLAIN_OCC(NPV, 3) \
-    AMICA_PLAIN_OCC(NPV, 4) AMICA_PLAIN_OCC(NPV, 5)
-    AMICA_PLAIN_OCC_NP(32)
-    AMICA_PLAIN_OCC_NP(64)
-    AMICA_PLAIN_OCC_NP(128)
-    AMICA_PLAIN_OCC_NP(256)
-#undef AMICA_PLAIN_OCC_NP
-#undef AMICA_PLAIN_OCC
+    if (plain_pad_channels(n) < 0 || m < 1 || m > 5 || M < 1 || M > kMaxModels) return -1;
+    const int NA = plain_work_channels(n);
+#define AMICA_PLAIN_CASE(NPV, NAV, MMV) \
+    if (NA == NAV && m == MMV) return max_active_clusters<NPV, NAV, MMV>(M);
+    AMICA_PLAIN_EACH
+#undef AMICA_PLAIN_CASE
     return -1;
 }
 
 cudaError_t launch_estep_plain(const EStepArgs& a, int NP, int nclusters, cudaStream_t st) {
-#define AMICA_PLAIN_CASE(NPV, MMV) \
-    if (NP == NPV && a.m == MMV) return launch_plain<NPV, MMV>(a, nclusters, st);
-#define AMICA_PLAIN_NP(NPV) \
-    AMICA_PLAIN_CASE(NPV, 1) AMICA_PLAIN_CASE(NPV, 2) AMICA_PLAIN_CASE(NPV, 3) \
-    AMICA_PLAIN_CASE(NPV, 4) AMICA_PLAIN_CASE(NPV, 5)
-    AMICA_PLAIN_NP(32)
-    AMICA_PLAIN_NP(64)
-    AMICA_PLAIN_NP(128)
-    AMICA_PLAIN_NP(256)
-#undef AMICA_PLAIN_NP
+    const int NA = plain_work_channels(a.n);
+#define AMICA_PLAIN_CASE(NPV, NAV, MMV) \
+    if (NP == NPV && NA == NAV && a.m == MMV) return launch_plain<NPV, NAV, MMV>(a, nclusters, st);
+    AMICA_PLAIN_EACH
 #undef AMICA_PLAIN_CASE
     return cudaErrorInvalidValue;
 }
+#undef AMICA_PLAIN_EACH
+#undef AMICA_PLAIN_EACH_M
 
 // the split mixed form (128 < n <= 256) runs its density-only kernel on the
 // channels this form pads to 256
