@@ -223,14 +223,24 @@ __global__ void __launch_bounds__(kWxThreads, 1)
             if (!ok) break;
             tc_fence_after();
             const int64_t t0 = (kt0 + kt) * kWxN;
+            // the pointer walks the rows, and only the last tile checks for the end
+            // (a multiplication and a comparison per store made this loop, 24
+            // instructions a sample, what bounded the kernel)
+            float* bp = Bout + (size_t)t0 * ldb;
+            const int left = a.T - t0 < kWxN ? (int)(a.T - t0) : kWxN;
 #pragma unroll 1
             for (int c0 = 0; c0 < kWxN; c0 += 16) {
                 float vh[16], vl[16];
                 tmem_ld16(tmem + lane_addr + kWxDhi + (uint32_t)(d * kWxN + c0), vh);
                 tmem_ld16(tmem + lane_addr + kWxDlo + (uint32_t)(d * kWxN + c0), vl);
+                if (left == kWxN) {
 #pragma unroll
-                for (int s = 0; s < 16; s++)
-                    if (t0 + c0 + s < a.T) Bout[(size_t)(t0 + c0 + s) * ldb] = vh[s] + vl[s];
+                    for (int s = 0; s < 16; s++, bp += ldb) *bp = vh[s] + vl[s];
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 16; s++, bp += ldb)
+                        if (c0 + s < left) *bp = vh[s] + vl[s];
+                }
             }
             tc_fence_before();
             __syncwarp();
