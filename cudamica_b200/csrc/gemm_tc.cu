@@ -223,9 +223,10 @@ __global__ void __launch_bounds__(kWxThreads, 1)
             if (!ok) break;
             tc_fence_after();
             const int64_t t0 = (kt0 + kt) * kWxN;
-            // the pointer walks the rows, and only the last tile checks for the end
-            // (a multiplication and a comparison per store made this loop, 24
-            // instructions a sample, what bounded the kernel)
+            // the pointer walks the rows, and only the last tile checks for the end:
+            // with a multiplication and a comparison per store this loop took 24
+            // instructions a sample instead of 10, and the kernel 339 us instead of
+            // 324 at n = 256, T = 100k, M = 4
             float* bp = Bout + (size_t)t0 * ldb;
             const int left = a.T - t0 < kWxN ? (int)(a.T - t0) : kWxN;
 #pragma unroll 1

@@ -31,16 +31,19 @@ constexpr int kT = 256;
 //   a(i, k) <- -a(i, k) / a(p, k),   a(i, j) <- a(i, j) - a(i, k) a(p, j) / a(p, k),
 // turns column k into column p_k of P.A^{-1}, so at the end W(j, p_k) = a(p_j, k).
 //
-// Columns are swept in panels of 16.  Warps 0-1 sweep a panel's columns alone
-// (thread r holds rows r and r + 64 of the panel in registers): the pivot of
+// Columns are swept in panels of 16.  Warps 0-3 sweep a panel's columns alone
+// (thread r holds row r of the panel in registers): the pivot of
 // column k only depends on column k as updated by the earlier pivots, and those
 // updates only read the pivot rows' panel entries.  The pivot key of a row is
 // the high word of |a| with its low 7 bits replaced by 127 - row (so the pivot
 // is within 2^-13 of the column's largest |a|, lowest row on ties); each warp's
 // best row publishes its panel row and its reciprocal (every row forms the
-// reciprocal of its candidate while the warp max runs), and after one 64-thread
-// barrier every thread takes the larger key, updates the next column first and
-// starts the next search before the rest of its rows.
+// reciprocal of its candidate while the warp max runs), and after one 128-thread
+// barrier every thread takes the largest key, updates the next column first and
+// starts the next search before the rest of its row.  What bounds the kernel is
+// this chain of n dependent pivots: with one row a thread it is shorter than
+// with two rows on two warps (the kernels around the E-step at n = 64: 74 -> 65
+// us, n = 128: 127 -> 115, n = 32: 43 -> 39, one model).
 //
 // Sweeping a panel's pivots (P, K) one after another is, on the other columns
 // C, the block sweep
@@ -48,7 +51,7 @@ constexpr int kT = 256;
 // X being the swept panel: FP64 products on the tensor cores (mma.sync
 // m8n8k4; tcgen05 has no FP64 kind) with operands in shared memory.  The
 // next panel's columns get it first (all warps), then warps 4-15 apply it to
-// the remaining columns while warps 0-1 sweep the next panel.
+// the remaining columns while warps 0-3 sweep the next panel.
 constexpr int kInvThreads = 512;
 constexpr int kInvN = 128;                            // padded order
 constexpr int kPanel = 16;                            // columns per panel
@@ -56,7 +59,7 @@ constexpr int kLdA = kInvN + 1;                       // odd: a warp reading a c
 constexpr int kLdX = kPanel + 4;                      // 16-byte rows; 40-word stride puts an 8 x 4 fragment on distinct banks
 constexpr size_t kInvSmem = sizeof(double) * ((size_t)kInvN * kLdA + 3 * (size_t)kInvN * kLdX);
 
-__device__ __forceinline__ void bar_panel() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+__device__ __forceinline__ void bar_panel() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // pivot key of row r holding v (0: not a candidate)
 __device__ __forceinline__ uint32_t pivot_key(double v, bool usable, int r) {
@@ -110,9 +113,9 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
     double* As = smem_inv;                            // a(r, j) at As[r * kLdA + j]
     double* Xs = As + kInvN * kLdA;                   // swept panels, two buffers: Xs[b & 1][r * kLdX + t]
     double* Pt = Xs + 2 * kInvN * kLdX;               // Pt[j * kLdX + t] = a(p_t, j) before the panel's update
-    __shared__ __align__(16) double crow_v[2][2][kPanel];   // each panel warp's candidate row
-    __shared__ uint32_t ckey[2][2];
-    __shared__ double cpiv[2][2], cinv[2][2];
+    __shared__ __align__(16) double crow_v[2][4][kPanel];   // each panel warp's candidate row
+    __shared__ __align__(16) uint32_t ckey[2][4];
+    __shared__ double cpiv[2][4], cinv[2][4];
     __shared__ double pivs[kInvN], wcs[kInvN], cperm[kInvN], cs[kInvN];
     __shared__ float sb_cl2[kMaxMix * kInvN];      // log2 normaliser per (mixture, channel)
     __shared__ int perm[kInvN], pinv[kInvN];
@@ -130,25 +133,21 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
         }
     if (tid < kInvN) pinv[tid] = 0x7fffffff;
     if (tid == 0) s_bad = 0;
-    // panel threads (tid < 64): rows r0 = tid and r1 = tid + 64, not yet pivot rows
-    const int r0 = tid, r1 = tid + 64;
-    bool us0 = r0 < n, us1 = r1 < n;
+    // panel threads (tid < 128): row r0 = tid, not yet a pivot row
+    const int r0 = tid;
+    bool us0 = r0 < n;
     const int npan = (n + kPanel - 1) / kPanel;
     __syncthreads();
     for (int b = 0; b <= npan; b++) {
         const int k0 = kPanel * b;
-        if (b < npan && warp < 2) {
+        if (b < npan && warp < 4) {
             double* Xb = Xs + (b & 1) * kInvN * kLdX;
-            double pa[kPanel], pb[kPanel];            // rows r0 and r1
+            double pa[kPanel];
 #pragma unroll
-            for (int t = 0; t < kPanel; t++) {
-                pa[t] = As[r0 * kLdA + k0 + t];
-                pb[t] = As[r1 * kLdA + k0 + t];
-            }
+            for (int t = 0; t < kPanel; t++) pa[t] = As[r0 * kLdA + k0 + t];
             bool bad = false;
-            uint32_t ka = pivot_key(pa[0], us0, r0), kb = pivot_key(pb[0], us1, r1);
-            uint32_t key = max(ka, kb);
-            double v = kb > ka ? pb[0] : pa[0];
+            uint32_t key = pivot_key(pa[0], us0, r0);
+            double v = pa[0];
             double rv = 1.0 / v;
             uint32_t wkey = __reduce_max_sync(0xffffffffu, key);
 #pragma unroll
@@ -158,42 +157,33 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
                 if (wkey == 0u) {
                     if (lane == 0) ckey[buf][warp] = 0u;
                 } else if (key == wkey) {             // one thread: the key names its row
-                    const bool second = kb == key;
 #pragma unroll
                     for (int j = 0; j < kPanel; j += 2)
-                        *reinterpret_cast<double2*>(&crow_v[buf][warp][j]) =
-                            second ? make_double2(pb[j], pb[j + 1]) : make_double2(pa[j], pa[j + 1]);
+                        *reinterpret_cast<double2*>(&crow_v[buf][warp][j]) = make_double2(pa[j], pa[j + 1]);
                     ckey[buf][warp] = key;
                     cpiv[buf][warp] = v;
                     cinv[buf][warp] = rv;
                 }
                 bar_panel();
-                const uint32_t kw0 = ckey[buf][0], kw1 = ckey[buf][1];
-                const int wb = kw1 > kw0 ? 1 : 0;     // distinct unless both 0
-                const uint32_t best = max(kw0, kw1);
-                const double piv = wb ? cpiv[buf][1] : cpiv[buf][0];
-                const double inv = wb ? cinv[buf][1] : cinv[buf][0];
-                const int tn = t + 1 < kPanel ? t + 1 : t;
-                const double pn = wb ? crow_v[buf][1][tn] : crow_v[buf][0][tn];
-                if (best == 0u || piv == 0.0) { bad = true; break; }   // same in every panel thread
-                const int p = 127 - (int)((best - 128u) & 127u);
+                const uint4 kw = *reinterpret_cast<const uint4*>(ckey[buf]);
+                const uint32_t best = max(max(kw.x, kw.y), max(kw.z, kw.w));
+                const int p = 127 - (int)((best - 128u) & 127u), wb = p >> 5;
+                const double piv = cpiv[buf][wb], inv = cinv[buf][wb];
                 const double* pp = crow_v[buf][wb];
+                const double pn = pp[t + 1 < kPanel ? t + 1 : t];
+                if (best == 0u || piv == 0.0) { bad = true; break; }   // same in every panel thread
                 if (tid == 0) { perm[k0 + t] = p; pinv[p] = k0 + t; pivs[k0 + t] = piv; }
-                const bool pa_is_p = r0 == p, pb_is_p = r1 == p;
-                us0 = us0 && !pa_is_p;
-                us1 = us1 && !pb_is_p;
-                const double fa = pa[t] * inv, fb = pb[t] * inv;
+                const bool is_p = r0 == p;
+                us0 = us0 && !is_p;
+                const double fa = pa[t] * inv;
                 if (t + 1 < kPanel) {                 // the next column first, and the next search
                     pa[t + 1] = fma(-fa, pn, pa[t + 1]);
-                    pb[t + 1] = fma(-fb, pn, pb[t + 1]);
-                    ka = pivot_key(pa[t + 1], us0, r0);
-                    kb = pivot_key(pb[t + 1], us1, r1);
-                    key = max(ka, kb);
-                    v = kb > ka ? pb[t + 1] : pa[t + 1];
+                    key = pivot_key(pa[t + 1], us0, r0);
+                    v = pa[t + 1];
                     rv = 1.0 / v;
                     wkey = __reduce_max_sync(0xffffffffu, key);
                 }
-                double ppv[kPanel];                   // the pivot row, read once for both rows
+                double ppv[kPanel];                   // the pivot row
 #pragma unroll
                 for (int j = 0; j < kPanel; j += 2) {
                     const double2 d = *reinterpret_cast<const double2*>(pp + j);
@@ -202,35 +192,22 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
                 }
 #pragma unroll
                 for (int j = 0; j < kPanel; j++)
-                    if (j != t && j != t + 1) {
-                        pa[j] = fma(-fa, ppv[j], pa[j]);
-                        pb[j] = fma(-fb, ppv[j], pb[j]);
-                    }
+                    if (j != t && j != t + 1) pa[j] = fma(-fa, ppv[j], pa[j]);
                 pa[t] = -fa;
-                pb[t] = -fb;
-                if (pa_is_p) {                        // the pivot row: its own entries over the pivot
+                if (is_p) {                           // the pivot row: its own entries over the pivot
 #pragma unroll
                     for (int j = 0; j < kPanel; j++) pa[j] = j == t ? inv : ppv[j] * inv;
-                }
-                if (pb_is_p) {
-#pragma unroll
-                    for (int j = 0; j < kPanel; j++) pb[j] = j == t ? inv : ppv[j] * inv;
                 }
             }
             if (bad && tid == 0) s_bad = 1;
 #pragma unroll
-            for (int t = 0; t < kPanel; t++) {
-                As[r0 * kLdA + k0 + t] = pa[t];
-                As[r1 * kLdA + k0 + t] = pb[t];
-            }
+            for (int t = 0; t < kPanel; t++) As[r0 * kLdA + k0 + t] = pa[t];
 #pragma unroll
-            for (int t = 0; t < kPanel; t += 2) {
+            for (int t = 0; t < kPanel; t += 2)
                 *reinterpret_cast<double2*>(&Xb[r0 * kLdX + t]) = make_double2(pa[t], pa[t + 1]);
-                *reinterpret_cast<double2*>(&Xb[r1 * kLdX + t]) = make_double2(pb[t], pb[t + 1]);
-            }
         } else if (b == 0) {
             // parameter-only work of the E-step constants, off the elimination's path
-            for (int e = tid - 64; e < m * NP; e += kInvThreads - 64) {
+            for (int e = tid - 128; e < m * NP; e += kInvThreads - 128) {
                 const int j = e / NP, i = e - j * NP;
                 float cl = 0.f;
                 if (i < n) {
@@ -240,8 +217,9 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
                 }
                 sb_cl2[e] = cl;
             }
-            if (tid >= 64 && tid < 64 + kInvN) cs[tid - 64] = tid - 64 < n ? c[(size_t)h * n + tid - 64] : 0.0;
-            if (tid == 64 + kInvN) s_lgm = log(gm[h]);
+            const int q = tid - 128;
+            if (q < kInvN) cs[q] = q < n ? c[(size_t)h * n + q] : 0.0;
+            if (q == kInvN) s_lgm = log(gm[h]);
         } else if (b >= 1 && (b == npan || warp >= 4)) {
             // the previous panel's block sweep on the columns outside it and
             // outside this panel (which got it already), in column strips of 8
