@@ -147,7 +147,7 @@ struct TcCohortItem {
 struct MStepBuffers {
     double *A, *Anew, *c, *alpha, *mu, *beta, *rho, *gm, *W, *ldet, *ltc64;
     double *partial, *raw, *stats, *work, *chunk;
-    double* gj;        // n > 128: M n^2 working matrices + M n pivot logs of the inverse
+    double* gj;        // n > 128: the inverse's swept panels (in M n^2 doubles) + M n pivot logs
     int64_t* bflag;          // M: Newton-condition violations found so far (zero between M-steps)
     int* use_newton;         // M: 1 Newton step, 0 natural gradient, -1 frozen model (no update)
     float *Wf, *wcf;

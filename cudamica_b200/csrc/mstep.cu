@@ -7,6 +7,7 @@
 // host SVD for pinv, a synchronous bflag copy, ...).  Here it is six small
 // kernels that stay on the device, so that a whole iteration can be captured
 // in one CUDA graph and no host synchronisation is needed between iterations.
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -17,6 +18,7 @@ using namespace amica;
 
 namespace {
 
+namespace cg = cooperative_groups;
 constexpr int kT = 256;
 
 // ---------------------------------------------------------------------------
@@ -334,104 +336,121 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_derive(
 // k_inverse_big: W_h = A_h^{-1} and log|pivots| for 128 < n <= 256, where the
 // n x n FP64 matrix no longer fits in one SM's shared memory.  The blocked
 // Gauss-Jordan elimination of k_inverse_derive (16-column panels, the same
-// pivot keys with 8 row bits, the block sweep on the FP64 tensor cores with
-// look-ahead) on a row-major working copy in global memory (L2-resident, 512
-// KB at n = 256); one CTA of 512 threads per model.  Warps 0-3 sweep a panel
-// (thread r holds rows r and r + 128, one 128-thread barrier per pivot);
-// warps 4-15 apply the previous panel's block sweep to the other columns,
-// reading and writing their accumulators in global memory.
+// pivot keys with 8 row bits, the block sweep on the FP64 tensor cores) over a
+// cluster of 8 CTAs a model, each holding the whole columns of every eighth
+// panel (up to 32 columns) in shared memory.  A panel's owner sweeps it (8
+// warps, one row a thread) and hands the swept panel to the others through
+// global memory (32 KB, L2-resident; two buffers) and its pivot rows through
+// distributed shared memory; one cluster barrier a panel.  The next panel's
+// owner brings that panel up to date first, then sweeps it while everyone
+// applies the block sweep to the rest.
+// What bounds it is the chain of n dependent pivots and, per panel, the barrier
+// and the trip through L2.  (One CTA a model on a matrix in L2, the block
+// sweeps reading and writing it there, took 700 us at n = 256, M = 4; this takes
+// 175, and the kernels around the E-step 294 us instead of 818.)
 constexpr int kMaxN = 256;
 constexpr int kBigN = kMaxN;
-constexpr size_t kBigSmem = sizeof(double) * 3 * (size_t)kBigN * kLdX;
+constexpr int kBigCtas = 8;                           // a panel each, round robin
+constexpr int kBigCols = kBigN / kBigCtas;            // columns a CTA holds
+constexpr int kLdS = kBigCols + 2;                    // 16-byte rows; 8 lanes reading 8 rows on distinct banks
+constexpr int kLdXc = kBigN + 4;                      // column stride of X: an 8 x 4 fragment on distinct banks
+constexpr size_t kBigSmem = sizeof(double) * ((size_t)kBigN * kLdS + 2 * (size_t)kPanel * kLdXc + (size_t)kBigCols * kLdX);
 
-__device__ __forceinline__ void bar_panel4() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void bar_panel8() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t pivot_key8(double v, bool usable, int r) {
     return usable ? ((((uint32_t)__double2hiint(v)) & 0x7fffff00u) | (uint32_t)(255 - r)) + 256u : 0u;
 }
 
-// the global-memory form of block_sweep_strip: a(i, 8 ct + [0, 8)) for the
-// row tiles rt0 + [0, nrt) of G (row-major, stride n; rows and columns at and
-// beyond n are skipped)
-__device__ __forceinline__ void block_sweep_strip_g(double* __restrict__ G, int n, const double* __restrict__ X,
-                                                    const double* __restrict__ Pt, const int* pinv, int k0,
-                                                    int ct, int rt0, int nrt, int lane) {
+// block_sweep_strip for a CTA's columns: the CTA's columns 8 ct + [0, 8) of rows
+// i0 + [0, 32), X column-major
+__device__ __forceinline__ void block_sweep_tile(double* __restrict__ S, const double* __restrict__ X,
+                                                 const double* __restrict__ Pt, const int* pinv, int k0,
+                                                 int ct, int i0, int lane) {
     const int g = lane >> 2, q = lane & 3;
-    const int j = 8 * ct + 2 * q;
-    const bool ok0 = j < n, ok1 = j + 1 < n;
-    double acc[8][2];
+    double acc[4][2];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        if (u < nrt) {
-            const int i = 8 * (rt0 + u) + g;
-            const bool ok = i < n && !((unsigned)(pinv[i] - k0) < (unsigned)kPanel);
-            acc[u][0] = ok && ok0 ? G[(size_t)i * n + j] : 0.0;
-            acc[u][1] = ok && ok1 ? G[(size_t)i * n + j + 1] : 0.0;
-        }
+    for (int u = 0; u < 4; u++) {
+        const int i = i0 + 8 * u + g;
+        const double2 d = *reinterpret_cast<const double2*>(&S[i * kLdS + 8 * ct + 2 * q]);
+        // a row pivoted in this panel starts from zero
+        const bool piv = (unsigned)(pinv[i] - k0) < (unsigned)kPanel;
+        acc[u][0] = piv ? 0.0 : d.x;
+        acc[u][1] = piv ? 0.0 : d.y;
     }
 #pragma unroll
     for (int s = 0; s < kPanel; s += 4) {
         const double bf = Pt[(8 * ct + g) * kLdX + s + q];
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (u < nrt) dmma884(acc[u][0], acc[u][1], X[(8 * (rt0 + u) + g) * kLdX + s + q], bf);
+        for (int u = 0; u < 4; u++) dmma884(acc[u][0], acc[u][1], X[(s + q) * kLdXc + i0 + 8 * u + g], bf);
     }
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        if (u < nrt) {
-            const int i = 8 * (rt0 + u) + g;
-            if (i < n) {
-                if (ok0) G[(size_t)i * n + j] = acc[u][0];
-                if (ok1) G[(size_t)i * n + j + 1] = acc[u][1];
-            }
-        }
-    }
+    for (int u = 0; u < 4; u++)
+        *reinterpret_cast<double2*>(&S[(i0 + 8 * u + g) * kLdS + 8 * ct + 2 * q]) = make_double2(acc[u][0], acc[u][1]);
 }
 
-__global__ void __launch_bounds__(kInvThreads, 1) k_inverse_big(const double* __restrict__ A,
-                                                               double* __restrict__ work,
-                                                               double* __restrict__ W,
-                                                               double* __restrict__ pivlog, int n,
-                                                               int* err) {
+__global__ void __cluster_dims__(kBigCtas, 1, 1) __launch_bounds__(kInvThreads, 1)
+    k_inverse_big(const double* __restrict__ A, double* work, double* __restrict__ W,
+                  double* __restrict__ pivlog, int n, int* err) {
     extern __shared__ __align__(16) double smem_big[];
-    double* Xs = smem_big;                            // swept panels, two buffers of 256 x kLdX
-    double* Pt = Xs + 2 * kBigN * kLdX;               // Pt[j * kLdX + t] = a(p_t, j) before the panel's update
-    __shared__ __align__(16) double crow_v[2][4][kPanel];
-    __shared__ uint32_t ckey[2][4];
-    __shared__ double cpiv[2][4], cinv[2][4];
-    __shared__ double pivs[kBigN];
+    double* S = smem_big;                             // a(r, column) at S[r * kLdS + local column]
+    double* Xs = S + kBigN * kLdS;                    // swept panels, two buffers: Xs[(b & 1) * 16 * kLdXc + t * kLdXc + r]
+    double* Pt = Xs + 2 * kPanel * kLdXc;             // Pt[local column * kLdX + t] = a(p_t, column) before the panel's update
+    __shared__ __align__(16) double crow_v[2][8][kPanel];
+    __shared__ __align__(16) uint32_t ckey[2][8];
+    __shared__ double cpiv[2][8], cinv[2][8];
+    __shared__ double pivs[kBigCols];
     __shared__ int perm[kBigN], pinv[kBigN];
-    __shared__ int s_bad;
-    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ int s_bad[2];                          // by panel parity: a fast CTA's next panel never hides one
+    cg::cluster_group cluster = cg::this_cluster();
+    const int me = (int)cluster.block_rank(), h = blockIdx.x / kBigCtas;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const double* Ah = A + (size_t)h * n * n;         // column-major a(r, j) = Ah[j n + r]
-    double* G = work + (size_t)h * n * n;             // row-major a(r, j) = G[r n + j]
-    for (int e = tid; e < n * n; e += kInvThreads) {
-        const int j = e / n, r = e - j * n;
-        G[(size_t)r * n + j] = Ah[e];
+    double* Xg = work + (size_t)h * 2 * kPanel * kBigN;   // two buffers, column-major
+    // the global column of local column jl: panel me + 8 (jl / 16)
+    auto column = [&](int jl) { return kPanel * (me + kBigCtas * (jl >> 4)) + (jl & (kPanel - 1)); };
+    for (int e = tid; e < kBigCols * kBigN; e += kInvThreads) {
+        const int r = e & (kBigN - 1), jl = e / kBigN, j = column(jl);
+        S[r * kLdS + jl] = r < n && j < n ? Ah[(size_t)j * n + r] : 0.0;
     }
     if (tid < kBigN) pinv[tid] = 0x7fffffff;
-    if (tid == 0) s_bad = 0;
-    const int r0 = tid, r1 = tid + 128;               // panel threads (tid < 128)
-    bool us0 = r0 < n, us1 = r1 < n;
-    const int npan = (n + kPanel - 1) / kPanel, ncs = (n + 7) / 8;
-    __syncthreads();
-    for (int b = 0; b <= npan; b++) {
-        const int k0 = kPanel * b;
-        if (b < npan && warp < 4) {
-            double* Xb = Xs + (b & 1) * kBigN * kLdX;
-            double pa[kPanel], pb[kPanel];
+    if (tid < 2) s_bad[tid] = 0;
+    const int npan = (n + kPanel - 1) / kPanel, nrg = (n + 31) / 32;
+    // the block sweep of panel `b` on the CTA's columns outside panel slot `skip`
+    auto sweep_rest = [&](int b, int skip, int w0, int nw) {
+        const double* Xb = Xs + (b & 1) * kPanel * kLdXc;
+        for (int e = warp - w0; e < 4 * nrg; e += nw) {
+            const int ct = e & 3;
+            if ((ct >> 1) != skip) block_sweep_tile(S, Xb, Pt, pinv, kPanel * b, ct, 32 * (e >> 2), lane);
+        }
+    };
+    cluster.sync();                                   // every CTA runs before the first remote store
+    bool bad = false;
+    for (int b = 0; b < npan; b++) {
+        const int k0 = kPanel * b, slot = b / kBigCtas;
+        const bool mine = b % kBigCtas == me;
+        double* Xb = Xs + (b & 1) * kPanel * kLdXc;
+        double* Xgb = Xg + (b & 1) * kPanel * kBigN;
+        if (!mine) {
+            // the previous panel's owner leaves that panel as it is
+            if (b > 0) sweep_rest(b - 1, (b - 1) % kBigCtas == me ? (b - 1) / kBigCtas : -1, 0, kInvThreads / 32);
+        } else if (warp >= 8) {
+            if (b > 0) sweep_rest(b - 1, slot, 8, 8);   // this panel got it already
+        } else {
+            const int r0 = tid;                       // the thread's row, and whether no panel has pivoted it
+            bool us0 = r0 < n && pinv[r0] == 0x7fffffff;
+            double pa[kPanel];
 #pragma unroll
-            for (int t = 0; t < kPanel; t++) {
-                const bool cok = k0 + t < n;
-                pa[t] = cok && r0 < n ? G[(size_t)r0 * n + k0 + t] : 0.0;
-                pb[t] = cok && r1 < n ? G[(size_t)r1 * n + k0 + t] : 0.0;
+            for (int t = 0; t < kPanel; t += 2) {
+                const double2 d = *reinterpret_cast<const double2*>(&S[r0 * kLdS + kPanel * slot + t]);
+                pa[t] = d.x;
+                pa[t + 1] = d.y;
             }
-            bool bad = false;
-            uint32_t ka = pivot_key8(pa[0], us0, r0), kb = pivot_key8(pb[0], us1, r1);
-            uint32_t key = max(ka, kb);
-            double v = kb > ka ? pb[0] : pa[0];
+            uint32_t key = pivot_key8(pa[0], us0, r0);
+            double v = pa[0];
             double rv = 1.0 / v;
             uint32_t wkey = __reduce_max_sync(0xffffffffu, key);
+            bool fail = false;
 #pragma unroll
             for (int t = 0; t < kPanel; t++) {
                 if (k0 + t >= n) break;               // uniform
@@ -439,45 +458,34 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_big(const double* __
                 if (wkey == 0u) {
                     if (lane == 0) ckey[buf][warp] = 0u;
                 } else if (key == wkey) {             // one thread: the key names its row
-                    const bool second = kb == key;
 #pragma unroll
                     for (int j = 0; j < kPanel; j += 2)
-                        *reinterpret_cast<double2*>(&crow_v[buf][warp][j]) =
-                            second ? make_double2(pb[j], pb[j + 1]) : make_double2(pa[j], pa[j + 1]);
+                        *reinterpret_cast<double2*>(&crow_v[buf][warp][j]) = make_double2(pa[j], pa[j + 1]);
                     ckey[buf][warp] = key;
                     cpiv[buf][warp] = v;
                     cinv[buf][warp] = rv;
                 }
-                bar_panel4();
-                const int tn = t + 1 < kPanel ? t + 1 : t;
-                uint32_t best = ckey[buf][0];
-                int wb = 0;
-                double piv = cpiv[buf][0], inv = cinv[buf][0], pn = crow_v[buf][0][tn];
-#pragma unroll
-                for (int qq = 1; qq < 4; qq++) {
-                    const uint32_t kq = ckey[buf][qq];
-                    const double pq = cpiv[buf][qq], iq = cinv[buf][qq], nq = crow_v[buf][qq][tn];
-                    if (kq > best) { best = kq; wb = qq; piv = pq; inv = iq; pn = nq; }
-                }
-                if (best == 0u || piv == 0.0) { bad = true; break; }   // same in every panel thread
-                const int p = 255 - (int)((best - 256u) & 255u);
+                bar_panel8();
+                const uint4 ka = *reinterpret_cast<const uint4*>(&ckey[buf][0]);
+                const uint4 kb = *reinterpret_cast<const uint4*>(&ckey[buf][4]);
+                const uint32_t best = max(max(max(ka.x, ka.y), max(ka.z, ka.w)), max(max(kb.x, kb.y), max(kb.z, kb.w)));
+                const int p = 255 - (int)((best - 256u) & 255u), wb = p >> 5;
+                const double piv = cpiv[buf][wb], inv = cinv[buf][wb];
                 const double* pp = crow_v[buf][wb];
-                if (tid == 0) { perm[k0 + t] = p; pinv[p] = k0 + t; pivs[k0 + t] = piv; }
-                const bool pa_is_p = r0 == p, pb_is_p = r1 == p;
-                us0 = us0 && !pa_is_p;
-                us1 = us1 && !pb_is_p;
-                const double fa = pa[t] * inv, fb = pb[t] * inv;
+                const double pn = pp[t + 1 < kPanel ? t + 1 : t];
+                if (best == 0u || piv == 0.0) { fail = true; break; }   // same in every panel thread
+                if (tid == 0) { perm[k0 + t] = p; pivs[kPanel * slot + t] = piv; }
+                const bool is_p = r0 == p;
+                us0 = us0 && !is_p;
+                const double fa = pa[t] * inv;
                 if (t + 1 < kPanel) {                 // the next column first, and the next search
                     pa[t + 1] = fma(-fa, pn, pa[t + 1]);
-                    pb[t + 1] = fma(-fb, pn, pb[t + 1]);
-                    ka = pivot_key8(pa[t + 1], us0, r0);
-                    kb = pivot_key8(pb[t + 1], us1, r1);
-                    key = max(ka, kb);
-                    v = kb > ka ? pb[t + 1] : pa[t + 1];
+                    key = pivot_key8(pa[t + 1], us0, r0);
+                    v = pa[t + 1];
                     rv = 1.0 / v;
                     wkey = __reduce_max_sync(0xffffffffu, key);
                 }
-                double ppv[kPanel];                   // the pivot row, read once for both rows
+                double ppv[kPanel];                   // the pivot row
 #pragma unroll
                 for (int j = 0; j < kPanel; j += 2) {
                     const double2 d = *reinterpret_cast<const double2*>(pp + j);
@@ -486,77 +494,71 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_inverse_big(const double* __
                 }
 #pragma unroll
                 for (int j = 0; j < kPanel; j++)
-                    if (j != t && j != t + 1) {
-                        pa[j] = fma(-fa, ppv[j], pa[j]);
-                        pb[j] = fma(-fb, ppv[j], pb[j]);
-                    }
+                    if (j != t && j != t + 1) pa[j] = fma(-fa, ppv[j], pa[j]);
                 pa[t] = -fa;
-                pb[t] = -fb;
-                if (pa_is_p) {                        // the pivot row: its own entries over the pivot
+                if (is_p) {                           // the pivot row: its own entries over the pivot
 #pragma unroll
                     for (int j = 0; j < kPanel; j++) pa[j] = j == t ? inv : ppv[j] * inv;
                 }
-                if (pb_is_p) {
-#pragma unroll
-                    for (int j = 0; j < kPanel; j++) pb[j] = j == t ? inv : ppv[j] * inv;
-                }
             }
-            if (bad && tid == 0) s_bad = 1;
 #pragma unroll
             for (int t = 0; t < kPanel; t++) {
-                if (k0 + t < n) {
-                    if (r0 < n) G[(size_t)r0 * n + k0 + t] = pa[t];
-                    if (r1 < n) G[(size_t)r1 * n + k0 + t] = pb[t];
-                }
+                Xgb[t * kBigN + r0] = pa[t];
+                Xb[t * kLdXc + r0] = pa[t];
             }
 #pragma unroll
-            for (int t = 0; t < kPanel; t += 2) {
-                *reinterpret_cast<double2*>(&Xb[r0 * kLdX + t]) = make_double2(pa[t], pa[t + 1]);
-                *reinterpret_cast<double2*>(&Xb[r1 * kLdX + t]) = make_double2(pb[t], pb[t + 1]);
-            }
-        } else if (b >= 1 && (b == npan || warp >= 4)) {
-            // the previous panel's block sweep outside it and outside this panel
-            const int kp = k0 - kPanel;
-            const double* Xp = Xs + ((b - 1) & 1) * kBigN * kLdX;
-            const int w0 = b == npan ? 0 : 4, nw = b == npan ? 16 : 12;
-            for (int ct = warp - w0; ct < ncs; ct += nw) {
-                const int j0 = 8 * ct;
-                if ((unsigned)(j0 - kp) < (unsigned)kPanel || (unsigned)(j0 - k0) < (unsigned)kPanel) continue;
-                for (int rt0 = 0; 8 * rt0 < n; rt0 += 8) block_sweep_strip_g(G, n, Xp, Pt, pinv, kp, ct, rt0, 8, lane);
+            for (int t = 0; t < kPanel; t += 2)
+                *reinterpret_cast<double2*>(&S[r0 * kLdS + kPanel * slot + t]) = make_double2(pa[t], pa[t + 1]);
+            bar_panel8();                             // perm is written
+            const int q = tid / kPanel, t = tid % kPanel;   // to CTA q: pivot row t
+            if (q < kBigCtas) {
+                if (fail && t == 0) cluster.map_shared_rank(s_bad, q)[b & 1] = 1;
+                if (!fail && q != me && k0 + t < n) cluster.map_shared_rank(perm, q)[k0 + t] = perm[k0 + t];
             }
         }
-        __syncthreads();
-        if (s_bad || b == npan) break;
-        // Pt for this panel: its pivot rows' entries outside it, now final up to it
-        const int w = min(kPanel, n - k0);
-        for (int e = tid; e < kPanel * kBigN; e += kInvThreads) {
-            const int j = e >> 4, t = e & (kPanel - 1);
-            if ((unsigned)(j - k0) < (unsigned)kPanel) continue;
-            Pt[j * kLdX + t] = t < w && j < n ? G[(size_t)perm[k0 + t] * n + j] : 0.0;
+        cluster.sync();
+        if (s_bad[b & 1]) { bad = true; break; }      // the same in every CTA
+        if (!mine) {
+            for (int e = tid; e < kPanel * kBigN / 2; e += kInvThreads) {
+                double2 d;                            // from L2, and not before the barrier
+                asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];"
+                             : "=d"(d.x), "=d"(d.y) : "l"(Xgb + 2 * e) : "memory");
+                const int t = e / (kBigN / 2), r = 2 * (e % (kBigN / 2));
+                *reinterpret_cast<double2*>(&Xb[t * kLdXc + r]) = d;
+            }
         }
-        __syncthreads();
-        if (b + 1 < npan) {
-            // the next panel's columns: 2 strips x 32 row tiles, 4 tiles per warp
-            const double* Xb = Xs + (b & 1) * kBigN * kLdX;
-            const int rt0 = 4 * (warp >> 1);
-            if (8 * rt0 < n) block_sweep_strip_g(G, n, Xb, Pt, pinv, k0, 2 * (b + 1) + (warp & 1), rt0, 4, lane);
+        // Pt for this panel: its pivot rows' entries in this CTA, final up to it
+        static_assert(kPanel * kBigCols == kInvThreads, "one entry of Pt a thread");
+        {
+            const int jl = tid / kPanel, t = tid % kPanel;
+            Pt[jl * kLdX + t] = k0 + t < n ? S[perm[k0 + t] * kLdS + jl] : 0.0;
         }
+        if (tid < kPanel && k0 + tid < n) pinv[perm[k0 + tid]] = k0 + tid;
         __syncthreads();
+        if (b + 1 < npan && (b + 1) % kBigCtas == me) {
+            // the next panel's columns first
+            const int s1 = (b + 1) / kBigCtas;
+            if ((warp >> 1) < nrg) block_sweep_tile(S, Xb, Pt, pinv, k0, 2 * s1 + (warp & 1), 32 * (warp >> 1), lane);
+            __syncthreads();
+        }
     }
-    if (s_bad) {
-        if (tid == 0) atomicOr(err, kErrSingular);
+    if (bad) {
+        if (me == 0 && tid == 0) atomicOr(err, kErrSingular);
         return;
     }
-    // W(j, q) = a(perm[j], pinv[q]), column-major W_h
+    sweep_rest(npan - 1, (npan - 1) % kBigCtas == me ? (npan - 1) / kBigCtas : -1, 0, kInvThreads / 32);
+    __syncthreads();
+    // W(j, q) = a(perm[j], pinv[q]), column-major W_h: column perm[k] from column k
     double* Wh = W + (size_t)h * n * n;
-    {
-        const int j = tid & (kBigN - 1);
-        if (j < n) {
-            const double* Gr = G + (size_t)perm[j] * n;
-            for (int q = tid >> 8; q < n; q += kInvThreads / kBigN) Wh[(size_t)q * n + j] = Gr[pinv[q]];
+    const int j = tid & (kBigN - 1);
+    if (j < n) {
+        const double* Sr = S + perm[j] * kLdS;
+        for (int jl = tid / kBigN; jl < kBigCols; jl += kInvThreads / kBigN) {
+            const int k = column(jl);
+            if (k < n) Wh[(size_t)perm[k] * n + j] = Sr[jl];
         }
     }
-    for (int k = tid; k < n; k += kInvThreads) pivlog[(size_t)h * n + k] = log(fabs(pivs[k]));
+    if (tid < kBigCols && column(tid) < n) pivlog[(size_t)h * n + column(tid)] = log(fabs(pivs[tid]));
 }
 
 // k_derive: log|det W_h|, the Lt constant and the FP32 E-step constants from a
@@ -1321,7 +1323,7 @@ cudaError_t launch_prep(const MStepBuffers& b, const MStepCfgHost& h, cudaStream
         cudaError_t e = cudaFuncSetAttribute(k_inverse_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)kBigSmem);
         if (e != cudaSuccess) return e;
-        k_inverse_big<<<h.M, kInvThreads, kBigSmem, st>>>(b.A, b.gj, b.W, pivlog, h.n, b.err);
+        k_inverse_big<<<kBigCtas * h.M, kInvThreads, kBigSmem, st>>>(b.A, b.gj, b.W, pivlog, h.n, b.err);
         k_derive<<<dim3(h.NP / 32, h.M), 256, 0, st>>>(b.W, pivlog, b.c, b.alpha, b.mu, b.beta, b.rho, b.gm, h.ldetS,
                                       b.ldet, b.ltc64, b.Wf, b.wcf, b.mp, h.n, h.m, h.NP);
         return cudaGetLastError();
