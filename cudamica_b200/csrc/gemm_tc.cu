@@ -1,6 +1,6 @@
 // The two contractions of the split mixed form (128 < n <= 256 channels) on the
 // 5th-generation tensor cores (tcgen05, kind::tf32, FP32 accumulation in tensor
-// memory), around the density-only E-step kernel (estep_plain.cu, EXT form):
+// memory), around the density-only E-step kernel (estep_dens.cu):
 //
 //   k_wx_tc  b_h(t) = W_hi,h x(t) + W_lo,h x(t) for every model h and sample t
 //            (src/amica.cu:1054-1069, the Dgemm of b = W x).  CTA = (model h,
@@ -45,7 +45,7 @@ constexpr int kWxN = 64;                 // samples per tile (MMA N)
 constexpr int kWxKC = 64;                // K columns per x stage (two 128-byte column blocks)
 constexpr int kWxChunks = kNP / kWxKC;   // stages per tile
 constexpr int kWxStages = 6;             // x stages
-constexpr int kWxThreads = 5 * 32;       // 4 epilogue warps + the control warp
+constexpr int kWxThreads = 6 * 32;       // 4 epilogue warps, the MMA warp, the load warp
 // tensor memory: W_lo [0, 256); D_hi buffers [256, 320) [320, 384); D_lo [384, 448) [448, 512)
 constexpr uint32_t kWxDhi = 256, kWxDlo = 384;
 struct WxShape {
@@ -78,6 +78,14 @@ struct WxArgs {
     int* err;
 };
 
+// What bounds it: the single thread that issues the MMAs (64 of 128 x 64 x 8 a
+// tile, each 32 to 48 cycles on the tensor pipe).  When one lane also waited for,
+// refilled and indexed the x stages, under a divergent branch, an MMA cost it 51
+// cycles and a chunk 475 more; now the loads have a warp of their own and the MMA
+// warp stays converged, with one elected lane issuing from uniform registers.
+// The prologue's loads of W are unrolled (42 us of the old kernel).  n = 256, M = 4,
+// T = 100k: 339 -> 190 us; the E-step at T = 400k, m = 5: 4.79 -> 4.24 ms.
+//
 // b = W_hi x + W_lo x with the two halves in separate accumulators, added in
 // FP32 by the epilogue: the W_lo products (2^-11 of the W_hi ones) are summed
 // among themselves and not into the large W_hi sum MMA by MMA.
@@ -88,7 +96,8 @@ __global__ void __launch_bounds__(kWxThreads, 1)
     uint64_t* bar = (uint64_t*)(sm + WxShape::OFF_BAR);
     uint32_t* tmem_holder = (uint32_t*)(sm + WxShape::OFF_MISC);
     volatile int* abort_flag = (volatile int*)(sm + WxShape::OFF_MISC + 8);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform to the compiler too
     const int slices = 2 * a.M;
     const int slice = blockIdx.x % slices, chunk = blockIdx.x / slices;
     const int h = slice >> 1, half = slice & 1;
@@ -111,6 +120,7 @@ __global__ void __launch_bounds__(kWxThreads, 1)
     // W_hi rows [128 half, 128 half + 128) of model h: the K-major A tile
     {
         const float* Wh = a.Whi + ((size_t)h * kNP + half * 128) * kNP;
+#pragma unroll 8
         for (int e4 = tid; e4 < 128 * (kNP / 4); e4 += kWxThreads) {
             const int i = e4 / (kNP / 4), k = (e4 % (kNP / 4)) * 4;
             const float4 v = *reinterpret_cast<const float4*>(Wh + (size_t)i * kNP + k);
@@ -126,16 +136,22 @@ __global__ void __launch_bounds__(kWxThreads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_holder;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_holder, 0);
     // W_lo of the same rows into tensor memory (row -> lane), RNA-rounded to TF32
     if (warp < 4) {
         const int r = warp * 32 + lane;
         const float* wl = a.Wlo + ((size_t)h * kNP + half * 128 + r) * kNP;
-#pragma unroll 1
+#pragma unroll 4
         for (int k0 = 0; k0 < kNP; k0 += 16) {
             float lo[16];
 #pragma unroll
-            for (int q = 0; q < 16; q++) lo[q] = tf32_rna(wl[k0 + q]);
+            for (int q = 0; q < 16; q += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(wl + k0 + q);
+                lo[q] = tf32_rna(v.x);
+                lo[q + 1] = tf32_rna(v.y);
+                lo[q + 2] = tf32_rna(v.z);
+                lo[q + 3] = tf32_rna(v.w);
+            }
             tmem_st16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)k0, lo);
         }
     }
@@ -143,69 +159,77 @@ __global__ void __launch_bounds__(kWxThreads, 1)
     __syncthreads();
     tc_fence_after();
 
-    if (warp == 4) {
-        // ---- control: TMA loads of x chunks (tile kt, K columns [64 kc, 64 kc + 64)
-        // = chunk u = 4 kt + kc), MMA issue from one thread
-        if (lane == 0 && ntl > 0) {
+    const int nu = ntl * kWxChunks;                   // chunk u: tile u / 4, K columns [64 (u % 4), ...)
+    if (warp == 5) {
+        // ---- TMA loads of x chunks
+        if (lane == 0) {
             const uint32_t sbase = smem_u32(sm);
-            const int nu = ntl * kWxChunks;
-            auto issue = [&](int u) {
+            int u = 0;
+            for (; u < nu; u++) {
                 const int s = u % kWxStages, kt = u / kWxChunks, kc = u % kWxChunks;
+                if (u >= kWxStages &&
+                    !mbar_wait(&bar[WX_EMPTY0 + s], (uint32_t)((u / kWxStages - 1) & 1), abort_flag, a.err))
+                    break;
                 const uint32_t xo = sbase + WxShape::OFF_X + (uint32_t)s * WxShape::X_BYTES;
                 mbar_expect_tx(&bar[WX_FULL0 + s], WxShape::X_BYTES);
 #pragma unroll
                 for (int cb = 0; cb < kWxKC / 32; cb++)
                     tma_load_2d(xo + (uint32_t)(cb * kWxN * 128), &xmap, (kc * (kWxKC / 32) + cb) * 32,
                                 (int)((kt0 + kt) * kWxN), &bar[WX_FULL0 + s]);
-            };
-            constexpr uint32_t ID = idesc_tf32(128, kWxN, 0, 0);
-            int issued = 0, consumed = 0;
-            while (issued < kWxStages && issued < nu) issue(issued++);
-            bool ok = true;
-            for (int u = 0; u < nu && ok; u++) {
-                const int s = u % kWxStages, kt = u / kWxChunks, kc = u % kWxChunks, d = kt & 1;
-                ok = mbar_wait(&bar[WX_FULL0 + s], (uint32_t)((u / kWxStages) & 1), abort_flag, a.err);
-                if (ok) consumed = u + 1;
-                if (ok && kc == 0 && kt >= 2)
-                    ok = mbar_wait(&bar[WX_DEMPTY0 + d], (uint32_t)(((kt >> 1) - 1) & 1), abort_flag, a.err);
+            }
+            // every load issued has landed before the CTA ends (bounded)
+            for (int t = u > kWxStages ? u - kWxStages : 0; t < u; t++)
+                mbar_wait(&bar[WX_FULL0 + (t % kWxStages)], (uint32_t)((t / kWxStages) & 1), abort_flag, a.err,
+                          false, false);
+        }
+        __syncwarp();
+    } else if (warp == 4) {
+        // ---- MMA issue.  The whole warp walks the chunks and one elected lane
+        // issues, so that descriptors are computed in uniform registers
+        const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(sm), 0);
+        constexpr uint32_t ID = idesc_tf32(128, kWxN, 0, 0);
+        bool ok = true;
+        int s = 0;
+        uint32_t ph = 0;
+        for (int kt = 0; kt < ntl && ok; kt++) {
+            const int d = kt & 1;
+            const uint32_t dhi = tmem + kWxDhi + (uint32_t)(d * kWxN);
+            const uint32_t dlo = tmem + kWxDlo + (uint32_t)(d * kWxN);
+            if (kt >= 2) ok = mbar_wait(&bar[WX_DEMPTY0 + d], (uint32_t)(((kt >> 1) - 1) & 1), abort_flag, a.err);
+#pragma unroll
+            for (int kc = 0; kc < kWxChunks; kc++) {
+                ok = ok && mbar_wait(&bar[WX_FULL0 + s], ph, abort_flag, a.err);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t xb = sbase + WxShape::OFF_X + (uint32_t)s * WxShape::X_BYTES;
-                const uint32_t dhi = tmem + kWxDhi + (uint32_t)(d * kWxN);
-                const uint32_t dlo = tmem + kWxDlo + (uint32_t)(d * kWxN);
                 // descriptors of this chunk's first K step; the others differ by
                 // constant address offsets (the address field is addr >> 4)
                 const uint64_t ad0 =
                     sdesc(sbase + WxShape::OFF_W + (uint32_t)(kc * (kWxKC / 32) * 128 * 128), 16, 1024);
                 const uint64_t bd0 = sdesc(xb, 16, 1024);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < kWxKC / 8; kk++) {
-                    const uint32_t koff = (uint32_t)((kk & 3) * 32);
-                    const uint64_t ad = ad0 + (((uint32_t)((kk >> 2) * 128 * 128) + koff) >> 4);
-                    const uint64_t bd = bd0 + (((uint32_t)((kk >> 2) * kWxN * 128) + koff) >> 4);
-                    const uint32_t acc = (kc > 0 || kk > 0) ? 1u : 0u;
-                    tc_mma_tf32(dhi, ad, bd, ID, acc);
-                    tc_mma_tf32_ta(dlo, tmem + (uint32_t)(kc * kWxKC + kk * 8), bd, ID, acc);
+                    for (int kk = 0; kk < kWxKC / 8; kk++) {
+                        const uint32_t koff = (uint32_t)((kk & 3) * 32);
+                        const uint64_t ad = ad0 + (((uint32_t)((kk >> 2) * 128 * 128) + koff) >> 4);
+                        const uint64_t bd = bd0 + (((uint32_t)((kk >> 2) * kWxN * 128) + koff) >> 4);
+                        const uint32_t acc = (kc > 0 || kk > 0) ? 1u : 0u;
+                        tc_mma_tf32(dhi, ad, bd, ID, acc);
+                        tc_mma_tf32_ta(dlo, tmem + (uint32_t)(kc * kWxKC + kk * 8), bd, ID, acc);
+                    }
+                    tc_commit(&bar[WX_EMPTY0 + s]);
+                    if (kc == kWxChunks - 1) tc_commit(&bar[WX_DFULL0 + d]);
                 }
-                tc_commit(&bar[WX_EMPTY0 + s]);
-                if (kc == kWxChunks - 1) tc_commit(&bar[WX_DFULL0 + d]);
-                // the stage of the chunk before the previous one is refilled: its
-                // MMAs have finished by now, so issuing does not wait on the
-                // tensor pipe while it still has this chunk's work queued
-                if (u >= 2 && u - 2 + kWxStages < nu) {
-                    const int sp = (u - 2) % kWxStages;
-                    ok = mbar_wait(&bar[WX_EMPTY0 + sp], (uint32_t)(((u - 2) / kWxStages) & 1), abort_flag,
-                                   a.err);
-                    if (!ok) break;
-                    issue(u - 2 + kWxStages);
-                    issued = u - 1 + kWxStages;
+                __syncwarp();
+                if (++s == kWxStages) {
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
-            // drain: every load issued has landed and every MMA has completed
-            // before the CTA frees its tensor memory (bounded)
-            for (int t = consumed; t < issued; t++)
-                mbar_wait(&bar[WX_FULL0 + (t % kWxStages)], (uint32_t)((t / kWxStages) & 1), abort_flag, a.err,
-                          false, false);
+        }
+        // every MMA has completed before the CTA frees its tensor memory (bounded)
+        if (ntl > 0 && elect_one()) {
             tc_commit(&bar[WX_DRAIN]);
             mbar_wait(&bar[WX_DRAIN], 0u, abort_flag, a.err, false, false);
         }
@@ -223,10 +247,9 @@ __global__ void __launch_bounds__(kWxThreads, 1)
             if (!ok) break;
             tc_fence_after();
             const int64_t t0 = (kt0 + kt) * kWxN;
-            // the pointer walks the rows, and only the last tile checks for the end:
-            // with a multiplication and a comparison per store this loop took 24
-            // instructions a sample instead of 10, and the kernel 339 us instead of
-            // 324 at n = 256, T = 100k, M = 4
+            // the pointer walks the rows, and only the last tile checks for the end
+            // (a multiplication and a comparison per store were 24 instructions a
+            // sample instead of 10)
             float* bp = Bout + (size_t)t0 * ldb;
             const int left = a.T - t0 < kWxN ? (int)(a.T - t0) : kWxN;
 #pragma unroll 1
