@@ -2,13 +2,14 @@
 // pipeline and the C ABI declared in include/amica_b200.h.
 //
 // One iteration is a fixed sequence of kernels on the context's stream:
-//   k_inverse_derive (FP64 inverse, log-det, E-step constants)
+//   k_inverse_derive (FP64 inverse, log-det, E-step constants; above 128
+//      channels k_inverse_big and k_derive)
 //   -> fused E-step (plain FP32 or tcgen05 TF32; above 128 channels the
 //      mixed form is the split one: b = W x as TF32 tensor-core GEMMs, the
 //      density-only E-step, then Psi = sum g x^T as TF32 GEMMs)
 //   -> k_reduce (deterministic FP64 reduction of per-CTA sums)
 //   -> k_mstep (parameters, control block) -> k_gemm64 (A update) -> k_reparm
-//   (-> k_reject on schedule)
+//   (-> the three rejection kernels on schedule)
 // with no host synchronisation, so amica_run() replays one captured CUDA graph
 // per iteration.  This replaces runamica()'s iteration body
 // (src/amica.cu:820-2541), which synchronised with the host ~T/block_size

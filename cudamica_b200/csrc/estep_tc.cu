@@ -136,7 +136,8 @@ int tc_num_shapes() { return 3; }
 // registers a thread, more than 3 density warpgroups leave (136): 2 warpgroups
 // measured 168 us against 280 at n = 64, T = 300k, m = 5.  With several models
 // and five mixtures the log2|y| cache fits beside 2 warpgroups only: 1.48 ms
-// against 1.60 at n = 128, T = 300k, M = 3 (m = 4 the other way: 1.33 against 1.19).
+// against 1.60 at n = 128, T = 300k, M = 3 (m = 4 the other way: 1.33 against
+// 1.19), both taken on tiles of consecutive samples.
 int tc_default_shape(int m, int M) { return m == 5 || (M == 1 && m == 4) ? 1 : 0; }
 static int shape_wg(int shape) { return shape == 0 ? 3 : 2; }
 // Samples per tile: 16 rows per warpgroup, R samples per row.

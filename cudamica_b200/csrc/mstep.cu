@@ -4,7 +4,7 @@
 //
 // The reference runs this part as ~40 small FP64 kernels, cuBLAS/MAGMA calls
 // and host round trips per iteration (src/amica.cu:835-924 and :1981-2512:
-// host SVD for pinv, a synchronous bflag copy, ...).  Here it is six small
+// host SVD for pinv, a synchronous bflag copy, ...).  Here it is a few small
 // kernels that stay on the device, so that a whole iteration can be captured
 // in one CUDA graph and no host synchronisation is needed between iterations.
 #include <cooperative_groups.h>

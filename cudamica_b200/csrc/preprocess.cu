@@ -3,14 +3,14 @@
 // mean, cuBLAS Dsyrk and MAGMA dsyevd / dgesv / dgetrf).
 //
 //   mean      FP64 column sums, per-CTA partials reduced in fixed order
-//   C         X_c^T X_c / T in FP64 (8 x 8 register blocks, one CTA per SM)
-//   S         do_sphere 1: 2 C^{-1/2} from a parallel-ordered cyclic Jacobi
-//             eigendecomposition (one CTA, round-robin disjoint rotations,
-//             matrix and eigenvectors in shared memory);
+//   C         X_c^T X_c / T on the FP64 tensor cores (k_cov_mma)
+//   S         do_sphere 1: 2 C^{-1/2} from the one-sided Jacobi of sphere_eig.cu
+//             or, when C is not numerically positive definite, the two-sided
+//             parallel-ordered Jacobi below;
 //             do_sphere 2: diag(1/std) (std with T-1, src/kernels.cu:148-161);
 //             do_sphere 0: I
 //   ldetS     -log|det S| = -sum log of the eigen-scales
-//   x         S (x - mean) in FP64, rounded once to FP32 into the padded
+//   x         S (x - mean) in FP64 (tensor cores, k_apply_sphere), rounded once to FP32 into the padded
 //             sample-major layout the E-step reads.
 #include <algorithm>
 #include <cmath>

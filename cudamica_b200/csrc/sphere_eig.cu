@@ -1,6 +1,6 @@
 // Eigendecomposition C = V diag(d) V^T of the channel covariance for the
 // sphering (replaces MAGMA's dsyevd in src/preprocess.cu:126-229), n <= 256, on
-// one thread-block cluster of up to 8 CTAs.
+// one thread-block cluster of up to 8 CTAs (16 above 192 channels).
 //
 //   1. C = L L^T, blocked Cholesky.
 //   2. One-sided Jacobi on the columns of L (Hestenes rotations; applied to the
