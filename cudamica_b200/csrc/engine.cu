@@ -140,7 +140,9 @@ struct amica_ctx {
     Status* d_status = nullptr;
     double* d_backup = nullptr;
     size_t backup_len = 0;        // bytes
-    int64_t iter = 0;             // ctrl->iter as of the last call
+    // ctrl->iter once everything queued on the stream has run (a batch of
+    // amica_run_async counts from its launch), and the backup's
+    int64_t iter = 0, backup_iter = 0;
     double* h_stage = nullptr;    // pinned: the block's parameters, and W
     bool stage_busy = false;      // a copy out of h_stage may be in flight
     IterRec* h_recs = nullptr;    // pinned: kPinnedRecs history records, then a single one
@@ -211,6 +213,7 @@ constexpr int64_t kPinnedRecs = 256;
 int snapshot_params(amica_ctx* c, bool restore) {
     if (restore) CK(cudaMemcpyAsync(c->d_block, c->d_backup, c->backup_len, cudaMemcpyDeviceToDevice, c->st));
     else CK(cudaMemcpyAsync(c->d_backup, c->d_block, c->backup_len, cudaMemcpyDeviceToDevice, c->st));
+    (restore ? c->iter : c->backup_iter) = restore ? c->backup_iter : c->iter;
     return AMICA_OK;
 }
 
@@ -333,17 +336,17 @@ int enqueue_recs(amica_ctx* c, int64_t it0, int64_t count) {
         CK(cudaMemcpyAsync(c->h_recs, c->b.hist + it0, sizeof(IterRec) * count, cudaMemcpyDeviceToHost, c->st));
     return AMICA_OK;
 }
-// The record of the single iteration after c->iter, in a slot of its own (a batch of
-// amica_run_async may be outstanding).  Past the end of the device's history it is
-// made from the control block.
+// The record of the last iteration queued (number c->iter, which counts it), in a
+// slot of its own (a batch of amica_run_async may be outstanding).  Past the end of
+// the device's history it is made from the control block.
 int enqueue_last_rec(amica_ctx* c) {
-    if (c->iter < c->b.hist_cap)
-        CK(cudaMemcpyAsync(c->h_recs + kPinnedRecs, c->b.hist + c->iter, sizeof(IterRec), cudaMemcpyDeviceToHost,
+    if (c->iter <= c->b.hist_cap)
+        CK(cudaMemcpyAsync(c->h_recs + kPinnedRecs, c->b.hist + c->iter - 1, sizeof(IterRec), cudaMemcpyDeviceToHost,
                            c->st));
     return AMICA_OK;
 }
 IterRec last_rec(const amica_ctx* c) {
-    if (c->iter < c->b.hist_cap) return c->h_recs[kPinnedRecs];
+    if (c->iter <= c->b.hist_cap) return c->h_recs[kPinnedRecs];
     const Ctrl& t = *c->h_ctrl;
     IterRec r{};
     r.ll = t.ll; r.lrate = t.lrate; r.iter = t.iter; r.newton = t.newton; r.ll_decreased = t.ll_decreased;
@@ -670,6 +673,8 @@ int amica_init(amica_ctx* c, const double* A0, const double* c0) {
     if (!c) return AMICA_ERR_INVALIDPARAM;
     CK(cudaSetDevice(c->dev));
     const int n = c->n, M = c->M, m = c->m;
+    // an outstanding batch writes the pinned control block that is set below
+    if (c->pending >= 0) CK(cudaStreamSynchronize(c->st));
     // built in the staging area, in the block's order
     TRY(stage(c));
     const size_t nnM = (size_t)M * n * n, mnM = (size_t)M * m * n;
@@ -738,6 +743,7 @@ int amica_em_step(amica_ctx* c, amica_iter_out* out) {
     TRY(snapshot_params(c, false));
     CK(cudaEventRecord(c->ev0, c->st));
     TRY(enqueue_iteration(c));
+    c->iter++;
     CK(cudaEventRecord(c->ev1, c->st));
     TRY(enqueue_status(c));
     TRY(enqueue_last_rec(c));
@@ -754,7 +760,6 @@ int amica_em_step(amica_ctx* c, amica_iter_out* out) {
         return e;
     }
     const IterRec r = last_rec(c);
-    c->iter = ctl.iter;
     c->hist.push_back(r);
     print_iter(c, r);
     fill_out(r, ctl, ms, out);
@@ -781,7 +786,10 @@ int amica_run_async(amica_ctx* c, int64_t maxiter) {
     if (it0 + maxiter > c->b.hist_cap) return AMICA_ERR_INVALIDPARAM;
     TRY(snapshot_params(c, false));
     CK(cudaEventRecord(c->ev0, c->st));
-    for (int64_t k = 0; k < maxiter; k++) CK(cudaGraphLaunch(c->graph, c->st));
+    for (int64_t k = 0; k < maxiter; k++) {
+        CK(cudaGraphLaunch(c->graph, c->st));
+        c->iter++;
+    }
     CK(cudaEventRecord(c->ev1, c->st));
     TRY(enqueue_status(c));
     TRY(enqueue_recs(c, it0, maxiter));
@@ -799,7 +807,6 @@ int amica_run_wait(amica_ctx* c, amica_iter_out* hist) {
     CK(cudaStreamSynchronize(c->st));
     c->have_estep = maxiter > 0 || c->have_estep;
     int e = status_error(c);
-    c->iter = c->h_ctrl->iter;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     std::vector<IterRec> recs(maxiter);
@@ -813,7 +820,6 @@ int amica_run_wait(amica_ctx* c, amica_iter_out* hist) {
     if (e == AMICA_ERR_NUMERIC) {
         snapshot_params(c, true);
         cudaStreamSynchronize(c->st);
-        c->iter = it0;
     }
     return e;
 }
@@ -1167,6 +1173,7 @@ int amica_shard_mstep(amica_ctx* c, const double* d_stats, int64_t nkeep_total, 
     // E-step of this shard counts its own again
     k_set_nkeep<<<1, 1, 0, c->st>>>(c->b.ctrl, nkeep_total);
     CK(launch_mstep(c->b, c->hc, false, c->d_P, c->d_keep, c->T, c->st));
+    c->iter++;
     k_set_nkeep<<<1, 1, 0, c->st>>>(c->b.ctrl, c->T);
     CK(cudaEventRecord(c->ev1, c->st));
     TRY(enqueue_status(c));
@@ -1183,7 +1190,6 @@ int amica_shard_mstep(amica_ctx* c, const double* d_stats, int64_t nkeep_total, 
         return e;
     }
     IterRec r = last_rec(c);
-    c->iter = ctl.iter;
     r.nkeep = nkeep_total;
     c->hist.push_back(r);
     print_iter(c, r);
@@ -1444,7 +1450,10 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
         CK(cudaStreamWaitEvent(co->st, co->evs[2 * s], 0));
     }
     CK(cudaEventRecord(co->ev0, co->st));
-    for (int64_t k = 0; k < iters; k++) CK(cudaGraphLaunch(co->graph, co->st));
+    for (int64_t k = 0; k < iters; k++) {
+        CK(cudaGraphLaunch(co->graph, co->st));
+        for (auto* c : co->subs) c->iter++;
+    }
     CK(cudaEventRecord(co->ev1, co->st));
     // each subject's status and records on its own stream, behind the graphs
     for (int s = 0; s < ns; s++) {
@@ -1463,7 +1472,6 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
         c->have_estep = c->have_estep || iters > 0;
         CK(cudaStreamSynchronize(c->st));
         int e = status_error(c);
-        c->iter = c->h_ctrl->iter;
         std::vector<IterRec> recs(iters);
         TRY(fetch_recs(c, it0[s], recs));
         for (int64_t k = 0; k < iters; k++) {
@@ -1475,7 +1483,6 @@ int amica_cohort_run(amica_cohort* co, int64_t iters, amica_iter_out* hist, doub
         if (e == AMICA_ERR_NUMERIC) {
             snapshot_params(c, true);
             cudaStreamSynchronize(c->st);
-            c->iter = it0[s];
         }
         if (first_err == AMICA_OK) first_err = e;
     }
