@@ -108,6 +108,20 @@ constexpr int kWloCol = 256;            // TMEM columns of W_lo, the A operand o
 // per half of each FP32x2 sum); 2.72 ms per E-step at n=128, T=1M, M=3, m=3
 // against 2.77 ms with 8
 constexpr int kFlush = 16;
+// Tiles that phi accumulates in tensor memory before it is added to the FP64 slot:
+// half of the CTA's tiles, between 32 and 128, in whole flush periods.  Every MMA
+// whose products are not all 0 loses about a last place of the running sum, always
+// towards 0, so phi's relative error grows with their number; a tile of kSegRows-row
+// segments has more of them than a run of samples had (a model that owns a third of
+// the blocks is met in 5/9 of the steps instead of 1/3).  Half as many tiles make up
+// for twice as many steps, the most that segments of two can give, and 128 bounds
+// the error of long fits.  Relative error of phi (n = 128, M = 3, m = 3, middle of a fit)
+// at T = 1M: 5.8e-5 in one period, 1.6e-5 now, at 300k: 2.1e-5 -> 1.5e-5; the E-step
+// at T = 1M takes 2.13 ms instead of 2.10 (periods of 64 tiles: 2.12 and 9e-6, of 32: 2.15).
+__host__ __device__ constexpr int phi_period_of(int ntile_local) {
+    const int half = ((ntile_local + 1) / 2 + kFlush - 1) / kFlush * kFlush;
+    return half < 32 ? 32 : half > 128 ? 128 : half;
+}
 // x stages: up to kMaxStages, each with a FULL (TMA landed) and an EMPTY
 // (MMAs done reading it) barrier
 constexpr int kMaxStages = 3;
@@ -196,6 +210,7 @@ __global__ void __launch_bounds__(TcCfg<WG, NST>::kThreads, 1)
     const int cid = blockIdx.x / M;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ntile_local = (a.ntiles > cid) ? (a.ntiles - cid + a.nclusters - 1) / a.nclusters : 0;
+    const int phi_period = phi_period_of(ntile_local);
 
     // ---- setup: barriers, W_h into the swizzled A tile, tensor memory
     if (tid == 0) {
