@@ -255,7 +255,7 @@ EStepArgs estep_args(amica_ctx* c) {
 
 // The split form's E-step: W -> (W_hi, W_lo), b = W_hi x + W_lo x (tensor-core
 // kernel), the density-only kernel, Psi = sum g x^T (tensor-core kernel, FP32
-// accumulation over at most 8192 samples, added into the partial slots in
+// accumulation over at most 4096 samples, added into the partial slots in
 // FP64).  W_hi has no bits below TF32 and x and g are stored rounded to TF32,
 // so only W_lo is rounded by the MMA.
 int enqueue_split_estep(amica_ctx* c, const EStepArgs& a) {

@@ -21,8 +21,8 @@
 //            stage with two plain bulk copies and issues MMA M=128 N=256 K=32
 //            into one of two 256-column tensor-memory accumulators; 4 flush
 //            warps add each accumulator into the chunk's FP64 partial slot
-//            every 256 blocks (8192 samples), so that no FP32 sum covers more
-//            than 8192 samples.  Each FP64 address has one writer and the
+//            every 64 to 128 blocks, so that no FP32 sum covers more than
+//            4096 samples.  Each FP64 address has one writer and the
 //            slots are summed in a fixed order: the result is deterministic.
 //
 // The data x is T + 3 rows of 256 floats (TF32 values); g and the images hold
@@ -287,7 +287,17 @@ __global__ void __launch_bounds__(kWxThreads, 1)
 constexpr int kGxT = 32;                 // samples per block (MMA K)
 constexpr int kGxStages = 4;
 constexpr int kGxThreads = 5 * 32;       // 4 flush warps + the control warp
-constexpr int kGxFlushTiles = 256;       // blocks per FP32 accumulation period
+// Blocks per FP32 accumulation period: half of the CTA's, between 64 and 128.  Each
+// MMA step with a non-zero product rounds the running sum towards 0, and blocks
+// whose samples come from eight segments of the data have more of these than runs
+// of samples had.  Relative error of phi against 64 bits (middle of a fit) with periods
+// of 256 blocks on runs of samples, on segments, and now: n = 256, T = 300k, M = 3 1.33e-5,
+// 1.49e-5, 1.30e-5; n = 200, T = 200k, M = 2 1.22e-5, 1.40e-5, 1.13e-5.  The E-step at n =
+// 256, T = 400k, M = 4, m = 5 takes 4.27 ms instead of 4.26.
+__host__ __device__ constexpr int gx_period_of(int ntl) {
+    const int half = (ntl + 1) / 2;
+    return half < 64 ? 64 : half > 128 ? 128 : half;
+}
 struct GxShape {
     static constexpr uint32_t A_BYTES = 128u * 128u;   // 128 rows x 32 samples
     static constexpr uint32_t B_BYTES = 256u * 128u;   // 256 rows x 32 samples
@@ -330,7 +340,7 @@ __global__ void __launch_bounds__(kGxThreads, 1) k_gx_tc(GxArgs a) {
     const int h = slice >> 1, half = slice & 1;
     const int64_t kt0 = a.nblocks * chunk / a.nchunks, kt1 = a.nblocks * (chunk + 1) / a.nchunks;
     const int ntl = (int)(kt1 - kt0);
-    const int nper = (ntl + kGxFlushTiles - 1) / kGxFlushTiles;
+    const int period = gx_period_of(ntl), nper = (ntl + period - 1) / period;
 
     if (tid == 0) {
         for (int s = 0; s < kGxStages; s++) {
@@ -399,9 +409,10 @@ __global__ void __launch_bounds__(kGxThreads, 1) k_gx_tc(GxArgs a) {
             int issued = 0, consumed = 0;
             while (issued < kGxStages && issued < ntl) issue(issued++);
             bool ok = true;
+            int p = 0, kp = 0;                        // period, and the block's number in it
             for (int kt = 0; kt < ntl && ok; kt++) {
-                const int s = kt % kGxStages, p = kt / kGxFlushTiles, db = p & 1;
-                const bool first = (kt % kGxFlushTiles) == 0;
+                const int s = kt % kGxStages, db = p & 1;
+                const bool first = kp == 0;
                 ok = mbar_wait(&bar[GX_FULL0 + s], (uint32_t)((kt / kGxStages) & 1), abort_flag, a.err);
                 if (ok) consumed = kt + 1;
                 if (ok && first && p >= 2)
@@ -414,7 +425,11 @@ __global__ void __launch_bounds__(kGxThreads, 1) k_gx_tc(GxArgs a) {
                     tc_mma_tf32(tmem + (uint32_t)(db * kNP), sdesc(ab + (uint32_t)(kk * 32), 16, 1024),
                                 sdesc(bb + (uint32_t)(kk * 32), 16, 1024), ID, (first && kk == 0) ? 0u : 1u);
                 tc_commit(&bar[GX_EMPTY0 + s]);
-                if ((kt % kGxFlushTiles) == kGxFlushTiles - 1 || kt == ntl - 1) tc_commit(&bar[GX_DFULL0 + db]);
+                if (++kp == period || kt == ntl - 1) {
+                    tc_commit(&bar[GX_DFULL0 + db]);
+                    kp = 0;
+                    p++;
+                }
                 if (kt >= 1 && kt - 1 + kGxStages < ntl) {
                     const int sp = (kt - 1) % kGxStages;
                     ok = mbar_wait(&bar[GX_EMPTY0 + sp], (uint32_t)(((kt - 1) / kGxStages) & 1), abort_flag,
