@@ -21,7 +21,7 @@
 // K always the padded count and runs of consecutive samples -> now: n = 71, T =
 // 200k, M = 2, m = 3: 1039 -> 668 us; n = 128, T = 300k, M = 3: 2.51 -> 2.36 ms; n =
 // 256, T = 50k, M = 2, m = 5: 1.27 -> 1.22 ms; n = 100, T = 200k, M = 1: 564 -> 534 us;
-// n = 32, T = 300k, M = 1: 199 -> 205 us.
+// n = 32, T = 300k, M = 1: 199 -> 197 us.
 #include <cooperative_groups.h>
 #include <cstdio>
 
@@ -68,8 +68,10 @@ struct PlainShape {
     static constexpr int NTT = THREADS / NTI;
     static constexpr int CT = kS / NTT;
     static_assert(NTI * NTT == THREADS && NTT * CT == kS, "b = W x tiling");
-    // Psi update: each thread RI x RK block, RI in two runs of RI / 2 channels
+    // Psi update: each thread RI x RK block, RI in two runs of RL = RI / 2 channels (one
+    // of two at NPL = 32, an 8-byte load: 205 -> 197 us at n = 32, T = 300k, M = 1, m = 3)
     static constexpr int RI = NPL / 16;
+    static constexpr int RL = RI > 2 ? RI / 2 : RI;
     static constexpr int RK = NK / (THREADS / 16);
     static_assert(RK * (THREADS / 16) == NK && RI % 2 == 0, "Psi tiling");
     static constexpr int LLD = NPL + 8;             // padded row of the lse tile (8 lanes per sample)
@@ -83,10 +85,13 @@ struct PlainShape {
     static constexpr size_t work_floats = tile_floats > fold_floats ? tile_floats : fold_floats;
     static constexpr size_t smem_floats = (size_t)NK * WLD + work_floats + 2 * kS + kS;
     static constexpr int NFOLD = REG64 ? NACC : (NACC * NPL + THREADS - 1) / THREADS;   // FP64 sums per thread
+    // CTAs per SM: one mixture of up to 32 channels fits two into the registers (128 a
+    // thread; 140 and one CTA: 169 us instead of 105 at n = 32, T = 300k, M = 1)
+    static constexpr int CTAS = NPL == 32 && MM == 1 ? 2 : 1;
 };
 
 template <int NP, int NA, int MM>
-__global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, 1) estep_plain_kernel(EStepArgs a) {
+__global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, PlainShape<NP, NA, MM>::CTAS) estep_plain_kernel(EStepArgs a) {
     using Sh = PlainShape<NP, NA, MM>;
     constexpr int NPL = Sh::NPL, Q = Sh::Q, THREADS = Sh::THREADS, NK = Sh::NK, NACC = Sh::NACC;
     extern __shared__ __align__(16) float sm[];
@@ -209,7 +214,7 @@ __global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, 1) estep_plai
         zero_sums();
     };
     double dLL = 0.0, dVs = 0.0;   // per-sample threads (tid < S)
-    constexpr int PRI = Sh::RI, PRK = Sh::RK;
+    constexpr int PRI = Sh::RI, PRL = Sh::RL, PRK = Sh::RK;
     float psi[PRI][PRK];
 #pragma unroll
     for (int r = 0; r < PRI; r++)
@@ -373,17 +378,17 @@ __global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, 1) estep_plai
         }
         if constexpr (Sh::REG64) fold();
         __syncthreads();
-        // ---- Psi_h += g x^T over the tile (thread: RI x RK block, its channels in two
-        // runs NPL / 2 apart, so that a warp's loads of g are free of bank conflicts)
+        // ---- Psi_h += g x^T over the tile (thread: RI x RK block, its channels in runs
+        // NPL / 2 apart, so that a warp's loads of g are free of bank conflicts)
         {
             const int pi = tid % 16, pk = tid / 16;
-            const int i0 = pi * (PRI / 2), k0 = pk * PRK;
+            const int i0 = pi * PRL, k0 = pk * PRK;
             if (k0 < kend) {
 #pragma unroll 4
                 for (int t = 0; t < kS; t++) {
                     float gv[PRI], xv[PRK];
 #pragma unroll
-                    for (int r = 0; r < PRI; r++) gv[r] = gs[t * NPL + (r >= PRI / 2 ? NPL / 2 - PRI / 2 : 0) + i0 + r];
+                    for (int r = 0; r < PRI; r++) gv[r] = gs[t * NPL + (r >= PRL ? NPL / 2 - PRL : 0) + i0 + r];
 #pragma unroll
                     for (int c = 0; c < PRK; c++) xv[c] = xs[t * Sh::XLD + k0 + c];
 #pragma unroll
@@ -465,12 +470,12 @@ __global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, 1) estep_plai
     }
     {
         const int pi = tid % 16, pk = tid / 16;
-        const int i0 = pi * (PRI / 2), k0 = pk * PRK;
+        const int i0 = pi * PRL, k0 = pk * PRK;
 #pragma unroll
         for (int r = 0; r < PRI; r++)
 #pragma unroll
             for (int c = 0; c < PRK; c++) {
-                const int i = i0c + (r >= PRI / 2 ? NPL / 2 - PRI / 2 : 0) + i0 + r, k = k0 + c;
+                const int i = i0c + (r >= PRL ? NPL / 2 - PRL : 0) + i0 + r, k = k0 + c;
                 if (i < n && k < n) out[L.psi() + (size_t)k * n + i] = (double)psi[r][c];
             }
     }
