@@ -63,6 +63,13 @@ struct PlainShape {
     static constexpr int NK = NP <= 128 ? NA : NP;  // columns of W and x held
     static constexpr int WLD = NPL + 4;             // padded row of W^T in smem
     static constexpr int XLD = NK + 4;              // padded row of the x tile
+    // x tile: XROWS samples at a time, XUNROLL of a thread's loads in flight: all, but
+    // with 2 to 4 mixtures at 128 channels, where the registers are short (m = 3: 322 us
+    // against 330 at T = 60k, M = 2; m = 5 388 against 380, m = 1, M = 1 158 against 154).
+    // One address from scratch per load cost 2 to 6% of the E-step.
+    static constexpr int XROWS = THREADS / (NK / 4);
+    static_assert(THREADS % (NK / 4) == 0 && XROWS % 4 == 0 && kS % XROWS == 0, "x tile");
+    static constexpr int XUNROLL = NK == 128 && MM >= 2 && MM <= 4 ? 4 : kS / XROWS;
     // GEMM b = W x: each thread 4 channels x CT samples
     static constexpr int NTI = NPL / 4;
     static constexpr int NTT = THREADS / NTI;
@@ -148,9 +155,10 @@ __global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, PlainShape<NP
         }
     }
     const float wci = a.wc[(size_t)h * NP + gch];
-    // this model's offset of Lt (with Q > 1 the per-sample threads add every model's;
-    // eight more registers for them measured 4% slower at n = 256)
+    // this model's offset of Lt; with Q > 1 the per-sample threads add every model's
     const float ltch = (float)(a.ltc64[h] - a.ltc64[0]);
+    __shared__ float ltcs[kMaxModels];
+    if (Q > 1 && tid < M) ltcs[tid] = (float)(a.ltc64[tid] - a.ltc64[0]);
 
     // FP32 sums of this thread's channel and sample group: A0..A6 of dens_acc per
     // mixture, sum v b, sum v b^2, sum g
@@ -226,13 +234,23 @@ __global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, PlainShape<NP
     for (int tile = cid; tile < a.ntiles; tile += a.nclusters, it++) {
         const int par = it & 1;
         __syncthreads();                              // the last tile's (or fold's) readers are done
-        // ---- stage the x tile (float4, coalesced; samples past T are zero)
-        for (int e = tid; e < kS * (NK / 4); e += THREADS) {
-            const int t = e / (NK / 4), k4 = e % (NK / 4);
-            const int64_t ts = plain_sample(tile, t, a.ntiles);
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (ts < a.T) v = reinterpret_cast<const float4*>(a.x + ts * a.ldx)[k4];
-            *reinterpret_cast<float4*>(xs + t * Sh::XLD + 4 * k4) = v;
+        // ---- stage the x tile (float4, coalesced; samples past T are zero): a thread's
+        // samples are whole segments apart, so its pointer walks
+        {
+            const int tr = tid / (NK / 4), k4 = tid % (NK / 4);
+            int64_t ts = plain_sample(tile, tr, a.ntiles);
+            const int64_t dts = (int64_t)Sh::XROWS * a.ntiles, dxp = dts * a.ldx;
+            const float* xp = a.x + ts * a.ldx + 4 * k4;
+            float* xd = xs + tr * Sh::XLD + 4 * k4;
+#pragma unroll(Sh::XUNROLL)
+            for (int u = 0; u < kS / Sh::XROWS; u++) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (ts < a.T) v = *reinterpret_cast<const float4*>(xp);
+                *reinterpret_cast<float4*>(xd) = v;
+                ts += dts;
+                xp += dxp;
+                xd += Sh::XROWS * Sh::XLD;
+            }
         }
         __syncthreads();
         // ---- b = W_h x  (thread: channels 4*ti..+3, samples tt*CT..+CT-1)
@@ -319,7 +337,7 @@ __global__ void __launch_bounds__(PlainShape<NP, NA, MM>::THREADS, PlainShape<NP
                         float s = 0.f;
 #pragma unroll
                         for (int b = 0; b < Q; b++) s += cluster.map_shared_rank(myslot, q * Q + b)[tid];
-                        L[q] = (float)(a.ltc64[q] - a.ltc64[0]) + kLn2 * s;
+                        L[q] = ltcs[q] + kLn2 * s;
                     }
                     lmax = fmaxf(lmax, L[q]);
                 }
