@@ -641,6 +641,7 @@ int amica_preprocess(amica_ctx* c) {
     CK(cudaSetDevice(c->dev));
     const long long fault = c->fault_wait_cycles;
     c->fault_wait_cycles = 0;                      // the hook arms one launch
+    c->have_x = false;                             // x is the sphering's scratch until it holds the data
     CK(launch_preprocess(c->d_rawx, c->T, c->n, (int)c->cfg.do_sphere, c->d_means, c->d_cov,
                          c->d_sphere, c->d_evwork, c->d_ldetS, c->d_x, c->NP, (c->use_tc || c->use_split) ? 1 : 0,
                          c->b.err, c->st, fault));
@@ -1223,6 +1224,7 @@ int amica_shard_sphere(amica_ctx* c, const double* d_scatter_total, int64_t T_to
     if (!c || !d_scatter_total || T_total < c->T || T_total < 2) return AMICA_ERR_INVALIDPARAM;
     if (!c->have_data || !c->have_shard_mean) return AMICA_ERR_STATE;
     CK(cudaSetDevice(c->dev));
+    c->have_x = false;                             // as in amica_preprocess
     CK(launch_shard_finish(c->d_rawx, c->T, c->n, (int)c->cfg.do_sphere, c->d_means, d_scatter_total, T_total,
                            c->d_cov, c->d_sphere, c->d_evwork, c->d_ldetS, c->d_x, c->NP,
                            (c->use_tc || c->use_split) ? 1 : 0, c->b.err, c->st));

@@ -968,7 +968,9 @@ cudaError_t launch_shard_finish(const float* raw, int64_t T, int n, int do_spher
 cudaError_t launch_convert_sphered(const double* xs, int64_t T, int n, float* x, int ldx, int tf32,
                                    cudaStream_t st) {
     k_convert<<<2048, 256, 0, st>>>(xs, T, n, x, ldx, tf32);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    // a sphering that ended with an error may have left scratch past T
+    return e != cudaSuccess ? e : cudaMemsetAsync(x + (size_t)T * ldx, 0, sizeof(float) * x_tail_len(ldx), st);
 }
 
 }  // namespace amica
