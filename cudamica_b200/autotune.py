@@ -1,10 +1,10 @@
 """Measured choice of the fused E-step's tile shape and launch shape.
 
 The fused mixed-form E-step (up to 128 channels) is compiled in three tile
-shapes (amica_cfg.tc_shape): 0 = the default for the model and mixture counts
-(3 density warpgroups and 48-sample tiles with 2 TMA stages of x; shape 1 with 5
-mixtures, or one model and 4), 1 = 2 warpgroups and 32-sample tiles with 2 stages, 2 = 2
-warpgroups with 3 stages.  The shape sets the samples per tile (MMA1 N, MMA2
+shapes (amica_set_tile_shape): 0 = 3 density warpgroups and 48-sample tiles with
+2 TMA stages of x, 1 = 2 warpgroups and 32-sample tiles with 2 stages, 2 = 2
+warpgroups with 3 stages.  (A new context starts in shape 0, with 5 mixtures, or
+one model and 4, in shape 1.)  The shape sets the samples per tile (MMA1 N, MMA2
 K), the density warps per SM and the x pipeline depth; the fastest depends on
 n (lane packing), M (cluster size) and m (registers and tensor-memory
 columns for the log2|y| cache), so best_tile_shape times each on the

@@ -853,7 +853,6 @@ int amica_set_tile_shape(amica_ctx* c, int64_t shape) {
     if (!c->use_tc) return AMICA_ERR_UNSUPPORTED;
     if (c->pending >= 0) return AMICA_ERR_STATE;
     CK(cudaSetDevice(c->dev));
-    if (shape == 0) shape = tc_default_shape(c->m, c->M);
     const int S = tc_tile_samples(c->n, (int)shape);
     const int ntiles = (int)((c->T + S - 1) / S);
     const int mc = tc_max_clusters(c->n, c->m, c->M, (int)shape);
@@ -1312,11 +1311,13 @@ int amica_cohort_create(amica_ctx* const* ctxs, int64_t nsub, amica_cohort** out
     *out = nullptr;
     const amica_ctx* c0 = ctxs[0];
     if (!c0) return AMICA_ERR_INVALIDPARAM;
+    const int shape = tc_default_shape(c0->m, 1);
     for (int64_t s = 0; s < nsub; s++) {
         const amica_ctx* c = ctxs[s];
         if (!c || c->dev != c0->dev || c->m != c0->m) return AMICA_ERR_INVALIDPARAM;
-        // the cohort kernel runs the default tile shape
-        if (!c->use_tc || c->M != 1 || c->tc_shape != tc_default_shape(c->m, 1)) return AMICA_ERR_UNSUPPORTED;
+        // the cohort kernel runs the default tile shape, whatever 0 or that shape the
+        // context itself is in
+        if (!c->use_tc || c->M != 1 || (c->tc_shape != 0 && c->tc_shape != shape)) return AMICA_ERR_UNSUPPORTED;
     }
     CK(cudaSetDevice(c0->dev));
     amica_cohort* co = new amica_cohort();
@@ -1326,7 +1327,10 @@ int amica_cohort_create(amica_ctx* const* ctxs, int64_t nsub, amica_cohort** out
     co->nctas = tc_cohort_ctas();
     // deal the concatenated tiles to the CTAs
     std::vector<int64_t> first(nsub + 1, 0);
-    for (int64_t s = 0; s < nsub; s++) first[s + 1] = first[s] + co->subs[s]->ntiles;
+    for (int64_t s = 0; s < nsub; s++) {
+        const int S = tc_tile_samples(co->subs[s]->n, shape);
+        first[s + 1] = first[s] + (co->subs[s]->T + S - 1) / S;
+    }
     const int64_t N = first[nsub];
     std::vector<TcCohortItem> items;
     std::vector<int> off(co->nctas + 1, 0), nitem(nsub, 0);
@@ -1359,7 +1363,7 @@ int amica_cohort_create(amica_ctx* const* ctxs, int64_t nsub, amica_cohort** out
             delete co;
             return AMICA_ERR_CUDA;
         }
-        co->nslots.push_back(nitem[s] * tc_partial_groups(c->n, c->tc_shape));
+        co->nslots.push_back(nitem[s] * tc_partial_groups(c->n, shape));
     }
     co->nitems = (int)items.size();
     int r = AMICA_OK;
@@ -1416,7 +1420,9 @@ static int cohort_capture(amica_cohort* co) {
         for (int s = 0; s < ns; s++) {
             amica_ctx* c = co->subs[s];
             CK(cudaStreamWaitEvent(c->st, co->mid, 0));
-            CK(launch_reduce_finalize(c->b, c->hc, co->nslots[s], false, c->st));
+            MStepCfgHost hc = c->hc;
+            hc.psi_step = tc_psi_step(tc_default_shape(c->m, 1));
+            CK(launch_reduce_finalize(c->b, hc, co->nslots[s], false, c->st));
             CK(launch_mstep(c->b, c->hc, true, c->d_P, c->d_keep, c->T, c->st));
             CK(cudaEventRecord(co->evs[2 * s + 1], c->st));
             CK(cudaStreamWaitEvent(co->st, co->evs[2 * s + 1], 0));

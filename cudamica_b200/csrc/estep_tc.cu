@@ -124,20 +124,22 @@ int tc_selftest(int mode, int N, int K, const float* hA, const float* hB, float*
 }
 
 // Tile shapes the context can run (TcCfg): 0 = 3 density warpgroups,
-// 48-sample tiles, 2 x stages (the default); 1 = 2 warpgroups, 32-sample tiles,
-// 2 stages; 2 = 2 warpgroups, 3 stages.
+// 48-sample tiles, 2 x stages; 1 = 2 warpgroups, 32-sample tiles, 2 stages; 2 = 2
+// warpgroups, 3 stages.
 cudaError_t launch_estep_tc_one(const EStepArgs& a, int nclusters, cudaStream_t st, int shape);
 int tc_wg2_max_clusters(int n, int m, int M, int nst);
 cudaError_t tc_wg2_launch(const EStepArgs& a, int nclusters, cudaStream_t st, int split, int nst);
 
 int tc_num_shapes() { return 3; }
-// The shape that shape 0, "the default", stands for.  With one model and four or
-// five mixtures the single-phase kernel's sums and parameters take about 170
-// registers a thread, more than 3 density warpgroups leave (136): 2 warpgroups
-// measured 168 us against 280 at n = 64, T = 300k, m = 5.  With several models
-// and five mixtures the log2|y| cache fits beside 2 warpgroups only: 1.48 ms
-// against 1.60 at n = 128, T = 300k, M = 3 (m = 4 the other way: 1.33 against
-// 1.19), both taken on tiles of consecutive samples.
+// The shape of a new context whose configuration names none, and of the cohort
+// kernel.  With one model and four or five mixtures the single-phase kernel's sums
+// and parameters take about 170 registers a thread, more than 3 density warpgroups
+// leave (136): 2 warpgroups measured 168 us against 282 at n = 64, T = 300k, m = 5,
+// 150 against 153 at m = 4 (n = 32: 72 against 78; n = 128: 287 against 285).  With several
+// models and five mixtures the log2|y| cache fits beside 2 warpgroups only: 1.12 ms
+// against 1.17 at n = 128, T = 400k, M = 2 at the start of a fit and 0.95 against 0.97 in
+// the middle; at M = 3, T = 300k 1.41 against 1.43 and 1.12 against 1.09 (m = 4 the other
+// way: 1.00 against 0.92 and 0.85 against 0.76 at M = 2).
 int tc_default_shape(int m, int M) { return m == 5 || (M == 1 && m == 4) ? 1 : 0; }
 static int shape_wg(int shape) { return shape == 0 ? 3 : 2; }
 // Samples per tile: 16 rows per warpgroup, R samples per row.

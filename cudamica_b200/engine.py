@@ -293,7 +293,8 @@ class Amica:
         _chk(lib().amica_test_arm_wait_fault(self._ctx, int(wait_cycles)), "amica_test_arm_wait_fault")
 
     def set_tile_shape(self, shape: int) -> None:
-        """The fused E-step's tile shape (amica_set_tile_shape): 0, 1 or 2."""
+        """The fused E-step's tile shape (amica_set_tile_shape): 0 (3 density
+        warpgroups), 1 or 2."""
         _chk(lib().amica_set_tile_shape(self._ctx, int(shape)), "amica_set_tile_shape")
 
     def set_grid(self, max_clusters: int) -> int:

@@ -68,9 +68,9 @@ typedef struct amica_cfg {
     int64_t tc_shape;       /* mixed form up to 128 channels: tile shape of the fused E-step,
                                0 the default for the model and mixture counts (3 density
                                warpgroups and 48-sample tiles with 2 x stages; shape 1 with
-                               5 mixtures, or one model and 4), 1 2 warpgroups and 32-sample tiles with 2 stages, 2 the
-                               same with 3 stages (cudamica_b200.autotune picks one by
-                               measurement) (new key) */
+                               5 mixtures, or one model and 4), 1 2 warpgroups and 32-sample
+                               tiles with 2 stages, 2 the same with 3 stages
+                               (cudamica_b200.autotune picks one by measurement) (new key) */
     double lrate0, lratemax, lnatrate, lratefact, rho0, rholrate, rhomin, rhomax, rejsig;
     double phi_split_rel;   /* the threshold of phi_split = 2 (default 1e-4) (new key) */
 } amica_cfg;
@@ -250,8 +250,8 @@ int amica_shard_scatter(amica_ctx *ctx, const double *d_sums_total, int64_t T_to
                         double *d_scatter);
 int amica_shard_sphere(amica_ctx *ctx, const double *d_scatter_total, int64_t T_total);
 
-/* Switch the fused E-step's tile shape (amica_cfg.tc_shape) of a mixed-form
- * context of at most 128 channels; the grid goes back to as many clusters as
+/* Switch the fused E-step's tile shape (amica_cfg.tc_shape; here 0 is always the 3
+ * density warpgroups) of a mixed-form context of at most 128 channels; the grid goes back to as many clusters as
  * fit (the partial sums are sized for every shape).  AMICA_ERR_UNSUPPORTED for
  * other contexts. */
 int amica_set_tile_shape(amica_ctx *ctx, int64_t shape);
