@@ -23,7 +23,8 @@
 // two grid barriers per round (n = 160: 15.9 ms).
 //
 // A covariance that is not numerically positive definite (a pivot below
-// n eps max diag: rank-deficient data) is left to that form: *done stays 0.
+// n eps max diag: rank-deficient data) is left to that form: *done stays 0.  So is
+// a device that has no 16 SMs for one cluster.
 #include <cooperative_groups.h>
 #include <cstdint>
 
@@ -34,7 +35,7 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr int kMaxCtas = 16;       // above 8: the non-portable cluster size
-constexpr int kMaxBlk = 16;        // columns per block (n = 256 on 8 CTAs)
+constexpr int kMaxBlk = 12;        // columns per block (n = 192 on 8 CTAs)
 constexpr int kMaxSweeps = 40;
 
 __device__ __forceinline__ double rcp_approx(double x) {
@@ -314,9 +315,9 @@ cudaError_t launch_eig(const double* C, double* V, double* evals, int n, int K, 
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         int fits = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fits, kern, &cfg);
-        if (e != cudaSuccess || fits < 1) {            // no 16 SMs in one place: half as many CTAs
+        if (e != cudaSuccess || fits < 1) {            // *done is 0
             cudaGetLastError();
-            return launch_eig<NE>(C, V, evals, n, 8, (n + 15) / 16, done, st);
+            return cudaSuccess;
         }
     }
     return cudaLaunchKernelEx(&cfg, kern, C, V, evals, n, b, done);
@@ -328,9 +329,9 @@ namespace amica {
 
 // V (n x n, column-major) and evals of the covariance C; *done = 1 when they
 // were written, 0 when C is not numerically positive definite.  The cluster has
-// as many CTAs as keep 8 to 12 columns in a block: a step's pairs then run one
-// per warp with two or three warps per scheduler (16 CTAs against 8: n = 256 2.2
-// ms against 2.8, n = 160 the same).
+// as many CTAs as keep 5 to 8 columns in a block (9 to 12 at 129 to 192 channels): a
+// step's pairs then run one per warp with two or three warps per scheduler (16 CTAs
+// against 8: n = 256 2.2 ms against 2.8, n = 160 the same).
 cudaError_t launch_eig_cluster(const double* C, double* V, double* evals, int n, int* done, cudaStream_t st) {
     if (n < 2 || n > 256) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(done, 0, sizeof(int), st);
