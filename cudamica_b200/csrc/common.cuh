@@ -44,7 +44,8 @@ struct Ctrl {
     int64_t iter, numdec, nkeep, nrej_total, rej_passes;
     int64_t newton, ll_decreased, no_newt, last_rejected;
     double rej_mean, rej_std;
-    // CTAs of the two M-step kernels that are done (zero between iterations)
+    // CTAs of the two M-step kernels that are done (both set to zero at the end of
+    // the first)
     int64_t mstep_done, reparm_done;
     // split correction of phi (tensor-core form): the flag the E-step reads
     int64_t phi_split;

@@ -879,7 +879,11 @@ int amica_run(amica_ctx* c, int64_t maxiter, amica_iter_out* hist) {
 }
 
 // Parameters in and out go through the pinned staging area in one copy up to this
-// size; above it the arrays are copied one by one from and to the caller's memory.
+// size; above it the arrays are copied one by one from and to the caller's memory,
+// which the driver pipelines while a staged copy waits for the whole memcpy.  Staged
+// against one by one: set_params and one iteration 113 and 130 us, get_params 35 and
+// 105 at 13 KB (n = 32, m = 3); 480 and 495, 255 and 260 at 1.1 MB (n = 256, M = 2, m = 5); 600
+// and 570, 370 and 380 at 2.2 MB (M = 4).
 constexpr size_t kStageBytes = 2u << 20;
 
 int amica_get_params(amica_ctx* c, double* A, double* W, double* cc, double* gm, double* alpha,

@@ -13,7 +13,7 @@
 //             B = x tile (K-major, TMA), D -> TMEM (2 buffers)
 //       MMA2  phi_h += G B^T            M=128 N=128 K=48
 //             A = G, B = the b tile, both K-major tiles written by the density
-//             warps, D -> TMEM for the CTA's life
+//             warps, D -> TMEM, from there to FP64 every 32 to 128 tiles
 //   warps 0-11 (3 warpgroups x 4 warps): thread = (TMEM lane, warpgroup =
 //     16-row slice).  Each reads its b values with tcgen05.ld, evaluates the
 //     generalized-Gaussian mixture densities and the log-sum-exp over
@@ -86,14 +86,6 @@ struct TcCfg {
                                   : 384u + (uint32_t)(kSub * (c - 2 * kGapChunks));
     }
 };
-using TcDef = TcCfg<3, 2>;               // shape 0
-constexpr int kS = TcDef::kS;            // samples per tile (MMA1 N)
-constexpr int kWG = TcDef::kWG;          // density warpgroups
-constexpr int kDensWarps = TcDef::kDensWarps;
-constexpr int kThreads = TcDef::kThreads;
-constexpr int kCtlRegs = TcDef::kCtlRegs;
-constexpr int kDensRegs = TcDef::kDensRegs;
-constexpr int kSub = TcDef::kSub;
 // A tile's rows come kSegRows at a time from kS / kSegRows segments of the data
 // (tile t: rows t kSegRows .. of every segment), not as one run.  The models of
 // consecutive samples are mostly the same, and a model whose responsibility for
@@ -126,12 +118,10 @@ __host__ __device__ constexpr int phi_period_of(int ntile_local) {
 // (MMAs done reading it) barrier
 constexpr int kMaxStages = 3;
 
-constexpr int kL2Chunks = TcDef::kL2Chunks;
-__device__ __forceinline__ uint32_t l2_chunk_col(int c) { return TcDef::l2col(c); }
 
 // SPLIT: the form with the split correction of phi (one x stage; the G and b
 // tiles twice as wide, their low parts in columns [kS, 2 kS)).
-template <int NP, bool SPLIT = false, class Cf = TcDef>
+template <int NP, bool SPLIT, class Cf>
 struct TcShape {
     static constexpr int kS = Cf::kS, kWG = Cf::kWG, kSub = Cf::kSub, kDensWarps = Cf::kDensWarps;
     static constexpr int KB = NP / 32;                       // 128-B column blocks of x / W
