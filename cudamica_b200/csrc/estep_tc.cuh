@@ -108,8 +108,8 @@ constexpr int kFlush = 16;
 // the blocks is met in 5/9 of the steps instead of 1/3).  Half as many tiles make up
 // for twice as many steps, the most that segments of two can give, and 128 bounds
 // the error of long fits.  Relative error of phi (n = 128, M = 3, m = 3, middle of a fit)
-// at T = 1M: 5.8e-5 in one period, 1.6e-5 now, at 300k: 2.1e-5 -> 1.5e-5; the E-step
-// at T = 1M takes 2.13 ms instead of 2.10 (periods of 64 tiles: 2.12 and 9e-6, of 32: 2.15).
+// at T = 1M: 5.8e-5 in one period, 1.6e-5 now, at 300k: 2.1e-5 -> 1.5e-5.  Taking phi out
+// costs the E-step 3 to 5 us each time (2.10 ms at T = 1M).
 __host__ __device__ constexpr int phi_period_of(int ntile_local) {
     const int half = ((ntile_local + 1) / 2 + kFlush - 1) / kFlush * kFlush;
     return half < 32 ? 32 : half > 128 ? 128 : half;
