@@ -17,11 +17,12 @@
 // the slots in a fixed order, so results are deterministic.
 //
 // Bound by the FP32 pipe and shared-memory loads of the two products and by MUFU
-// latency with 8 to 12 warps per SM.  E-step, with lanes for 32, 64 or 128 channels,
-// K always the padded count and runs of consecutive samples -> now: n = 71, T =
-// 200k, M = 2, m = 3: 1039 -> 668 us; n = 128, T = 300k, M = 3: 2.51 -> 2.36 ms; n =
-// 256, T = 50k, M = 2, m = 5: 1.27 -> 1.22 ms; n = 100, T = 200k, M = 1: 564 -> 534 us;
-// n = 32, T = 300k, M = 1: 199 -> 197 us.
+// latency with 8 to 12 warps per SM.  E-step in the middle of a fit, with lanes for 32,
+// 64 or 128 channels, K always the padded count and runs of consecutive samples ->
+// now: n = 71, T = 200k, M = 2, m = 3: 1039 -> 617 us; n = 128, T = 300k, M = 3: 2.52 -> 2.33
+// ms; n = 256, T = 50k, M = 2, m = 5: 1.27 -> 1.19 ms; n = 100, T = 200k, M = 1: 565 -> 529 us;
+// n = 32, T = 300k, M = 1: 199 -> 189 us.  At the start of a fit, where no responsibility is
+// 0 yet: 1077 -> 652 us, 2.61 -> 2.57 ms, 1.27 -> 1.23 ms.
 #include <cooperative_groups.h>
 #include <cstdio>
 
